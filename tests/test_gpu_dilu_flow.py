@@ -1,0 +1,135 @@
+"""DILU sweeps and factor as a dataflow (every row waits for the values it
+reads): equal to the oracle bit for bit at the sizes where the row and chunk
+bookkeeping changes (a warp, a 256-row chunk and their neighbours), with rows
+of more entries than a thread holds in registers, host-driven, in graph mode
+and in a batch; FP32 inner solves equal to the per-level kernels."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def merged_polymesh(x, nx, ny, nz, seed, first, count):
+    """The channel's mesh with rows of `count` cells along x merged into one
+    cell each (faces inside a merged cell dropped), so a cell has up to
+    4 count + 2 neighbours; the cell at (first, 1, 1) takes the highest number
+    and the one at (first, 2, 2) the lowest, so one row has all its entries
+    below the diagonal and another all above."""
+    pm = x.channel_polymesh(nx, ny, nz, seed=None)
+    nc = nx * ny * nz
+    rep = np.arange(nc)
+    heads = []
+    for j, k in ((1, 1), (2, 2)):
+        ids = [first + i + nx * (j + ny * k) for i in range(count)]
+        rep[ids] = ids[0]
+        heads.append(ids[0])
+    rng = np.random.default_rng(seed)
+    order = [heads[1]] + [c for c in rng.permutation(np.unique(rep)) if c not in heads] + [heads[0]]
+    new = np.empty(nc, dtype=np.int64)
+    new[order] = np.arange(len(order))
+    cell = new[rep]
+    nI = pm.n_internal_faces
+    off, nodes = np.asarray(pm.face_offsets), np.asarray(pm.face_nodes)
+    o, n = cell[pm.owner], cell[pm.neighbour]
+    faces, own, nei = [], [], []
+    for f in range(pm.n_faces):
+        q = nodes[off[f]:off[f + 1]]
+        if f < nI:
+            if o[f] == n[f]:
+                continue
+            a, b = int(o[f]), int(n[f])
+            faces.append(q if a < b else q[::-1])
+            own.append(min(a, b))
+            nei.append(max(a, b))
+        else:
+            faces.append(q)
+            own.append(int(o[f]))
+    return type(pm)(points=pm.points, face_offsets=np.cumsum([0] + [len(q) for q in faces]).astype(np.int32),
+                    face_nodes=np.concatenate(faces).astype(np.int32), owner=np.array(own, dtype=np.int32),
+                    neighbour=np.array(nei, dtype=np.int32), patch_names=list(pm.patch_names),
+                    patch_sizes=list(pm.patch_sizes))
+
+
+MESHES = {
+    "31": lambda x: x.channel_polymesh(31, 1, 1, seed=1),
+    "32": lambda x: x.channel_polymesh(4, 4, 2, seed=2),
+    "33": lambda x: x.channel_polymesh(11, 3, 1, seed=3),
+    "255": lambda x: x.channel_polymesh(17, 5, 3, seed=4),
+    "256": lambda x: x.channel_polymesh(16, 4, 4, seed=5),
+    "257": lambda x: x.channel_polymesh(257, 1, 1, seed=None),  # 257 levels
+    "4620": lambda x: x.channel_polymesh(22, 15, 14, seed=6),
+    "merged": lambda x: merged_polymesh(x, 9, 6, 6, 7, 2, 3),
+}
+
+
+def _config(x, mesh, prec="fp64"):
+    model, config = x.cases.channel_case(mesh, iterations=3, precision=prec)
+    p = config.solvers["p"]
+    config.solvers["p"] = x.SolverSetup(solver=x.Cg(), preconditioner=x.DILU(), convergence=p.convergence,
+                                        relax=p.relax, rtol=0.05)
+    return x.build_config(model, config)
+
+
+def _start(x, c, mesh):
+    rng = np.random.default_rng(3)
+    c.set_field(x._abi.FIELD_U, 0.1 * rng.standard_normal((3, mesh.n_cells)))
+    c.set_field(x._abi.FIELD_P, np.zeros(mesh.n_cells))
+
+
+def _run(x, c, mesh, iters=3):
+    _start(x, c, mesh)
+    res, _ = c.simple_iterate(iters)
+    return res, c.get_field(x._abi.FIELD_U), c.get_field(x._abi.FIELD_P)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("name", list(MESHES))
+def test_dilu_flow_parity(x, orc, ctx, name, graph):
+    mesh = x.build_mesh3(MESHES[name](x))
+    if name == "merged":
+        assert np.diff(mesh.cell_faces_offset).max() == 14
+    cfg, keep = _config(x, mesh)
+    dm = x.DeviceMesh(ctx, mesh)
+    g = x.Case(dm, cfg)
+    g.set_graph_mode(graph)
+    o = orc.OracleCase(orc.OracleMesh.from_mesh3(mesh), cfg)
+    for a, b in zip(_run(x, g, mesh), _run(x, o, mesh)):
+        assert np.array_equal(a, b)
+    g.close()
+    dm.close()
+
+
+@pytest.mark.parametrize("name", ["33", "4620", "merged"])
+def test_dilu_flow_mixed_and_batch(x, ctx, name):
+    """Mixed precision: the default sweeps equal the per-level kernels, alone
+    and as a batch member beside a case of another size."""
+    mesh, other = x.build_mesh3(MESHES[name](x)), x.build_mesh3(MESHES["257"](x))
+    out = []
+    for mode in (2, 0):
+        cfg, keep = _config(x, mesh, "mixed")
+        dm = x.DeviceMesh(ctx, mesh)
+        c = x.Case(dm, cfg)
+        c.set_inner_cg(1)
+        c.set_dilu_mode(mode)
+        out.append(_run(x, c, mesh))
+        c.close()
+        dm.close()
+    batch = x.api.Batch(ctx, 2, 1 << 33)
+    members = []
+    for m in (other, mesh):
+        cfg, keep = _config(x, m, "mixed")
+        dm = x.DeviceMesh(ctx, m)
+        c = x.Case(dm, cfg)
+        _start(x, c, m)
+        assert batch.add(c)
+        members.append((c, dm, keep))
+    res = np.array([batch.simple_iterate()[0][1] for _ in range(3)])
+    c = members[1][0]
+    out.append((res, c.get_field(x._abi.FIELD_U), c.get_field(x._abi.FIELD_P)))
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            assert np.array_equal(a, b)
+    batch.close()
+    for c, dm, _ in members:
+        c.close()
+        dm.close()

@@ -4,10 +4,11 @@
 //  * the row mapping and block size of the SpMVs that carry no reduction
 //    (the BiCGSTAB SpMV): the canonical tile kernel or 1/2/4 rows per thread
 //    in blocks of 128/256/512 threads;
-//  * how a DILU application runs: one block sweeping every level (systems of
-//    up to 262,144 rows), one launch per level, or every level in one
-//    cooperative launch with a grid barrier between levels (systems of more
-//    than 32,768 rows).
+//  * how a DILU application runs: rows waiting for the values they read
+//    (dataflow), or, where that may lose, one block sweeping every level
+//    (systems of up to 4,096 rows), one launch per level, or every level in
+//    one cooperative launch with a grid barrier between levels (systems of
+//    more than 524,288 rows).
 // Each candidate is timed with CUDA events on the case's own matrix at first
 // use; choices are cached per size class (value size, log2 rows, entries per
 // row), so later cases of the same class reuse them without timing.
@@ -67,18 +68,26 @@ static SpmvShape tune_spmv(Case& C, Equation& E, const T* nz, const T* x, T* y) 
 }
 
 // the fastest DILU form on this system: 1 one-block sweeps, 2 one launch per
-// level, 3 one cooperative launch over every level
+// level, 3 one cooperative launch over every level, 4 dataflow.  Candidates by
+// size (measured on B200, us per application, dataflow against the best other
+// form): the one-block sweeps come within reach only below some 4k rows
+// (1,518 rows FP32: 20.3 / 18.6; 3,700 rows: 31.1 / 31.6; 6,400 rows FP64:
+// 26.7 / 43.3), the level forms only above 0.5M (884,736 rows FP32: 117 / 155;
+// 2.1M rows: 233 / 192, FP64 283 / 252)
 template <class T>
 static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, T* out) {
     const int reps = (int)std::max(3L, std::min(20L, 20000000L / std::max(E.nnz_csr, 1L)));
-    const bool sb = E.use_block, sg = E.use_grid;
-    int best = 2;
+    const bool sb = E.use_block, sg = E.use_grid, sf = E.use_flow;
+    kr_flow_unset(C.stream, C.flow_scratch<T>(out), (size_t)E.n * sizeof(T));
+    int best = 4;
     float best_ms = 1e30f;
-    for (int form = 1; form <= 3; ++form) {
-        if (form == 1 && E.n > 4 * DILU_BLOCK_MAX_ROWS) continue;
-        if (form == 3 && E.n <= DILU_BLOCK_MAX_ROWS / 2) continue;
+    if (E.n > 4096 && E.n <= 524288) return best;
+    for (int form = 1; form <= 4; ++form) {
+        if (form == 1 && E.n > 4096) continue;
+        if ((form == 2 || form == 3) && E.n <= 524288) continue;
         E.use_block = form == 1;
         E.use_grid = form == 3;
+        E.use_flow = form == 4;
         float ms = time_ms(C.stream, C.ev[6], C.ev[7], reps, [&] { C.dilu_ldiv(E, nz, D, b, out, nullptr); });
         if (ms < best_ms) {
             best_ms = ms;
@@ -87,6 +96,7 @@ static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, 
     }
     E.use_block = sb;
     E.use_grid = sg;
+    E.use_flow = sf;
     return best;
 }
 
@@ -120,6 +130,7 @@ void Case::autotune() {
         if (dilu_mode != 0) {
             E.use_block = dilu_mode == 1;
             E.use_grid = dilu_mode == 3;
+            E.use_flow = E.flow_D = false;
         } else if (SS.precond == XCAL_PRECOND_DILU) {
             TuneKey k = key_of(1, tsz, E);
             std::unique_lock<std::mutex> lk(g_tune_mu);
@@ -136,6 +147,7 @@ void Case::autotune() {
             }
             E.use_block = form == 1;
             E.use_grid = form == 3;
+            E.use_flow = form == 4;
         }
     }
     sync();

@@ -45,11 +45,11 @@ struct Batch {
     DBuf<int2> tmap_act;             // subset (mixed-precision outer steps)
     DBuf<unsigned char> sys[2][4];   // [fp64, fp32][Ux, Uy, Uz, p] descriptor tables
     DBuf<BAux> aux[4];               // [Ux, Uy, Uz, p] FP64-side tables
-    DBuf<int2> dlo[2], dup[2];       // merged DILU levels per equation (large systems)
-    std::vector<int> dlo_off[2], dup_off[2];
-    DBuf<int> small_ids;             // systems that run DILU as one block
-    int n_small = 0;
-    int small_n = 0;                 // rows of the largest of them
+    DBuf<int2> flow_items;           // DILU sweeps: (case, chunk of positions), chunk by chunk
+    int n_flow = 0;
+    DBuf<unsigned int> tickets;      // DILU sweeps: forward and backward chunk counters
+    DBuf<int> ferr;                  // a DILU dataflow wait gave up
+    int* hferr = nullptr;            // pinned
     DBuf<unsigned int> bars;         // persistent CG: barrier state per system
     DBuf<int> mem_ids;               // persistent CG, cluster form: member systems grouped by cluster size
     int* hmem = nullptr;             // pinned staging of mem_ids
@@ -145,16 +145,25 @@ struct Batch {
         bars.zero(stream);
         perr.alloc(1);
         perr.zero(stream);
+        tickets.alloc(2);
+        tickets.zero(stream);
+        ferr.alloc(1);
+        ferr.zero(stream);
+        XCAL_CUDA(cudaMallocHost(&hferr, sizeof(int)));
     }
     ~Batch() {
         if (stream) cudaStreamSynchronize(stream);
         drop_graphs();
         for (auto& gs : case_graph) drop_case_graphs(gs);
-        for (size_t i = 0; i < cases.size(); ++i) cases[i]->stream = own[i];
+        for (size_t i = 0; i < cases.size(); ++i) {
+            cases[i]->stream = own[i];
+            cases[i]->batch_err = nullptr;
+        }
         for (cudaEvent_t e : joined) cudaEventDestroy(e);
         if (forked) cudaEventDestroy(forked);
         if (hS) cudaFreeHost(hS);
         if (hmem) cudaFreeHost(hmem);
+        if (hferr) cudaFreeHost(hferr);
         for (int g = 0; g < 5; ++g) {
             if (gstream[g]) {
                 cudaStreamSynchronize(gstream[g]);
@@ -225,6 +234,7 @@ struct Batch {
         case_graph.emplace_back();
         own.push_back(c->stream);
         c->stream = stream;
+        c->batch_err = ferr.p;
         cases.push_back(c);
         footprint.push_back(charge);
         used += charge;
@@ -236,6 +246,7 @@ struct Batch {
         if (i < 0) fail(XCAL_ERR_INVALID, "batch: case not admitted");
         sync();
         c->stream = own[i];
+        c->batch_err = nullptr;
         used -= footprint[i];
         cudaEventDestroy(joined[i]);
         joined.erase(joined.begin() + i);
@@ -282,6 +293,7 @@ struct Batch {
             if (SS.solver == XCAL_SOLVER_CG && SS.precond == XCAL_PRECOND_NONE) B.vec[KV_Z] = B.vec[KV_R];
             B.lo = level_view<T>(E, 0);
             B.up = level_view<T>(E, 1);
+            B.flow_y = c->flow_scratch<T>(B.vec[SS.solver == XCAL_SOLVER_CG ? KV_Z : KV_R]);
         }
         sys[prec][slot].upload((const unsigned char*)h.data(), h.size() * sizeof(BSys<T>), stream);
     }
@@ -325,6 +337,7 @@ struct Batch {
                 B.uslice = E.usell.slice.p;
                 B.uval = E.usell.val.p;
                 B.uval32 = E.usell.val32.p;
+                B.flow_y = c->flow_scratch<double>(cg && c->cfg.precision == XCAL_PREC_FP64 ? c->ws.z.p : nullptr);
             }
             B.n = E.n;
             B.ntiles = (E.n + RED_TILE - 1) / RED_TILE;
@@ -354,46 +367,15 @@ struct Batch {
                     fill_sys<double>(0, slot);
                 fill_aux(slot);
             }
-            // small systems: one block per DILU application
-            std::vector<int> ids;
-            small_n = 0;
-            for (int i = 0; i < nc; ++i)
-                if (cases[i]->U.dilu_block()) {
-                    ids.push_back(i);
-                    small_n = std::max(small_n, cases[i]->U.n);
-                }
-            n_small = (int)ids.size();
-            if (ids.empty()) ids.push_back(0);
-            small_ids.upload(ids, stream);
-            // DILU levels of the other systems merged across cases: level l
-            // holds every such case's level-l rows
-            for (int e = 0; e < 2; ++e) {
-                for (int dir = 0; dir < 2; ++dir) {
-                    size_t L = 0;
-                    for (Case* c : cases) {
-                        Equation& E = e == 0 ? c->U : c->P;
-                        if (E.dilu_block()) continue;
-                        const std::vector<int>& off = dir == 0 ? E.lower_off : E.upper_off;
-                        if (off.size() > 1) L = std::max(L, off.size() - 1);
-                    }
-                    std::vector<int> moff(L + 1, 0);
-                    std::vector<int2> rows;
-                    for (size_t l = 0; l < L; ++l) {
-                        for (int i = 0; i < nc; ++i) {
-                            Equation& E = e == 0 ? cases[i]->U : cases[i]->P;
-                            if (E.dilu_block()) continue;
-                            const std::vector<int>& off = dir == 0 ? E.lower_off : E.upper_off;
-                            const std::vector<int>& hr = dir == 0 ? E.h_lower_rows : E.h_upper_rows;
-                            if (l + 1 >= off.size()) continue;
-                            for (int k = off[l]; k < off[l + 1]; ++k) rows.push_back(make_int2(i, hr[k]));
-                        }
-                        moff[l + 1] = (int)rows.size();
-                    }
-                    if (rows.empty()) rows.push_back(make_int2(0, 0));
-                    (dir == 0 ? dlo[e] : dup[e]).upload(rows, stream);
-                    (dir == 0 ? dlo_off[e] : dup_off[e]) = moff;
-                }
-            }
+            // the DILU sweeps' work list: chunk 0 of every case, then chunk 1, ...
+            std::vector<int2> items;
+            int maxn = 0;
+            for (Case* c : cases) maxn = std::max(maxn, c->U.n);
+            for (int ch = 0; ch * FLOW_THREADS < maxn; ++ch)
+                for (int i = 0; i < nc; ++i)
+                    if (ch * FLOW_THREADS < cases[i]->U.n) items.push_back(make_int2(i, ch));
+            n_flow = (int)items.size();
+            flow_items.upload(items, stream);
         }
         sync();
         dirty = false;
@@ -401,13 +383,12 @@ struct Batch {
 
     // ---- batched Krylov solve --------------------------------------------
     template <class T>
-    void apply_M(int prec, int slot, int e, int pt, const int2* tm, int nt, int in, int out, int use_S) {
+    void apply_M(int prec, int slot, int pt, const int2* tm, int nt, int in, int out, int use_S) {
         const BSys<T>* sy = (const BSys<T>*)sys[prec][slot].p;
         if (pt == XCAL_PRECOND_JACOBI)
             kb_jacobi_apply<T>(stream, sy, tm, nt, in, out, use_S);
         else if (pt == XCAL_PRECOND_DILU)
-            kb_dilu<T>(stream, sy, small_ids.p, n_small, small_n, dlo[e].p, dlo_off[e], dup[e].p, dup_off[e], in, out,
-                       use_S);
+            kb_dilu<T>(stream, sy, flow_items.p, n_flow, tickets.p, ferr.p, in, out, use_S);
         else
             kb_copy<T>(stream, sy, tm, nt, in, out, use_S);
     }
@@ -417,15 +398,14 @@ struct Batch {
     template <class T>
     void krylov(int prec, int slot, const xcal_solver_setup& SS, const int2* tm, int nt,
                 const std::vector<int>& members) {
-        const int e = slot < 3 ? 0 : 1;
         const BSys<T>* sy = (const BSys<T>*)sys[prec][slot].p;
         const int pt = SS.precond;
         const bool cg = SS.solver == XCAL_SOLVER_CG;
         if (cg) {
-            if (pt != XCAL_PRECOND_NONE) apply_M<T>(prec, slot, e, pt, tm, nt, KV_R, KV_Z, 0);
+            if (pt != XCAL_PRECOND_NONE) apply_M<T>(prec, slot, pt, tm, nt, KV_R, KV_Z, 0);
             kb_cg_start<T>(stream, sy, tm, nt);
         } else {
-            apply_M<T>(prec, slot, e, pt, tm, nt, KV_R0, KV_R, 0);
+            apply_M<T>(prec, slot, pt, tm, nt, KV_R0, KV_R, 0);
             kb_bicg_start<T>(stream, sy, tm, nt);
         }
         int itmax = 0;
@@ -532,7 +512,6 @@ struct Batch {
     // one Krylov iteration of every system (early exit where done)
     template <class T>
     void iterate(int prec, int slot, const xcal_solver_setup& SS, const int2* tm, int nt) {
-        const int e = slot < 3 ? 0 : 1;
         const BSys<T>* sy = (const BSys<T>*)sys[prec][slot].p;
         const int pt = SS.precond;
         const bool cg = SS.solver == XCAL_SOLVER_CG;
@@ -544,16 +523,16 @@ struct Batch {
                         kb_cg_update<T>(stream, sy, tm, nt, 1);
                     } else {
                         kb_cg_update<T>(stream, sy, tm, nt, 0);
-                        if (pt == XCAL_PRECOND_DILU) apply_M<T>(prec, slot, e, pt, tm, nt, KV_R, KV_Z, 1);
+                        if (pt == XCAL_PRECOND_DILU) apply_M<T>(prec, slot, pt, tm, nt, KV_R, KV_Z, 1);
                         kb_cg_rz<T>(stream, sy, tm, nt);
                     }
                 } else {
                     kb_spmv<T>(stream, sy, tm, nt, KV_P, KV_Q);
-                    apply_M<T>(prec, slot, e, pt, tm, nt, KV_Q, KV_V, 1);
+                    apply_M<T>(prec, slot, pt, tm, nt, KV_Q, KV_V, 1);
                     kb_bicg_alpha<T>(stream, sy, tm, nt);
                     kb_bicg_s<T>(stream, sy, tm, nt);
                     kb_spmv<T>(stream, sy, tm, nt, KV_S, KV_Q);
-                    apply_M<T>(prec, slot, e, pt, tm, nt, KV_Q, KV_T, 1);
+                    apply_M<T>(prec, slot, pt, tm, nt, KV_Q, KV_T, 1);
                     kb_bicg_omega<T>(stream, sy, tm, nt);
                     kb_bicg_xr<T>(stream, sy, tm, nt);
                     kb_bicg_p<T>(stream, sy, tm, nt);
@@ -645,6 +624,7 @@ struct Batch {
         };
         const clk::time_point t0 = clk::now();
         rebuild();
+        XCAL_CUDA(cudaMemsetAsync(ferr.p, 0, sizeof(int), stream));
         bool fresh = false;
         for (Case* c : cases) {
             fresh = fresh || !c->initialised;
@@ -727,7 +707,9 @@ struct Batch {
                 if (c->has_k()) c->turbulence();
             });
         XCAL_CUDA(cudaMemcpyAsync(hres, res.p, 4 * cases.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
+        XCAL_CUDA(cudaMemcpyAsync(hferr, ferr.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
         sync();
+        if (*hferr) fail(XCAL_ERR_TIMEOUT, "batch: a DILU sweep's wait gave up");
         const clk::time_point t4 = clk::now();
         ++iterations;
         phase_ms[1] += us;

@@ -39,8 +39,9 @@ struct BSys {
     double* part1;
     int n;
     int ntiles;
-    // level-ordered triangles (one-block DILU sweeps of small systems)
+    // level-ordered triangles and the scratch of the DILU sweeps
     LevelView<T> lo, up;
+    T* flow_y;
 };
 
 // FP64 side of one equation slot of a case inside a batched solve: the
@@ -75,6 +76,7 @@ struct BAux {
     const int* uslice;
     double* uval;
     float* uval32;
+    double* flow_y;     // the sweeps' scratch (FP32 solves use it as floats)
     int n, ntiles;
 };
 
@@ -89,7 +91,7 @@ void kb_correct(cudaStream_t s, const BAux* aux, const int2* tmap, int ntiles_to
 void kb_residual(cudaStream_t s, const BAux* aux, const int2* tmap, int ntiles_total);
 void kb_to_float(cudaStream_t s, const BAux* aux, const int2* tmap, int ntiles_total);
 // level copies of the DILU triangles: values from nz (fp32: nz32) and the
-// lower triangle's 1/D per slot from P (fp32: P32)
+// lower triangle's 1/D per slot from P (fp32: P32); the sweeps' scratch unset
 void kb_level_refresh(cudaStream_t s, const BAux* aux, const int2* tmap, int ntiles_total, int fp32);
 
 // batched launchers (kernels_batch.cu); tmap has ntiles_total entries
@@ -100,14 +102,12 @@ void kb_jacobi_apply(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int n
                      int use_S);
 template <class T>
 void kb_copy(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int ntiles_total, int in, int out, int use_S);
-// DILU application: systems listed in small_ids (n <= DILU_BLOCK_MAX_ROWS)
-// one block each over their level-ordered triangles (y in shared memory when
-// the largest of them, small_n rows, fits), the others level by level over
-// merged (system, row) lists
+// DILU application of every system (k_dilu_flow's rows, forward then
+// backward): items lists (system, chunk of FLOW_THREADS positions) in chunk
+// order; tickets: two words, zeroed here; err as in kr_dilu_flow
 template <class T>
-void kb_dilu(cudaStream_t s, const BSys<T>* sys, const int* small_ids, int n_small, int small_n, const int2* lo_rows,
-             const std::vector<int>& lo_off, const int2* up_rows, const std::vector<int>& up_off, int in, int out,
-             int use_S);
+void kb_dilu(cudaStream_t s, const BSys<T>* sys, const int2* items, int n_items, unsigned int* tickets, int* err,
+             int in, int out, int use_S);
 template <class T>
 void kb_cg_start(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int ntiles_total);
 // every system's CG solve (Jacobi: jacobi = 1; none: 0) in one cooperative

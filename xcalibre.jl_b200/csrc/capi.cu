@@ -473,6 +473,7 @@ int32_t xcal_case_set_dilu_mode(xcal_case* cs, int32_t mode) {
     if (mode != 0) {
         c->U.use_block = c->P.use_block = mode == 1;
         c->U.use_grid = c->P.use_grid = mode == 3;
+        c->U.use_flow = c->P.use_flow = c->U.flow_D = c->P.flow_D = false;
     }
     if (c->step_graph) {  // a captured step holds the previous form
         c->sync();
@@ -491,7 +492,7 @@ int32_t xcal_case_tuning(xcal_case* cs, int32_t* out6) {
         for (int e = 0; e < 2; ++e) {
             out6[3 * e] = E[e]->spmv_shape.rows_per_thread;
             out6[3 * e + 1] = E[e]->spmv_shape.block;
-            out6[3 * e + 2] = E[e]->use_block ? 1 : (E[e]->use_grid ? 2 : 0);
+            out6[3 * e + 2] = E[e]->use_flow ? 2 : E[e]->use_block ? 1 : (E[e]->use_grid ? 2 : 0);
         }
     })
 }

@@ -426,7 +426,7 @@ static void build_fold(Equation& E, cudaStream_t s, bool uniform_ok) {
 void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& bcs, int nvec,
                            bool need_dilu, cudaStream_t s) {
     int n = E.n = m.nC;
-    E.use_block = n <= DILU_BLOCK_MAX_ROWS;
+    E.use_flow = E.flow_D = need_dilu;
     std::vector<std::vector<int>> extra(n);
     for (const xcal_bc& bc : bcs) {
         if (bc.type != XCAL_BC_PERIODIC_PARENT) continue;
@@ -1395,6 +1395,10 @@ void Case::update_precond_E(Equation& E, int pt) {
     if (pt == XCAL_PRECOND_JACOBI) {
         kr_jacobi_update(stream, E.view(), E.nz.p, E.P.p);
     } else if (pt == XCAL_PRECOND_DILU) {
+        if (E.flow_D) {
+            kr_dilu_D_flow(stream, E.n, level_d_view(E), E.nz.p, E.P.p, ws.bar.p, flow_err());
+            return;
+        }
         if (E.dilu_block()) {
             kr_dilu_D_lv_block(stream, E.n, level_d_view(E), E.nz.p, E.P.p);
             return;
@@ -1407,11 +1411,28 @@ void Case::update_precond_E(Equation& E, int pt) {
     }
 }
 
+// Forward results of a dataflow DILU application: a workspace vector its
+// solve does not use.  FP64: z in BiCGSTAB, s in CG (whose preconditioned
+// residual is z); FP32 inner solves: the FP64 z
+template <class T>
+T* Case::flow_scratch(const T* out) {
+    if constexpr (sizeof(T) == 8)
+        return out == ws.z.p ? ws.s.p : ws.z.p;
+    else
+        return reinterpret_cast<T*>(ws.z.p);
+}
+template double* Case::flow_scratch<double>(const double*);
+template float* Case::flow_scratch<float>(const float*);
+
 template <class T>
 void Case::dilu_ldiv(Equation& E, const T* nz, const T* D, const T* b, T* out, const KScalars* S) {
     // both paths read the level-ordered triangles (values and 1/D refreshed
     // by dilu_refresh before the solve); nz is the matrix those mirror
     (void)nz;
+    if (E.use_flow && coop_ok_here() &&
+        kr_dilu_flow(stream, E.n, level_view<T>(E, 0), level_view<T>(E, 1), D, b, flow_scratch<T>(out), out,
+                     ws.bar.p, flow_err(), S))
+        return;
     if (E.dilu_block()) {
         kr_dilu_block(stream, E.n, level_view<T>(E, 0), level_view<T>(E, 1), D, b, out, S);
         return;
@@ -1432,8 +1453,14 @@ void Case::dilu_ldiv(Equation& E, const T* nz, const T* D, const T* b, T* out, c
 // copy the current off-diagonal values into the level-ordered triangles and
 // form the lower triangle's 1/D per slot (FP64 values and D, or the FP32
 // copies nz32 / P32 for the mixed inner solves); D must be current
-void Case::dilu_refresh(Equation& E, bool fp32) {
+void Case::dilu_refresh(Equation& E, bool fp32, bool cg) {
     if (E.lower_off.empty()) return;
+    if (E.use_flow) {  // the dataflow sweeps' scratch starts unset
+        if (fp32)
+            kr_flow_unset(stream, flow_scratch<float>(nullptr), (size_t)E.n * sizeof(float));
+        else
+            kr_flow_unset(stream, flow_scratch<double>(cg ? ws.z.p : nullptr), (size_t)E.n * sizeof(double));
+    }
     for (LevelSell* L : {&E.lsell, &E.usell}) {
         if (fp32) {
             kr_gather_vals(stream, L->nslots, L->src.p, E.nz32.p, L->val32.p);
@@ -1752,7 +1779,7 @@ void Case::solve_captured(int eqn, int comp) {
                          (SS.precond == XCAL_PRECOND_JACOBI || SS.precond == XCAL_PRECOND_NONE);
     const int jac = SS.precond == XCAL_PRECOND_JACOBI ? 1 : 0;
     if (!mixed) {
-        if (SS.precond == XCAL_PRECOND_DILU) dilu_refresh(E, false);
+        if (SS.precond == XCAL_PRECOND_DILU) dilu_refresh(E, false, SS.solver == XCAL_SOLVER_CG);
         KrylovVecs<double> V{ws.x.p, ws.r.p, ws.z.p, ws.p.p, ws.q.p, ws.v.p, ws.s.p, ws.t.p};
         const double* r0 = SS.solver == XCAL_SOLVER_CG ? V.r : V.q;
         kr_init_resid(stream, A, E.nz.p, b, field, ws.dx.p, V.x, SS.solver == XCAL_SOLVER_CG ? V.r : V.q);
@@ -1787,7 +1814,7 @@ void Case::solve_captured(int eqn, int comp) {
     } else {
         kr_to_float(stream, E.nnz, E.nz.p, E.nz32.p);
         if (SS.precond != XCAL_PRECOND_NONE) kr_to_float(stream, n, E.P.p, E.P32.p);
-        if (SS.precond == XCAL_PRECOND_DILU) dilu_refresh(E, true);
+        if (SS.precond == XCAL_PRECOND_DILU) dilu_refresh(E, true, SS.solver == XCAL_SOLVER_CG);
         KrylovVecs<float> V{ws.fx.p, ws.fr.p, ws.fz.p, ws.fp.p, ws.fq.p, ws.fv.p, ws.fs.p, ws.ft.p};
         const bool cg = SS.solver == XCAL_SOLVER_CG;
         float* rhs = cg ? V.r : ws.fd.p;
@@ -1889,12 +1916,12 @@ double Case::solve_system_ref(const SolveRef& R, int* iters, bool fp64) {
     // the DILU factor and applications as cooperative launches report a
     // barrier wait that gave up through ws.err, read back with the residual
     // below (it stays 0 otherwise)
-    const bool grid_dilu = SS.precond == XCAL_PRECOND_DILU && E.use_grid && !E.dilu_block();
+    const bool grid_dilu = SS.precond == XCAL_PRECOND_DILU && (E.use_flow || E.flow_D || (E.use_grid && !E.dilu_block()));
     if (cfg.precision == XCAL_PREC_MIXED && !fp64) {
         solve_mixed(E, SS, field, b, S, hS, gk, iters);
     } else {
         XCAL_CUDA(cudaMemcpyAsync(S, hS, sizeof(KScalars), cudaMemcpyHostToDevice, stream));
-        if (SS.precond == XCAL_PRECOND_DILU) dilu_refresh(E, false);
+        if (SS.precond == XCAL_PRECOND_DILU) dilu_refresh(E, false, SS.solver == XCAL_SOLVER_CG);
         KrylovVecs<double> V{ws.x.p, ws.r.p, ws.z.p, ws.p.p, ws.q.p, ws.v.p, ws.s.p, ws.t.p};
         if (SS.solver == XCAL_SOLVER_CG) {
             kr_init_resid(stream, A, nz, b, field, ws.dx.p, V.x, V.r);
@@ -1965,7 +1992,7 @@ void Case::solve_mixed(Equation& E, const xcal_solver_setup& SS, double* field, 
     } else {
         kr_to_float(stream, E.nnz, E.nz.p, E.nz32.p);
         if (SS.precond != XCAL_PRECOND_NONE) kr_to_float(stream, n, E.P.p, E.P32.p);
-        if (SS.precond == XCAL_PRECOND_DILU) dilu_refresh(E, true);
+        if (SS.precond == XCAL_PRECOND_DILU) dilu_refresh(E, true, SS.solver == XCAL_SOLVER_CG);
     }
     KrylovVecs<float> V{ws.fx.p, ws.fr.p, ws.fz.p, ws.fp.p, ws.fq.p, ws.fv.p, ws.fs.p, ws.ft.p};
     hS->mixed = 1;

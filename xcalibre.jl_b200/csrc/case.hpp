@@ -108,7 +108,9 @@ struct Equation {
     DBuf<int> d_lower_off, d_upper_off;           // level offsets (one-block sweeps)
     LevelSell lsell, usell;                       // level-ordered triangles (level-kernel sweeps)
     // launch choices (autotune.cu); neither changes any result
-    bool use_block = false;   // DILU as one-block sweeps (default: n <= DILU_BLOCK_MAX_ROWS)
+    bool use_flow = false;    // DILU applications as dataflow sweeps (k_dilu_flow); else:
+    bool use_block = false;   // DILU as one-block sweeps
+    bool flow_D = false;      // the DILU factor as a dataflow (k_dilu_D_flow)
     bool use_grid = false;    // else as one cooperative launch over every level (k_dilu_grid)
     SpmvShape spmv_shape;     // BiCGSTAB SpMV row mapping / block size
     bool dilu_block() const { return use_block; }
@@ -314,7 +316,14 @@ struct Case {
     void dilu_ldiv(Equation& E, const T* nz, const T* D, const T* b, T* out, const KScalars* S);
     template <class T>
     void apply_M(Equation& E, int ptype, const T* nz, const T* P, const T* in, T* out, const KScalars* S);
-    void dilu_refresh(Equation& E, bool fp32);
+    // cg: the solve is a CG (its z is the sweeps' output, not their scratch)
+    void dilu_refresh(Equation& E, bool fp32, bool cg);
+    template <class T>
+    T* flow_scratch(const T* out);
+    // where the dataflow kernels report a wait that gave up: the case's own
+    // flag, or the batch's while the case is resident in one
+    int* batch_err = nullptr;
+    int* flow_err() { return batch_err ? batch_err : ws.err.p; }
     template <class T>
     void krylov_iterate(Equation& E, const xcal_solver_setup& SS, const T* nz, const T* P, const T* c, const T* r0,
                         const KrylovVecs<T>& V, KScalars* S, KScalars* hS, int gk);

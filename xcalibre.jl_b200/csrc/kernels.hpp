@@ -235,12 +235,6 @@ void kr_jacobi_update(cudaStream_t s, const CSRView& A, const double* nz, double
 void kr_jacobi_smooth(cudaStream_t s, const CSRView& A, const double* nz, const double* b, double* x, double* xt,
                       int loops, double omega);
 void kr_dilu_D(cudaStream_t s, const int* rows, int nrows, const CSRView& A, const double* nz, double* D);
-template <class T>
-void kr_dilu_fwd(cudaStream_t s, const int* rows, int nrows, const CSRView& A, const T* nz, const T* D, const T* b,
-                 T* y, const KScalars* S);
-template <class T>
-void kr_dilu_bwd(cudaStream_t s, const int* rows, int nrows, const CSRView& A, const T* nz, const T* D, T* x,
-                 const KScalars* S);
 // DILU level sweeps over level-ordered triangles (positions k0..k1 of one
 // level); the forward sweep reads dinv (T(1)/D of each slot's column,
 // kr_level_dinv) instead of dividing per entry -- the same values
@@ -255,7 +249,6 @@ void kr_dilu_bwd_lv(cudaStream_t s, int k0, int k1, const int* rows, const int* 
                     const int* col, const T* val, const T* D, T* x, const KScalars* S);
 template <class T>
 void kr_gather_vals(cudaStream_t s, long n, const int* src, const T* vals, T* dst);
-// small systems (n <= DILU_BLOCK_MAX_ROWS): whole sweeps in one block
 // the lower triangle in level order, as the DILU factor reads it: per
 // position k its row, the diagonal slot of that row (dslot), and per entry
 // (in the row's own order) the column, the slot of a_ij (src) and of a_ji
@@ -278,8 +271,6 @@ struct LevelDView {
 void kr_dilu_D_lv_block(cudaStream_t s, int n, const LevelDView& L, const double* nz, double* D);
 bool kr_dilu_D_lv_grid(cudaStream_t s, const LevelDView& L, const double* nz, double* D, unsigned int* bar,
                        int* err);
-void kr_dilu_D_block(cudaStream_t s, const int* rows, const int* off, int nlev, const CSRView& A, const double* nz,
-                     double* D);
 // one triangle in level order, as the one-block sweep reads it: level l is
 // positions off[l] .. off[l+1] of rows[]; position k keeps cnt[k] slots at
 // slice[k/32] + k%32 + 32 j (values val, and for the lower triangle dinv)
@@ -306,10 +297,23 @@ void kr_dilu_block(cudaStream_t s, int n, const LevelView<T>& lo, const LevelVie
 template <class T>
 bool kr_dilu_grid(cudaStream_t s, const LevelView<T>& lo, const LevelView<T>& up, const T* D, const T* b, T* y,
                   unsigned int* bar, int* err, const KScalars* S);
-// the DILU factor D (every level of the lower triangle) as one cooperative
-// launch; rows/off: the lower triangle's level lists on the device
-bool kr_dilu_D_grid(cudaStream_t s, const int* rows, const int* off, int nlev, const CSRView& A, const double* nz,
-                    double* D, unsigned int* bar, int* err);
+// the same application as one cooperative launch in which every row waits for
+// just the values it reads (k_dilu_flow); false: nothing launched.  y: n
+// scratch values, unset (kr_flow_unset) on entry, left unset; out must alias
+// neither b nor y.  err: set when a wait gave up (y and out are then
+// incomplete)
+template <class T>
+bool kr_dilu_flow(cudaStream_t s, int n, const LevelView<T>& lo, const LevelView<T>& up, const T* D, const T* b,
+                  T* y, T* out, unsigned int* bar, int* err, const KScalars* S);
+// co-resident blocks of FLOW_THREADS threads of a dataflow kernel (0: none)
+constexpr int FLOW_THREADS = 256;
+int flow_grid(const void* kernel);
+// marks values as not yet computed (all bits one)
+void kr_flow_unset(cudaStream_t s, void* p, size_t bytes);
+// the DILU factor in the same way (D is set to unset values first; ticket:
+// one word, zeroed here), an ordinary launch
+void kr_dilu_D_flow(cudaStream_t s, int n, const LevelDView& L, const double* nz, double* D, unsigned int* ticket,
+                    int* err);
 void kr_residual(cudaStream_t s, const CSRView& A, const double* nz, const double* x, const double* b, KScalars* S,
                  double* part0, double* part1, double* out);
 // device-driven solve control of graph mode (conditional WHILE nodes)

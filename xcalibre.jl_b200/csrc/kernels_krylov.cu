@@ -291,17 +291,6 @@ __global__ void __launch_bounds__(DILU_BLOCK_THREADS) k_dilu_D_lv_block(int n, L
     }
 }
 
-// the D factor of a small system in one block, level by level
-__global__ void __launch_bounds__(DILU_BLOCK_THREADS) k_dilu_D_block(const int* __restrict__ rows,
-                                                                     const int* __restrict__ off, int nlev,
-                                                                     CSRView A, const double* __restrict__ nz,
-                                                                     double* D) {
-    for (int l = 0; l < nlev; ++l) {
-        for (int k = off[l] + threadIdx.x; k < off[l + 1]; k += blockDim.x) dilu_D_row(A, nz, D, rows[k]);
-        __syncthreads();
-    }
-}
-
 // a whole DILU application (forward + backward sweeps) of a small system in one block
 template <class T>
 __global__ void __launch_bounds__(DILU_BLOCK_THREADS) k_dilu_block(int n, LevelView<T> lo, LevelView<T> up,
@@ -426,23 +415,9 @@ __global__ void __launch_bounds__(DILU_GRID_THREADS, sizeof(T) == 4 ? 2 : 1) k_d
     }
 }
 
-// The DILU factor D of a large system in one cooperative launch: the lower
-// triangle's levels spread over the grid, a grid barrier between levels,
-// each row's arithmetic that of k_dilu_D (dilu_D_row).
-__global__ void __launch_bounds__(DILU_GRID_THREADS) k_dilu_D_grid(const int* __restrict__ rows,
-                                                                   const int* __restrict__ off, int nlev, CSRView A,
-                                                                   const double* __restrict__ nz, double* D,
-                                                                   unsigned int* bar, int* err) {
-    __shared__ int sh_err;
-    const int start = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    unsigned int nb = 0;
-    for (int l = 0; l < nlev; ++l) {
-        for (int k = off[l] + start; k < off[l + 1]; k += stride) dilu_D_row(A, nz, D, rows[k]);
-        if (l + 1 < nlev && !grid_barrier(bar, gridDim.x, nb, err, &sh_err)) return;
-    }
-}
-
-// the same over the level-ordered lower triangle
+// The DILU factor D of a large system in one cooperative launch: the levels of
+// the level-ordered lower triangle spread over the grid, a grid barrier
+// between levels, each row's arithmetic that of k_dilu_D (dilu_D_row)
 __global__ void __launch_bounds__(DILU_GRID_THREADS) k_dilu_D_lv_grid(LevelDView L, const double* __restrict__ nz,
                                                                       double* D, unsigned int* bar, int* err) {
     __shared__ int sh_err;
@@ -454,6 +429,76 @@ __global__ void __launch_bounds__(DILU_GRID_THREADS) k_dilu_D_lv_grid(LevelDView
     }
 }
 
+// ---- DILU sweeps as a dataflow over the level order (krylov_bodies.cuh) ----
+// One application: the forward rows, a grid barrier, the backward rows.  y:
+// scratch, all unset on entry and again on exit; out must alias neither b
+// nor y (the forward rows mark out as unset, which every block sees after the
+// barrier).
+template <class T>
+__global__ void __launch_bounds__(FLOW_THREADS) k_dilu_flow(int n, LevelView<T> lo, LevelView<T> up,
+                                                            const T* __restrict__ D, const T* __restrict__ b, T* y,
+                                                            T* out, unsigned int* bar, int* err, const KScalars* S) {
+    __shared__ int sh_err;
+    if (S && S->done) return;
+    const int start = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    const int warp0 = start & ~31;  // the warp's lanes leave the row loops together
+    for (int k0 = warp0; k0 < n; k0 += stride)
+        if (!flow_lower_rows(n, lo, b, y, out, k0, err)) break;
+    unsigned int nb = 0;
+    if (!grid_barrier(bar, gridDim.x, nb, err, &sh_err)) return;
+    for (int k0 = warp0; k0 < n; k0 += stride)
+        if (!flow_upper_rows(n, up, D, y, out, k0, err)) return;
+}
+
+// The DILU factor as the same dataflow: D starts unset; D_i needs the D of
+// its lower neighbours (dilu_D_pos's operands and order).  No barrier: the
+// blocks draw chunks of positions from a ticket, so a chunk's dependencies
+// belong to chunks already drawn by running blocks, and the kernel needs no
+// co-residency (it also runs inside a batch's per-case graphs).
+__global__ void __launch_bounds__(FLOW_THREADS) k_dilu_D_flow(int n, LevelDView L, const double* __restrict__ nz,
+                                                              double* D, unsigned int* ticket, int* err) {
+    __shared__ int sh_chunk;
+    const int chunks = (n + FLOW_THREADS - 1) / FLOW_THREADS;
+    for (;;) {
+        const int chunk = flow_ticket(ticket, &sh_chunk);
+        if (chunk >= chunks) return;
+        const int k = chunk * FLOW_THREADS + threadIdx.x;
+        int i = 0, c = -1, base = 0;
+        int cj[FLOW_U];
+        double pj[FLOW_U], yv[FLOW_U];
+        double d = 0.0;
+        if (k < n) {
+            i = L.rows[k];
+            c = L.cnt[k];
+            base = L.slice[k / SELL_C] + (k % SELL_C);
+            int sj[FLOW_U], tj[FLOW_U];
+#pragma unroll
+            for (int j = 0; j < FLOW_U; ++j)
+                if (j < c) {
+                    const int e = base + SELL_C * j;
+                    cj[j] = ld_stream(L.col + e);
+                    sj[j] = ld_stream(L.src + e);
+                    tj[j] = ld_stream(L.tsrc + e);
+                }
+            d = nz[L.dslot[k]];
+#pragma unroll
+            for (int j = 0; j < FLOW_U; ++j)
+                if (j < c) pj[j] = nz[tj[j]] * nz[sj[j]];
+        }
+        if (!flow_wait((const double*)D, L.col, base, c, cj, yv, err, [&] {
+#pragma unroll
+                for (int j = 0; j < FLOW_U; ++j)
+                    if (j < c) d = d - pj[j] / yv[j];
+                for (int j = FLOW_U; j < c; ++j) {
+                    const int e = base + SELL_C * j;
+                    d = d - (nz[ld_stream(L.tsrc + e)] * nz[ld_stream(L.src + e)]) / ld_flow(D + ld_stream(L.col + e));
+                }
+                st_flow(D + i, d);
+            }))
+            return;
+    }
+}
+
 // dinv[e] = T(1) / D[col[e]] (the forward sweep's per-entry reciprocal)
 template <class T>
 __global__ void k_level_dinv(long n, const int* __restrict__ col, const T* __restrict__ D, T* dinv) {
@@ -461,29 +506,9 @@ __global__ void k_level_dinv(long n, const int* __restrict__ col, const T* __res
         dinv[e] = T(1) / D[ld_stream(col + e)];
 }
 
-// forward_substitution! (preconditioners_1_DILU.jl:84-98), one level
-template <class T>
-__global__ void k_dilu_fwd(const int* __restrict__ rows, int nrows, CSRView A, const T* __restrict__ nz,
-                           const T* __restrict__ D, const T* __restrict__ b, T* y, const KScalars* S) {
-    if (S && S->done) return;
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nrows) return;
-    dilu_fwd_row(A, nz, D, b, y, rows[t]);
-}
-
-// backward_substitution! (preconditioners_1_DILU.jl:100-114), one level, in place
-template <class T>
-__global__ void k_dilu_bwd(const int* __restrict__ rows, int nrows, CSRView A, const T* __restrict__ nz,
-                           const T* __restrict__ D, T* x, const KScalars* S) {
-    if (S && S->done) return;
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nrows) return;
-    dilu_bwd_row(A, nz, D, x, rows[t]);
-}
-
 // DILU sweeps over the level-ordered triangles: thread per position k of a
 // level (row rows[k]); the entries are the row's own, in the row's order, so
-// each row's sum is dilu_fwd_row's / dilu_bwd_row's
+// each row's sum runs in the row's own entry order
 template <class T>
 __global__ void k_dilu_fwd_lv(int k0, int k1, const int* __restrict__ rows, const int* __restrict__ slice,
                               const unsigned char* __restrict__ cnt, const int* __restrict__ col,
@@ -1052,20 +1077,6 @@ void kr_dilu_D(cudaStream_t s, const int* rows, int nrows, const CSRView& A, con
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
-void kr_dilu_fwd(cudaStream_t s, const int* rows, int nrows, const CSRView& A, const T* nz, const T* D, const T* b,
-                 T* y, const KScalars* S) {
-    if (nrows <= 0) return;
-    k_dilu_fwd<T><<<(nrows + 255) / 256, 256, 0, s>>>(rows, nrows, A, nz, D, b, y, S);
-    XCAL_CHECK_LAUNCH();
-}
-template <class T>
-void kr_dilu_bwd(cudaStream_t s, const int* rows, int nrows, const CSRView& A, const T* nz, const T* D, T* x,
-                 const KScalars* S) {
-    if (nrows <= 0) return;
-    k_dilu_bwd<T><<<(nrows + 255) / 256, 256, 0, s>>>(rows, nrows, A, nz, D, x, S);
-    XCAL_CHECK_LAUNCH();
-}
-template <class T>
 void kr_dilu_fwd_lv(cudaStream_t s, int k0, int k1, const int* rows, const int* slice, const unsigned char* cnt,
                     const int* col, const T* val, const T* dinv, const T* b, T* y, const KScalars* S) {
     if (k1 <= k0) return;
@@ -1137,12 +1148,6 @@ bool kr_dilu_D_lv_grid(cudaStream_t s, const LevelDView& L, const double* nz, do
     XCAL_CHECK_LAUNCH();
     return true;
 }
-void kr_dilu_D_block(cudaStream_t s, const int* rows, const int* off, int nlev, const CSRView& A, const double* nz,
-                     double* D) {
-    if (nlev <= 0) return;
-    k_dilu_D_block<<<1, DILU_BLOCK_THREADS, 0, s>>>(rows, off, nlev, A, nz, D);
-    XCAL_CHECK_LAUNCH();
-}
 template <class T>
 void kr_dilu_block(cudaStream_t s, int n, const LevelView<T>& lo, const LevelView<T>& up, const T* D, const T* b,
                    T* y, const KScalars* S) {
@@ -1191,36 +1196,57 @@ bool kr_dilu_grid(cudaStream_t s, const LevelView<T>& lo, const LevelView<T>& up
     XCAL_CHECK_LAUNCH();
     return true;
 }
-bool kr_dilu_D_grid(cudaStream_t s, const int* rows, const int* off, int nlev, const CSRView& A, const double* nz,
-                    double* D, unsigned int* bar, int* err) {
-    static int blocks = -1;
-    if (blocks < 0) {
+int flow_grid(const void* kernel) {
+    static std::mutex mu;
+    static std::map<const void*, int> blocks;  // per kernel, one device type
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = blocks.find(kernel);
+    if (it == blocks.end()) {
         int dev = 0, sms = 0, per = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k_dilu_D_grid, DILU_GRID_THREADS, 0) ==
-                cudaSuccess)
-            blocks = sms * std::min(per, 2);
-        else
-            blocks = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, FLOW_THREADS, 0) != cudaSuccess)
+            sms = per = 0;
         cudaGetLastError();
+        it = blocks.emplace(kernel, sms * per).first;
     }
-    if (blocks <= 0 || nlev <= 0) return false;
+    return it->second;
+}
+template <class T>
+bool kr_dilu_flow(cudaStream_t s, int n, const LevelView<T>& lo, const LevelView<T>& up, const T* D, const T* b,
+                  T* y, T* out, unsigned int* bar, int* err, const KScalars* S) {
+    const int blocks = std::min(flow_grid((const void*)k_dilu_flow<T>), (n + FLOW_THREADS - 1) / FLOW_THREADS);
+    if (blocks <= 0 || (const T*)out == b || out == y) return false;
     XCAL_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), s));
-    CSRView Av = A;
-    void* args[] = {(void*)&rows, (void*)&off, &nlev, &Av, (void*)&nz, &D, &bar, &err};
+    LevelView<T> l = lo, u = up;
+    void* args[] = {&n, &l, &u, (void*)&D, (void*)&b, &y, &out, &bar, &err, (void*)&S};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(DILU_GRID_THREADS);
+    cfg.blockDim = dim3(FLOW_THREADS);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    XCAL_CUDA(cudaLaunchKernelExC(&cfg, (const void*)k_dilu_D_grid, args));
+    XCAL_CUDA(cudaLaunchKernelExC(&cfg, (const void*)k_dilu_flow<T>, args));
     XCAL_CHECK_LAUNCH();
     return true;
+}
+template bool kr_dilu_flow<double>(cudaStream_t, int, const LevelView<double>&, const LevelView<double>&,
+                                   const double*, const double*, double*, double*, unsigned int*, int*,
+                                   const KScalars*);
+template bool kr_dilu_flow<float>(cudaStream_t, int, const LevelView<float>&, const LevelView<float>&, const float*,
+                                  const float*, float*, float*, unsigned int*, int*, const KScalars*);
+void kr_flow_unset(cudaStream_t s, void* p, size_t bytes) { XCAL_CUDA(cudaMemsetAsync(p, 0xff, bytes, s)); }
+void kr_dilu_D_flow(cudaStream_t s, int n, const LevelDView& L, const double* nz, double* D, unsigned int* ticket,
+                    int* err) {
+    if (n <= 0) return;
+    kr_flow_unset(s, D, (size_t)n * sizeof(double));
+    XCAL_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s));
+    const int blocks = std::min(flow_grid((const void*)k_dilu_D_flow), (n + FLOW_THREADS - 1) / FLOW_THREADS);
+    k_dilu_D_flow<<<std::max(blocks, 1), FLOW_THREADS, 0, s>>>(n, L, nz, D, ticket, err);
+    XCAL_CHECK_LAUNCH();
 }
 template bool kr_dilu_grid<double>(cudaStream_t, const LevelView<double>&, const LevelView<double>&, const double*,
                                    const double*, double*, unsigned int*, int*, const KScalars*);
@@ -1286,10 +1312,6 @@ void kr_record(cudaStream_t s, const KScalars* S, int* out) {
     template void kr_bicg_xr<T>(cudaStream_t, int, T*, const T*, const T*, T*, const T*, KScalars*, double*,     \
                                 double*);                                                                       \
     template void kr_bicg_p<T>(cudaStream_t, int, const T*, const T*, T*, const KScalars*);                      \
-    template void kr_dilu_fwd<T>(cudaStream_t, const int*, int, const CSRView&, const T*, const T*, const T*, T*, \
-                                 const KScalars*);                                                              \
-    template void kr_dilu_bwd<T>(cudaStream_t, const int*, int, const CSRView&, const T*, const T*, T*,          \
-                                 const KScalars*);                                                              \
     template void kr_dilu_block<T>(cudaStream_t, int, const LevelView<T>&, const LevelView<T>&, const T*,       \
                                    const T*, T*, const KScalars*);                                              \
     template void kr_level_dinv<T>(cudaStream_t, long, const int*, const T*, T*);                                \

@@ -459,31 +459,7 @@ __device__ __forceinline__ void bicg_p_body(const TileCtx& tc, int n, const T* _
     }
 }
 
-// forward_substitution! row i (preconditioners_1_DILU.jl:84-98)
-template <class T>
-__device__ __forceinline__ void dilu_fwd_row(const CSRView& A, const T* __restrict__ nz, const T* __restrict__ D,
-                                             const T* __restrict__ b, T* y, int i) {
-    int ds = A.diag[i];
-    T sum = T(0);
-    for (int e = row_base(A, i); e < ds; e += SELL_C) {
-        int j = ld_stream(A.colval + e);
-        sum = sum + (ld_stream(nz + e) * y[j]) * (T(1) / D[j]);
-    }
-    y[i] = b[i] - sum;
-}
-
-// backward_substitution! row i (preconditioners_1_DILU.jl:100-114), in place
-template <class T>
-__device__ __forceinline__ void dilu_bwd_row(const CSRView& A, const T* __restrict__ nz, const T* __restrict__ D,
-                                             T* x, int i) {
-    int ds = A.diag[i];
-    T sum = T(0);
-    int e1 = row_base(A, i) + SELL_C * A.len[i];
-    for (int e = ds + SELL_C; e < e1; e += SELL_C) sum = sum + ld_stream(nz + e) * x[ld_stream(A.colval + e)];
-    x[i] = (x[i] - sum) / D[i];
-}
-
-// A DILU application of a small system (n <= DILU_BLOCK_MAX_ROWS) as one
+// A DILU application of a small system as one
 // block: every level of the forward sweep, then of the backward sweep, with a
 // block barrier between levels (rows of a level are independent).  It reads
 // the level-ordered triangles (position k of level order: cnt[k] slots at
@@ -495,8 +471,6 @@ __device__ __forceinline__ void dilu_bwd_row(const CSRView& A, const T* __restri
 // (preconditioners_1_DILU.jl:84-114) in the row's own entry order:
 //   forward  y_i = b_i - sum_j (a_ij y_j) (1/D_j)      (j < i)
 //   backward x_i = (x_i - sum_j a_ij x_j) / D_i        (j > i)
-// -- the values of the CSR-row sweeps (dilu_fwd_row / dilu_bwd_row), bit
-// for bit.
 constexpr int DILU_BLOCK_THREADS = 1024;
 
 // One level of a sweep over level positions k0..k1.  FP32: each thread
@@ -583,6 +557,183 @@ __device__ __forceinline__ void dilu_level_sweep(int n, const LevelView<T>& lo, 
     }
     if (ys != y)
         for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = ys[i];
+}
+
+// ---- DILU sweeps as a dataflow over the level order ----
+// A level barrier costs a launch or a grid barrier per level (about 4 us
+// each, 11-40 levels per application) although a row needs only its own few
+// neighbours.  Here every row waits for exactly the values it reads, and the
+// value is its own flag: the result array starts as a bit pattern that no
+// row ever stores (all ones, a NaN; a row whose result is NaN stores the
+// canonical one), so one relaxed load both polls and fetches, with no fence
+// and no flag array.  Rows are dealt out in level order, over co-resident
+// blocks (cooperative launch) or by tickets, and a warp takes its rows in
+// ascending position; a row's dependencies have smaller positions, so the
+// first unfinished row always runs and nothing can wait in a circle.  Waits
+// are bounded: after FLOW_SPIN_LIMIT polls *err is set and every block leaves.
+// Each row's arithmetic is that of the level kernels, in the row's entry
+// order, so the results are theirs bit for bit.  What bounds it: the chain of
+// dependent L2 round trips, one per level (about 1.05 us), then DRAM.
+// Measured on B200 per application, this against the fastest level form
+// (FP64, 2 x 13..20 levels): 6,400 rows 27 / 43 us, 27,025 rows 37 / 88 us,
+// 62,403 rows 45 / 123 us, 116,440 rows 48 / 119 us; FP32 262,144 rows
+// 61 / 131 us, 884,736 rows 117 / 155 us.  At 2.1M rows the level order's
+// scattered vector accesses cost more than its barriers (283 / 252 us), so
+// the autotuner times both.
+constexpr int FLOW_U = 6;  // slots per row held in registers (a hexahedral row has at most 6 in one triangle)
+constexpr int FLOW_SPIN_LIMIT = 1 << 21;
+
+__device__ __forceinline__ double ld_flow(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float ld_flow(const float* p) {
+    float v;
+    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool flow_unset(double v) { return __double_as_longlong(v) == -1LL; }
+__device__ __forceinline__ bool flow_unset(float v) { return __float_as_int(v) == -1; }
+__device__ __forceinline__ void st_flow(double* p, double v) {
+    if (isnan(v)) v = __longlong_as_double(0x7ff8000000000000LL);
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_flow(float* p, float v) {
+    if (isnan(v)) v = __int_as_float(0x7fc00000);
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+template <class T>
+__device__ __forceinline__ T flow_unset_value();
+template <>
+__device__ __forceinline__ double flow_unset_value<double>() { return __longlong_as_double(-1LL); }
+template <>
+__device__ __forceinline__ float flow_unset_value<float>() { return __int_as_float(-1); }
+
+// Polls the values ys[col] of one row's c slots (the first FLOW_U's columns
+// in cj, values landing in yv) until all are set, then runs `finish` --
+// inside the loop, so that a row another lane of the warp waits for is
+// stored without the warp having to leave the loop together.  Every lane of
+// the warp calls it (c < 0: no row).  false: gave up.
+template <class T, class F>
+__device__ __forceinline__ bool flow_wait(const T* ys, const int* __restrict__ col, int base, int c,
+                                          const int (&cj)[FLOW_U], T (&yv)[FLOW_U], int* err, F&& finish) {
+    bool fin = c < 0;
+#pragma unroll
+    for (int j = 0; j < FLOW_U; ++j)
+        if (j < c) yv[j] = ld_flow(ys + cj[j]);
+    for (int spins = 0;; ++spins) {
+        if (!fin) {
+            bool ready = true;
+#pragma unroll
+            for (int j = 0; j < FLOW_U; ++j)
+                if (j < c && flow_unset(yv[j])) ready = false;
+            for (int j = FLOW_U; ready && j < c; ++j)
+                ready = !flow_unset(ld_flow(ys + ld_stream(col + base + SELL_C * j)));
+            if (ready) {
+                finish();
+                fin = true;
+            }
+        }
+        if (__all_sync(0xffffffffu, fin)) return true;
+        if (spins > FLOW_SPIN_LIMIT || ((spins & 1023) == 1023 && *(volatile int*)err)) {
+            *(volatile int*)err = 1;
+            return false;
+        }
+        if (!fin) {
+#pragma unroll
+            for (int j = 0; j < FLOW_U; ++j)
+                if (j < c && flow_unset(yv[j])) yv[j] = ld_flow(ys + cj[j]);
+        }
+    }
+}
+
+// a block's next chunk of work, drawn from a counter that only grows: chunks
+// are handed out in order to blocks that run, so waiting on an earlier chunk
+// always ends
+__device__ __forceinline__ int flow_ticket(unsigned int* ticket, int* sh) {
+    __syncthreads();
+    if (threadIdx.x == 0) *sh = (int)atomicAdd(ticket, 1u);
+    __syncthreads();
+    return *sh;
+}
+
+// forward_substitution! (preconditioners_1_DILU.jl:84-98) of the warp's
+// positions k0 .. k0 + 31 of the lower level order into y (unset before);
+// marks out's rows unset for the backward rows
+template <class T>
+__device__ __forceinline__ bool flow_lower_rows(int n, const LevelView<T>& lo, const T* __restrict__ b, T* y, T* out,
+                                                int k0, int* err) {
+    const int k = k0 + (threadIdx.x & 31);
+    int i = 0, c = -1, base = 0;
+    int cj[FLOW_U];
+    T vj[FLOW_U], dj[FLOW_U], yv[FLOW_U];
+    T rhs = T(0);
+    if (k < n) {
+        i = lo.rows[k];
+        c = lo.cnt[k];
+        base = lo.slice[k / SELL_C] + (k % SELL_C);
+#pragma unroll
+        for (int j = 0; j < FLOW_U; ++j)
+            if (j < c) {
+                const int e = base + SELL_C * j;
+                cj[j] = ld_stream(lo.col + e);
+                vj[j] = ld_stream(lo.val + e);
+                dj[j] = ld_stream(lo.dinv + e);
+            }
+        rhs = b[i];
+        out[i] = flow_unset_value<T>();
+    }
+    return flow_wait((const T*)y, lo.col, base, c, cj, yv, err, [&] {
+        T sum = T(0);
+#pragma unroll
+        for (int j = 0; j < FLOW_U; ++j)
+            if (j < c) sum = sum + (vj[j] * yv[j]) * dj[j];
+        for (int j = FLOW_U; j < c; ++j) {
+            const int e = base + SELL_C * j;
+            sum = sum + (ld_stream(lo.val + e) * ld_flow(y + ld_stream(lo.col + e))) * ld_stream(lo.dinv + e);
+        }
+        st_flow(y + i, rhs - sum);
+    });
+}
+
+// backward_substitution! (preconditioners_1_DILU.jl:100-114) of the warp's
+// positions of the upper level order into out (unset before, its forward
+// values in y, which are marked unset again)
+template <class T>
+__device__ __forceinline__ bool flow_upper_rows(int n, const LevelView<T>& up, const T* __restrict__ D, T* y, T* out,
+                                                int k0, int* err) {
+    const int k = k0 + (threadIdx.x & 31);
+    int i = 0, c = -1, base = 0;
+    int cj[FLOW_U];
+    T vj[FLOW_U], yv[FLOW_U];
+    T yi = T(0), Di = T(0);
+    if (k < n) {
+        i = up.rows[k];
+        c = up.cnt[k];
+        base = up.slice[k / SELL_C] + (k % SELL_C);
+#pragma unroll
+        for (int j = 0; j < FLOW_U; ++j)
+            if (j < c) {
+                const int e = base + SELL_C * j;
+                cj[j] = ld_stream(up.col + e);
+                vj[j] = ld_stream(up.val + e);
+            }
+        yi = ld_flow(y + i);
+        Di = D[i];
+        y[i] = flow_unset_value<T>();
+    }
+    return flow_wait((const T*)out, up.col, base, c, cj, yv, err, [&] {
+        T sum = T(0);
+#pragma unroll
+        for (int j = 0; j < FLOW_U; ++j)
+            if (j < c) sum = sum + vj[j] * yv[j];
+        for (int j = FLOW_U; j < c; ++j) {
+            const int e = base + SELL_C * j;
+            sum = sum + ld_stream(up.val + e) * ld_flow((const T*)out + ld_stream(up.col + e));
+        }
+        st_flow(out + i, (yi - sum) / Di);
+    });
 }
 
 // update_dilu_diagonal! row i (preconditioners_1_DILU.jl:43-82)

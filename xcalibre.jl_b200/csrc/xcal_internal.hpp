@@ -140,9 +140,6 @@ struct MeshView {
 // reference's CSR order (ascending original column); padding entries (up to
 // the slice's longest row) are never read.
 constexpr int SELL_C = 32;
-// systems up to this many rows apply DILU (and build its factor) in one
-// block, level after level, instead of one launch per level
-constexpr int DILU_BLOCK_MAX_ROWS = 65536;
 // persistent CG, narrow form: prefetch a tile's matrix slots into L2 during
 // the second barrier when all slots (values + columns) take at most this many
 // bytes (measured: faster for a 74 MB matrix, slower for 117 and 175 MB)

@@ -276,6 +276,7 @@ struct Batch {
             B.S = S.p + i;
             B.part0 = c->ws.part0.p;
             B.part1 = c->ws.part1.p;
+            B.ring = c->ws.ring.p;
             if constexpr (sizeof(T) == 8) {
                 B.nz = (const T*)E.nz.p;
                 B.P = (const T*)E.P.p;
@@ -423,9 +424,26 @@ struct Batch {
             const int jac = pt == XCAL_PRECOND_JACOBI ? 1 : 0;
             int max_tiles = 0;
             for (int i : members) max_tiles = std::max(max_tiles, (cases[i]->U.n + RED_TILE - 1) / RED_TILE);
+            int slots = 0, halo = 0;  // of the members' pressure systems (0 slots: one has too many tiles)
+            for (int i : members) {
+                const CSRView A = (slot < 3 ? cases[i]->U : cases[i]->P).view();
+                slots = A.tile_slots > 0 && (slots > 0 || i == members[0]) ? std::max(slots, A.tile_slots) : 0;
+                halo = std::max(halo, A.tile_halo);
+            }
+            auto finished = [&](const char* what) {
+                int errflag = 0;
+                XCAL_CUDA(cudaMemcpyAsync(hS, S.p, cases.size() * sizeof(KScalars), cudaMemcpyDeviceToHost,
+                                          stream));
+                XCAL_CUDA(cudaMemcpyAsync(&errflag, perr.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+                sync();
+                if (errflag) fail(XCAL_ERR_TIMEOUT, what);
+                for (int i : members)
+                    if (!hS[i].done) fail(XCAL_ERR_TIMEOUT, "batch: persistent CG did not report completion");
+            };
             bool cluster = false;
             if (all_persist && (width == 0 || width == PERSIST_CLUSTER_ONLY) && max_tiles <= PERSIST_CLUSTER_MAX)
-                cluster = cluster_cg<T>(sy, members, jac, itmax + 1);
+                cluster = (width == 0 && slots > 0 && cluster_cg<T>(sy, members, slots, halo, jac, itmax + 1)) ||
+                          cluster_cg<T>(sy, members, 0, 0, jac, itmax + 1);
             if (cluster) {
                 XCAL_CUDA(cudaMemcpyAsync(hS, S.p, cases.size() * sizeof(KScalars), cudaMemcpyDeviceToHost,
                                           stream));
@@ -434,16 +452,14 @@ struct Batch {
                     if (!hS[i].done) fail(XCAL_ERR_TIMEOUT, "batch: persistent CG did not report completion");
                 return;
             }
+            if (all_persist && width == 0 &&
+                kb_cg_resident<T>(stream, sy, tm, nt, slots, halo, jac, perr.p, itmax + 1)) {
+                finished("batch: resident CG wait gave up");
+                return;
+            }
             if (all_persist && width != PERSIST_CLUSTER_ONLY &&
                 kb_cg_persist<T>(stream, sy, tm, nt, jac, bars.p, (int)cases.size(), perr.p, itmax + 1, width)) {
-                int errflag = 0;
-                XCAL_CUDA(cudaMemcpyAsync(hS, S.p, cases.size() * sizeof(KScalars), cudaMemcpyDeviceToHost,
-                                          stream));
-                XCAL_CUDA(cudaMemcpyAsync(&errflag, perr.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
-                sync();
-                if (errflag) fail(XCAL_ERR_TIMEOUT, "batch: persistent CG grid barrier wait gave up");
-                for (int i : members)
-                    if (!hS[i].done) fail(XCAL_ERR_TIMEOUT, "batch: persistent CG did not report completion");
+                finished("batch: persistent CG grid barrier wait gave up");
                 return;
             }
         }
@@ -477,10 +493,11 @@ struct Batch {
 
     // every member's CG in the cluster form, members grouped by the cluster
     // size they need (1, 2, 4, 8 or 16 blocks: a cluster per member), one
-    // launch per group, the groups on their own streams; false (nothing
-    // launched) when the device cannot run some group's cluster size
+    // launch per group, the groups on their own streams; slots > 0: the
+    // matrix-resident kernel; false (nothing launched) when the device cannot
+    // run some group's cluster size
     template <class T>
-    bool cluster_cg(const BSys<T>* sy, const std::vector<int>& members, int jac, int max_iters) {
+    bool cluster_cg(const BSys<T>* sy, const std::vector<int>& members, int slots, int halo, int jac, int max_iters) {
         std::vector<int> grp[5];
         for (int i : members) {
             const int t = (cases[i]->U.n + RED_TILE - 1) / RED_TILE;
@@ -489,7 +506,7 @@ struct Batch {
             grp[g].push_back(i);
         }
         for (int g = 0; g < 5; ++g)
-            if (!grp[g].empty() && persist_cluster_size(kb_cg_persist_cluster_kernel<T>(), 1 << g) != (1 << g))
+            if (!grp[g].empty() && kb_cg_cluster_size<T>(1 << g, slots, halo) != (1 << g))
                 return false;
         int off = 0;
         for (int g = 0; g < 5; ++g) {
@@ -501,7 +518,8 @@ struct Batch {
         for (int g = 0; g < 5; ++g) {
             if (grp[g].empty()) continue;
             XCAL_CUDA(cudaStreamWaitEvent(gstream[g], forked, 0));
-            kb_cg_persist_cluster<T>(gstream[g], sy, mem_ids.p + off, (int)grp[g].size(), 1 << g, jac, max_iters);
+            kb_cg_persist_cluster<T>(gstream[g], sy, mem_ids.p + off, (int)grp[g].size(), 1 << g, slots, halo, jac,
+                                     max_iters);
             XCAL_CUDA(cudaEventRecord(gjoined[g], gstream[g]));
             XCAL_CUDA(cudaStreamWaitEvent(stream, gjoined[g], 0));
             off += (int)grp[g].size();
@@ -779,6 +797,9 @@ size_t estimate_case_bytes(long nC, long nF, long nB, int mixed, int dilu_U, int
     // partials and small buffers
     b += nC * (26.0 + 9.0) * 8.0 + nF * 8.0 * 8.0 + (mixed ? 52.0 * nC + 16384.0 : 0.0);
     b += 3.0 * 8.0 * (nC / 2048 + 1) + 4096.0;
+    // resident CG: four buffers of a partial per tile and block
+    const double T = (nC + 2047) / 2048;
+    if (T <= RES_TILES_MAX) b += 32.0 * T * T;
     // permutations (mesh) and the field staging buffer (case)
     b += 8.0 * nC + 8.0 * nF + 8.0 * std::max(nC, nF);
     return (size_t)b;

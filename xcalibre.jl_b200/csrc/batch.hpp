@@ -37,6 +37,7 @@ struct BSys {
     KScalars* S;
     double* part0;
     double* part1;
+    double* ring;  // resident CG: 4 ntiles^2 doubles
     int n;
     int ntiles;
     // level-ordered triangles and the scratch of the DILU sweeps
@@ -117,15 +118,24 @@ void kb_cg_start(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int ntile
 template <class T>
 bool kb_cg_persist(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int ntiles_total, int jacobi,
                    unsigned int* bars, int nbars, int* err, int max_iters, int width = 0);
+// the resident form (cg_resident_body; slots, halo: the largest A.tile_slots
+// and A.tile_halo of the systems): every system in one cooperative launch
+// over the tile map; false (nothing launched) when the tiles exceed one per
+// SM or the slots shared memory
+template <class T>
+bool kb_cg_resident(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int ntiles_total, int slots, int halo,
+                    int jacobi, int* err, int max_iters);
 // the cluster form: every listed system (ids[0..nsys)) as one thread-block
-// cluster of the size its largest member needs; false (nothing launched)
-// when max_tiles exceeds PERSIST_CLUSTER_MAX or the device cannot run it
+// cluster of the size its largest member needs, with its matrix in shared
+// memory (slots > 0: as in kb_cg_resident) or not (slots 0); false (nothing
+// launched) when max_tiles exceeds PERSIST_CLUSTER_MAX or the device cannot
+// run it
 template <class T>
-bool kb_cg_persist_cluster(cudaStream_t s, const BSys<T>* sys, const int* ids, int nsys, int max_tiles, int jacobi,
-                           int max_iters);
-// the cluster-form kernel (for persist_cluster_size queries)
+bool kb_cg_persist_cluster(cudaStream_t s, const BSys<T>* sys, const int* ids, int nsys, int max_tiles, int slots,
+                           int halo, int jacobi, int max_iters);
+// the cluster size that launch would use (0: it cannot run)
 template <class T>
-const void* kb_cg_persist_cluster_kernel();
+int kb_cg_cluster_size(int tiles, int slots, int halo);
 template <class T>
 void kb_cg_spmv(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int ntiles_total);
 template <class T>

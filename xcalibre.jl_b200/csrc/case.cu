@@ -54,6 +54,8 @@ CSRView Equation::view() const {
     v.diag = d_diag.p;
     v.trans = d_trans.p;
     v.cf_slot = d_cf_slot.p;
+    v.tile_slots = tile_slots;
+    v.tile_halo = tile_halo;
     v.fslot = d_fslot.p;
     return v;
 }
@@ -475,6 +477,19 @@ void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& b
     }
     rows_s.clear();
     rows_s.shrink_to_fit();
+    constexpr int TILE = 2048;
+    E.tile_slots = E.tile_halo = 0;
+    for (int r0 = 0; r0 < n && n <= RES_TILES_MAX * TILE; r0 += TILE) {
+        const int r1 = std::min(n, r0 + TILE);
+        int halo = 0;
+        for (int r = r0; r < r1; ++r)
+            for (int k = 0; k < E.len[r]; ++k) {
+                const int c = E.colval[E.base(r) + SELL_C * k];
+                halo += c < r0 || c >= r1;
+            }
+        E.tile_slots = std::max(E.tile_slots, E.slice[(r1 + SELL_C - 1) / SELL_C] - E.slice[r0 / SELL_C]);
+        E.tile_halo = std::max(E.tile_halo, halo);
+    }
     E.diag.resize(n);
     for (int c = 0; c < n; ++c) E.diag[c] = E.find(c, c);
     std::vector<int> trans(E.nnz, 0), cf_slot(m.cf_face.size()), fslot(m.nI);
@@ -888,6 +903,7 @@ Case::Case(xcal_ctx* c, const DevMesh* m, const xcal_config* cf) : ctx(c), mesh(
     }
     ws.part0.alloc(T);
     ws.part1.alloc(T);
+    if (T <= RES_TILES_MAX) ws.ring.alloc(4L * T * T);
     ws.bar.alloc(2);
     ws.bar.zero(stream);
     ws.err.alloc(1);
@@ -1519,7 +1535,7 @@ void Case::krylov_start(Equation& E, const xcal_solver_setup& SS, const T* nz, c
     if (SS.solver == XCAL_SOLVER_CG) {
         T* zz = pt == XCAL_PRECOND_NONE ? V.r : V.z;
         if (pt != XCAL_PRECOND_NONE) apply_M(E, pt, nz, P, (const T*)V.r, zz, (const KScalars*)nullptr);
-        kr_cg_start(stream, n, (const T*)V.r, (const T*)zz, V.p, S, ws.part0.p);
+        kr_cg_start(stream, n, (const T*)V.r, (const T*)zz, V.p, S, ws.part0.p, ws.ring.p);
     } else {
         apply_M(E, pt, nz, P, r0, V.r, (const KScalars*)nullptr);
         kr_bicg_start(stream, n, c, (const T*)V.r, V.p, S, ws.part0.p, ws.part1.p);
@@ -1598,7 +1614,7 @@ void Case::krylov_iterate(Equation& E, const xcal_solver_setup& SS, const T* nz,
         if (profiling) XCAL_CUDA(cudaEventRecord(ev[5], stream));
         T* zz = pt == XCAL_PRECOND_NONE ? V.r : V.z;
         if (kr_cg_persist(stream, E.view(), nz, P, pt == XCAL_PRECOND_JACOBI ? 1 : 0, V.x, V.r, zz, V.p, V.v, S,
-                          ws.part0.p, ws.part1.p, ws.bar.p, ws.err.p, hS->itmax + 1,
+                          ws.part0.p, ws.part1.p, ws.ring.p, ws.bar.p, ws.err.p, hS->itmax + 1,
                           persistent_cg > 1 ? persistent_cg : 0,
                           E.nnz * (long)(sizeof(T) + 4) <= PERSIST_PF_MAX_BYTES ? 256 : 0)) {
             if (profiling) XCAL_CUDA(cudaEventRecord(ev[6], stream));
@@ -1785,7 +1801,7 @@ void Case::solve_captured(int eqn, int comp) {
         kr_init_resid(stream, A, E.nz.p, b, field, ws.dx.p, V.x, SS.solver == XCAL_SOLVER_CG ? V.r : V.q);
         krylov_start<double>(E, SS, E.nz.p, E.P.p, b, r0, V, S);
         const bool ran = persist && kr_cg_persist(stream, A, E.nz.p, E.P.p, jac, V.x, V.r, jac ? V.z : V.r, V.p, V.v,
-                                                  S, ws.part0.p, ws.part1.p, ws.bar.p, ws.err.p, itmax + 1, pwidth,
+                                                  S, ws.part0.p, ws.part1.p, ws.ring.p, ws.bar.p, ws.err.p, itmax + 1, pwidth,
                                                   E.nnz * 12L <= PERSIST_PF_MAX_BYTES ? 256 : 0, false);
         if (!ran)
             capture_while([&](cudaGraphConditionalHandle h) {
@@ -1825,7 +1841,7 @@ void Case::solve_captured(int eqn, int comp) {
             krylov_start<float>(E, SS, E.nz32.p, E.P32.p, (const float*)rhs, (const float*)rhs, V, S);
             const bool ran =
                 persist && kr_cg_persist(stream, A, E.nz32.p, E.P32.p, jac, V.x, V.r, jac ? V.z : V.r, V.p, V.v, S,
-                                         ws.part0.p, ws.part1.p, ws.bar.p, ws.err.p, itmax + 1, pwidth,
+                                         ws.part0.p, ws.part1.p, ws.ring.p, ws.bar.p, ws.err.p, itmax + 1, pwidth,
                                          E.nnz * 8L <= PERSIST_PF_MAX_BYTES ? 256 : 0, false);
             if (!ran)
                 capture_while([&](cudaGraphConditionalHandle hi) {

@@ -87,6 +87,7 @@ struct Equation {
     std::vector<unsigned char> len;
     DBuf<int> d_slice, d_colval, d_diag, d_trans, d_cf_slot, d_fslot;
     DBuf<unsigned char> d_len;
+    int tile_slots = 0, tile_halo = 0;  // CSRView: what the resident CG keeps per tile
     int base(int r) const { return slice[r / SELL_C] + r % SELL_C; }
     DBuf<double> nz, nz0, diag0, P;
     DBuf<float> nz32, P32;  // mixed precision: FP32 copies for the inner solves
@@ -142,6 +143,7 @@ struct BCTable {
 
 struct KrylovWS {
     DBuf<double> x, dx, r, z, p, q, v, s, t, part0, part1;
+    DBuf<double> ring;  // resident CG: four buffers of a partial per tile and block
     DBuf<float> fx, fr, fz, fp, fq, fv, fs, ft, fd;  // mixed precision inner vectors
     DBuf<double> fpart;  // folded inner CG: block partials (2 x FOLD_MAX_BLOCKS)
     DBuf<float2> frp;    // folded inner CG: two buffers of n (r, p_old) pairs

@@ -157,7 +157,7 @@ void kr_jacobi_apply(cudaStream_t s, int n, const T* P, const T* r, T* z, const 
 template <class T>
 void kr_copy(cudaStream_t s, int n, const T* a, T* b, const KScalars* S);
 template <class T>
-void kr_cg_start(cudaStream_t s, int n, const T* r, const T* z, T* p, KScalars* S, double* part);
+void kr_cg_start(cudaStream_t s, int n, const T* r, const T* z, T* p, KScalars* S, double* part, double* ring);
 // CG direction p_k lives in P0 (k even) / P1 (k odd); p_0 = z is stored in P0
 template <class T>
 void kr_cg_spmv(cudaStream_t s, const CSRView& A, const T* nz, const T* z, T* P0, T* P1, T* q, KScalars* S,
@@ -173,10 +173,13 @@ void kr_cg_rz(cudaStream_t s, int n, const T* r, const T* z, KScalars* S, double
 // bar: 2 words of barrier state, err: set when a barrier wait gave up.
 template <class T>
 bool kr_cg_persist(cudaStream_t s, const CSRView& A, const T* nz, const T* P, int jacobi, T* x, T* r, T* z, T* P0,
-                   T* P1, KScalars* S, double* part, double* part2, unsigned int* bar, int* err, int max_iters,
-                   int width = 0, int pf_kb = 0, bool reset_err = true);
-// width: 0 = the cluster form where the system has at most
-// PERSIST_CLUSTER_MAX tiles, else the widest cooperative form that fits;
+                   T* P1, KScalars* S, double* part, double* part2, double* ring, unsigned int* bar, int* err,
+                   int max_iters, int width = 0, int pf_kb = 0, bool reset_err = true);
+// ring: 4 ntiles^2 doubles (systems of at most RES_TILES_MAX tiles), set up by kr_cg_start
+// width: 0 = the resident form (cg_resident_body) where the system has at
+// most one tile per SM and its tiles' slots fit shared memory, else the
+// cluster form where it has at most PERSIST_CLUSTER_MAX tiles, else the
+// widest cooperative form that fits;
 // PERSIST_CLUSTER_ONLY = the cluster form only; 256 / 512 / 1024 = that
 // cooperative form only.  false: nothing launched (does not fit).
 constexpr int PERSIST_CLUSTER_ONLY = 2;
@@ -212,9 +215,14 @@ bool persist_launch(PersistCaps& c, int w, const void* kernel, int ntiles, cudaS
 // cluster size for `tiles`: the smallest power of two >= tiles that the
 // device schedules for this kernel, or 0 (too many tiles / not schedulable).
 constexpr int PERSIST_CLUSTER_MAX = 16;
-int persist_cluster_size(const void* kernel, int tiles);
+int persist_cluster_size(const void* kernel, int tiles, size_t smem = 0);
 // launch nclusters clusters of C blocks (one system each)
-void persist_cluster_launch(const void* kernel, int C, int nclusters, cudaStream_t s, void** args);
+void persist_cluster_launch(const void* kernel, int C, int nclusters, cudaStream_t s, void** args, size_t smem = 0);
+// Resident form: whether `kernel` (RES_THREADS threads a block) runs with
+// `smem` bytes of dynamic shared memory, and the device's SM count (0: not)
+int resident_sms(const void* kernel, size_t smem);
+// cooperative launch of the resident form over ntiles blocks
+void resident_launch(const void* kernel, int ntiles, size_t smem, cudaStream_t s, void** args);
 void kr_finish(cudaStream_t s, int n, const double* x, const double* dx, double* field);
 template <class T>
 void kr_bicg_start(cudaStream_t s, int n, const T* c, const T* r, T* p, KScalars* S, double* part0, double* part1);

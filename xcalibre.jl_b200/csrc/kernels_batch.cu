@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(FLOW_THREADS) kbk_dilu_flow(const BSys<T>* __r
 template <class T>
 __global__ void kbk_cg_start(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
-    cg_start_body<T>(tc, B.n, B.vec[KV_R], B.vec[KV_Z], B.vec[KV_P], B.S, B.part0);
+    cg_start_body<T>(tc, B.n, B.vec[KV_R], B.vec[KV_Z], B.vec[KV_P], B.S, B.part0, B.ring);
 }
 
 template <class T>
@@ -134,6 +134,31 @@ __global__ void __launch_bounds__(NT, persist_min_blocks(NT))
     XCAL_BSYS
     cg_persist_body<T, NT>(tc, B.A, B.nz, B.P, jacobi, B.vec[KV_X], B.vec[KV_R], B.vec[KV_Z], B.vec[KV_P],
                            B.vec[KV_V], B.S, B.part0, B.part1, bars + 2 * tm.x, err, max_iters, 0);
+}
+
+// every system's whole CG solve with its matrix in shared memory, one block
+// per tile of the batch
+template <class T>
+__global__ void __launch_bounds__(RES_THREADS, 1)
+    kbk_cg_resident(const BSys<T>* __restrict__ sys, const int2* tmap, int jacobi, int* err, int max_iters, int slots,
+                    int halo) {
+    extern __shared__ __align__(16) unsigned char res_smem[];
+    XCAL_BSYS
+    cg_resident_body<T, false>(tc, B.A, B.nz, B.P, jacobi, B.vec[KV_X], B.vec[KV_R], B.vec[KV_Z], B.vec[KV_P], B.S, B.ring,
+                        err, max_iters, slots, halo, res_smem);
+}
+
+// the same for systems of at most 16 tiles, each the blocks of one cluster
+template <class T>
+__global__ void __launch_bounds__(RES_THREADS, 1)
+    kbk_cg_resident_cl(const BSys<T>* __restrict__ sys, const int* __restrict__ ids, int C, int jacobi, int max_iters,
+                       int slots, int halo) {
+    extern __shared__ __align__(16) unsigned char res_smem[];
+    const BSys<T>& B = sys[ids[blockIdx.x / C]];
+    const TileCtx tc{(int)(blockIdx.x % C), B.ntiles};
+    if (tc.tile >= tc.ntiles) return;
+    cg_resident_body<T, true>(tc, B.A, B.nz, B.P, jacobi, B.vec[KV_X], B.vec[KV_R], B.vec[KV_Z], B.vec[KV_P], B.S,
+                              nullptr, nullptr, max_iters, slots, halo, res_smem);
 }
 
 // cluster form: system ids[b / C] is the cluster of blocks b (rank b % C)
@@ -359,16 +384,36 @@ bool kb_cg_persist(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int nti
     return persist_launch(caps, w, kern[w], ntiles_total, s, args);
 }
 template <class T>
-const void* kb_cg_persist_cluster_kernel() {
-    return (const void*)kbk_cg_persist_cl<T>;
+bool kb_cg_resident(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int ntiles_total, int slots, int halo,
+                    int jacobi, int* err, int max_iters) {
+    const void* k = (const void*)kbk_cg_resident<T>;
+    if (slots <= 0 || halo > RES_HALO_MAX) return false;
+    const size_t smem = res_smem_bytes<T>(slots, halo);
+    if (ntiles_total <= 0 || ntiles_total > resident_sms(k, smem)) return false;
+    XCAL_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+    void* args[] = {(void*)&sys, (void*)&tmap, &jacobi, &err, &max_iters, &slots, &halo};
+    resident_launch(k, ntiles_total, smem, s, args);
+    return true;
 }
 template <class T>
-bool kb_cg_persist_cluster(cudaStream_t s, const BSys<T>* sys, const int* ids, int nsys, int max_tiles, int jacobi,
-                           int max_iters) {
-    const void* k = (const void*)kbk_cg_persist_cl<T>;
-    const int C = persist_cluster_size(k, max_tiles);
+int kb_cg_cluster_size(int tiles, int slots, int halo) {
+    if (slots <= 0) return persist_cluster_size((const void*)kbk_cg_persist_cl<T>, tiles);
+    const size_t smem = res_smem_bytes<T>(slots, halo);
+    const void* k = (const void*)kbk_cg_resident_cl<T>;
+    return halo <= RES_HALO_MAX && resident_sms(k, smem) > 0 ? persist_cluster_size(k, tiles, smem) : 0;
+}
+template <class T>
+bool kb_cg_persist_cluster(cudaStream_t s, const BSys<T>* sys, const int* ids, int nsys, int max_tiles, int slots,
+                           int halo, int jacobi, int max_iters) {
+    const int C = kb_cg_cluster_size<T>(max_tiles, slots, halo);
     if (C == 0 || nsys <= 0) return false;
     int Cv = C;
+    if (slots > 0) {
+        void* args[] = {(void*)&sys, (void*)&ids, &Cv, &jacobi, &max_iters, &slots, &halo};
+        persist_cluster_launch((const void*)kbk_cg_resident_cl<T>, C, nsys, s, args, res_smem_bytes<T>(slots, halo));
+        return true;
+    }
+    const void* k = (const void*)kbk_cg_persist_cl<T>;
     void* args[] = {(void*)&sys, (void*)&ids, &Cv, &jacobi, &max_iters};
     persist_cluster_launch(k, C, nsys, s, args);
     return true;
@@ -422,8 +467,9 @@ void kb_bicg_p(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int ntiles_
     template void kb_cg_start<T>(cudaStream_t, const BSys<T>*, const int2*, int);                                  \
     template bool kb_cg_persist<T>(cudaStream_t, const BSys<T>*, const int2*, int, int, unsigned int*, int, int*,  \
                                    int, int);                                                                     \
-    template bool kb_cg_persist_cluster<T>(cudaStream_t, const BSys<T>*, const int*, int, int, int, int);          \
-    template const void* kb_cg_persist_cluster_kernel<T>();                                                         \
+    template bool kb_cg_resident<T>(cudaStream_t, const BSys<T>*, const int2*, int, int, int, int, int*, int);     \
+    template bool kb_cg_persist_cluster<T>(cudaStream_t, const BSys<T>*, const int*, int, int, int, int, int, int); \
+    template int kb_cg_cluster_size<T>(int, int, int);                                                             \
     template void kb_cg_spmv<T>(cudaStream_t, const BSys<T>*, const int2*, int);                                   \
     template void kb_cg_update<T>(cudaStream_t, const BSys<T>*, const int2*, int, int);                            \
     template void kb_cg_rz<T>(cudaStream_t, const BSys<T>*, const int2*, int);                                     \

@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <tuple>
 
 #include "kernels.hpp"
 #include "krylov_bodies.cuh"
@@ -109,8 +110,8 @@ __global__ void k_copy(int n, const T* __restrict__ a, T* b, const KScalars* S) 
 // p = z; gamma = <r,z>; initial stopping tests
 template <class T>
 __global__ void k_cg_start(int n, const T* __restrict__ r, const T* __restrict__ z, T* p, KScalars* S,
-                           double* part) {
-    cg_start_body<T>(grid_tiles(), n, r, z, p, S, part);
+                           double* part, double* ring) {
+    cg_start_body<T>(grid_tiles(), n, r, z, p, S, part, ring);
 }
 
 // q = A p_k; pAp = <p_k,q>; zero-curvature test; alpha = gamma / pAp
@@ -142,6 +143,29 @@ __global__ void __launch_bounds__(NT, persist_min_blocks(NT))
                  int pf_kb) {
     cg_persist_body<T, NT>(grid_tiles(), A, nz, Pj, jacobi, x, r, z, P0, P1, S, part, part2, bar, err, max_iters,
                            pf_kb);
+}
+
+// one block per tile, the tile's slots in dynamic shared memory
+// (cg_resident_body)
+template <class T>
+__global__ void __launch_bounds__(RES_THREADS, 1)
+    k_cg_resident(CSRView A, const T* __restrict__ nz, const T* __restrict__ Pj, int jacobi, T* x, const T* r, T* z,
+                  const T* p, KScalars* S, double* ring, int* err, int max_iters, int slots, int halo) {
+    extern __shared__ __align__(16) unsigned char res_smem[];
+    cg_resident_body<T, false>(grid_tiles(), A, nz, Pj, jacobi, x, r, z, p, S, ring, err, max_iters, slots, halo,
+                               res_smem);
+}
+
+// the same with the grid as one cluster, block b owning tile b
+template <class T>
+__global__ void __launch_bounds__(RES_THREADS, 1)
+    k_cg_resident_cl(CSRView A, const T* __restrict__ nz, const T* __restrict__ Pj, int jacobi, T* x, const T* r, T* z,
+                     const T* p, KScalars* S, int max_iters, int slots, int halo) {
+    extern __shared__ __align__(16) unsigned char res_smem[];
+    const TileCtx tc{(int)blockIdx.x, (A.n + RED_TILE - 1) / RED_TILE};
+    if (tc.tile >= tc.ntiles) return;
+    cg_resident_body<T, true>(tc, A, nz, Pj, jacobi, x, r, z, p, S, nullptr, nullptr, max_iters, slots, halo,
+                              res_smem);
 }
 
 // one block per SM, every G-th tile (cg_persist_mt_body); q in dynamic
@@ -815,8 +839,8 @@ void kr_copy(cudaStream_t s, int n, const T* a, T* b, const KScalars* S) {
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
-void kr_cg_start(cudaStream_t s, int n, const T* r, const T* z, T* p, KScalars* S, double* part) {
-    k_cg_start<T><<<TILE_LAUNCH(n), s>>>(n, r, z, p, S, part);
+void kr_cg_start(cudaStream_t s, int n, const T* r, const T* z, T* p, KScalars* S, double* part, double* ring) {
+    k_cg_start<T><<<TILE_LAUNCH(n), s>>>(n, r, z, p, S, part, ring);
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
@@ -869,15 +893,49 @@ bool persist_launch(PersistCaps& c, int w, const void* kernel, int ntiles, cudaS
     return true;
 }
 
-int persist_cluster_size(const void* kernel, int tiles) {
+int resident_sms(const void* kernel, size_t smem) {
+    if (smem > (size_t)RES_SMEM_MAX) return 0;
+    static std::mutex mu;
+    static std::map<const void*, int> sms;  // per kernel, one device type
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = sms.find(kernel);
+    if (it == sms.end()) {
+        int dev = 0, m = 0, per = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM_MAX) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, RES_THREADS, RES_SMEM_MAX) != cudaSuccess)
+            per = 0;
+        cudaGetLastError();
+        it = sms.emplace(kernel, per > 0 ? m : 0).first;
+    }
+    return it->second;
+}
+
+void resident_launch(const void* kernel, int ntiles, size_t smem, cudaStream_t s, void** args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ntiles);
+    cfg.blockDim = dim3(RES_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    XCAL_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+    XCAL_CHECK_LAUNCH();
+}
+
+int persist_cluster_size(const void* kernel, int tiles, size_t smem) {
     if (tiles <= 0 || tiles > PERSIST_CLUSTER_MAX) return 0;
     int C = 1;
     while (C < tiles) C *= 2;
     // schedulability per (kernel, C), found once
     static std::mutex mu;
-    static std::map<std::pair<const void*, int>, bool> ok;
+    static std::map<std::tuple<const void*, int, size_t>, bool> ok;
     std::lock_guard<std::mutex> lk(mu);
-    auto key = std::make_pair(kernel, C);
+    auto key = std::make_tuple(kernel, C, smem);
     auto it = ok.find(key);
     if (it == ok.end()) {
         bool good = true;
@@ -888,6 +946,7 @@ int persist_cluster_size(const void* kernel, int tiles) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(C);
             cfg.blockDim = dim3(1024);
+            cfg.dynamicSmemBytes = smem;
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeClusterDimension;
             at[0].val.clusterDim.x = C;
@@ -903,10 +962,11 @@ int persist_cluster_size(const void* kernel, int tiles) {
     return it->second ? C : 0;
 }
 
-void persist_cluster_launch(const void* kernel, int C, int nclusters, cudaStream_t s, void** args) {
+void persist_cluster_launch(const void* kernel, int C, int nclusters, cudaStream_t s, void** args, size_t smem) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C * nclusters);
     cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -921,12 +981,38 @@ void persist_cluster_launch(const void* kernel, int C, int nclusters, cudaStream
 
 template <class T>
 bool kr_cg_persist(cudaStream_t s, const CSRView& A, const T* nz, const T* P, int jacobi, T* x, T* r, T* z, T* P0,
-                   T* P1, KScalars* S, double* part, double* part2, unsigned int* bar, int* err, int max_iters,
-                   int width, int pf_kb, bool reset_err) {
+                   T* P1, KScalars* S, double* part, double* part2, double* ring, unsigned int* bar, int* err,
+                   int max_iters, int width, int pf_kb, bool reset_err) {
     static PersistCaps caps;  // co-resident blocks per width (per process, one device type)
     static const void* const kern[3] = {(const void*)k_cg_persist<T, 1024>, (const void*)k_cg_persist<T, 512>,
                                         (const void*)k_cg_persist<T, RED_THREADS>};
     const int nt = tiles(A.n);
+    // one tile per SM: the matrix stays in shared memory
+    if ((width == 0 || width == PERSIST_COOP_ONLY) && A.tile_slots > 0 && A.tile_halo <= RES_HALO_MAX) {
+        const void* kr = (const void*)k_cg_resident<T>;
+        int slots = A.tile_slots, halo = A.tile_halo;
+        const size_t smem = res_smem_bytes<T>(slots, halo);
+        const void* kc = (const void*)k_cg_resident_cl<T>;
+        if (width == 0 && nt <= PERSIST_CLUSTER_MAX && resident_sms(kc, smem) > 0) {
+            const int C = persist_cluster_size(kc, nt, smem);
+            if (C > 0) {
+                CSRView Av = A;
+                void* args[] = {&Av, (void*)&nz, (void*)&P, &jacobi, &x,     &r,
+                                &z,  &P0,        &S,        &max_iters, &slots, &halo};
+                if (reset_err) XCAL_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+                persist_cluster_launch(kc, C, 1, s, args, smem);
+                return true;
+            }
+        }
+        if (nt <= std::min(resident_sms(kr, smem), RES_TILES_MAX)) {
+            if (reset_err) XCAL_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+            CSRView Av = A;
+            void* args[] = {&Av, (void*)&nz, (void*)&P, &jacobi, &x,   &r,     &z,    &P0,
+                            &S,  &ring,      &err,      &max_iters, &slots, &halo};
+            resident_launch(kr, nt, smem, s, args);
+            return true;
+        }
+    }
     // the automatic choice past the one-tile-per-block forms: one block per
     // SM owning up to three tiles (measured on B200, FP64: 42.1 against 47.1
     // us per iteration at 432 tiles; at 1,024 tiles the narrow form is
@@ -941,7 +1027,7 @@ bool kr_cg_persist(cudaStream_t s, const CSRView& A, const T* nz, const T* P, in
             cudaGetLastError();
         }
         if (sms_auto > 0 && nt > 2 * sms_auto && nt <= 3 * sms_auto &&
-            kr_cg_persist(s, A, nz, P, jacobi, x, r, z, P0, P1, S, part, part2, bar, err, max_iters, PERSIST_MT1024,
+            kr_cg_persist(s, A, nz, P, jacobi, x, r, z, P0, P1, S, part, part2, ring, bar, err, max_iters, PERSIST_MT1024,
                           pf_kb, reset_err))
             return true;
     }
@@ -1297,14 +1383,15 @@ void kr_record(cudaStream_t s, const KScalars* S, int* out) {
                                     const KScalars*);                                                           \
     template void kr_jacobi_apply<T>(cudaStream_t, int, const T*, const T*, T*, const KScalars*);                \
     template void kr_copy<T>(cudaStream_t, int, const T*, T*, const KScalars*);                                  \
-    template void kr_cg_start<T>(cudaStream_t, int, const T*, const T*, T*, KScalars*, double*);                 \
+    template void kr_cg_start<T>(cudaStream_t, int, const T*, const T*, T*, KScalars*, double*, double*);        \
     template void kr_cg_spmv<T>(cudaStream_t, const CSRView&, const T*, const T*, T*, T*, T*, KScalars*,         \
                                 double*);                                                                       \
     template void kr_cg_update<T>(cudaStream_t, int, T*, const T*, const T*, T*, const T*, T*, const T*, int,    \
                                   KScalars*, double*);                                                          \
     template void kr_cg_rz<T>(cudaStream_t, int, const T*, const T*, KScalars*, double*);                        \
     template bool kr_cg_persist<T>(cudaStream_t, const CSRView&, const T*, const T*, int, T*, T*, T*, T*, T*,    \
-                                   KScalars*, double*, double*, unsigned int*, int*, int, int, int, bool);      \
+                                   KScalars*, double*, double*, double*, unsigned int*, int*, int, int, int,    \
+                                   bool);                                                                       \
     template void kr_bicg_start<T>(cudaStream_t, int, const T*, const T*, T*, KScalars*, double*, double*);      \
     template void kr_bicg_alpha<T>(cudaStream_t, int, const T*, const T*, KScalars*, double*);                   \
     template void kr_bicg_s<T>(cudaStream_t, int, const T*, const T*, const T*, T*, T*, const KScalars*);        \

@@ -134,9 +134,14 @@ __device__ __forceinline__ void cg_start_scalars(KScalars* S, double gamma) {
 
 template <class T>
 __device__ __forceinline__ void cg_start_body(const TileCtx& tc, int n, const T* __restrict__ r, const T* __restrict__ z, T* p, KScalars* S,
-                           double* part) {
+                           double* part, double* ring) {
     __shared__ double sm[8];
     double acc = 0.0;
+    // the resident CG's exchange buffers start unset (cg_resident_body)
+    if (tc.ntiles <= RES_TILES_MAX)
+        for (int k = threadIdx.x; k < 4 * tc.ntiles; k += blockDim.x)
+            ring[((size_t)(k / tc.ntiles) * tc.ntiles + tc.tile) * tc.ntiles + k % tc.ntiles] =
+                __longlong_as_double(-1LL);
     for (int k = 0; k < RED_ITEMS; ++k) {
         int i = tile_row(tc, k);
         if (i < n) {
@@ -591,6 +596,11 @@ __device__ __forceinline__ double ld_flow(const double* p) {
 __device__ __forceinline__ float ld_flow(const float* p) {
     float v;
     asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double ld_flow_acquire(const double* p) {
+    double v;
+    asm volatile("ld.acquire.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ bool flow_unset(double v) { return __double_as_longlong(v) == -1LL; }
@@ -1258,6 +1268,335 @@ __device__ __forceinline__ void cg_persist_mt_body(const CSRView& A, const T* __
         S->pNorm2 = pNorm2;
         S->alpha = alpha;
         S->rNorm = rNorm;
+    }
+}
+
+// ---- persistent CG with the matrix resident in shared memory ----
+// For systems of at most one canonical tile per SM.  The block of tile t
+// keeps the tile's slots (values, and columns as 16-bit local indices) in
+// shared memory for the whole solve, and x, r, z, p, q of its rows in
+// registers (1024 threads, two rows each), so an iteration touches L2 only
+// for the values other tiles own: the tile's halo, one entry per slot whose
+// column lies outside it.  Per iteration
+//   each thread forms p_k = z + beta p_{k-1} for its rows and its halo
+//   entries once (not once per slot), into shared memory;
+//   q = A p_k from shared memory; <p_k, q>;
+//   x += alpha p_k, r -= alpha q, z = P r; z published; <r, z>.
+// (A halo entry's p_{k-1} is what this thread formed for it in the last
+// iteration, so p is never published.)  The two reductions are also the
+// iteration's only synchronisation: a block writes its tile partial into its
+// column of every block's row of a buffer whose entries start unset
+// (flow_unset), and polls its own row -- one store-to-load latency where the
+// barrier forms paid an arrival, a poll and a second read, and no line that
+// every block polls (one shared row measured 1.5-3 us more per reduction at
+// 14-64 tiles).  Each reduction alternates between two buffers.  A block
+// leaves its row unset as it reads it; an entry is written again two
+// iterations later, by a block that has acquired this one's <r, z> in between,
+// whose release covers the reset and z.  <p, q> needs no release: its block has
+// written nothing since but its own rows' resets, and whoever overwrites the z
+// it read depends on the
+// partial those reads went into.  Arithmetic and
+// reduction trees are cg_persist_body's, so the results are the same bit for
+// bit.  Waits are bounded as in grid_barrier.
+//
+// What bounds it: shared-memory bandwidth of the slots (2048 rows x 7 slots x
+// 18 bytes and their bank conflicts, 1.2 us FP32, 2.4 us FP64) and the two
+// exchanges (1.2-1.5 us each in a cluster, 2.5-3.5 us through L2).  Measured
+// on B200, us per iteration, this against the forms without the matrix in
+// shared memory (FP64): 1,073 rows 4.0 / 7.0, 7,500 rows 6.1 / 11.2, 27,025
+// rows 7.7 / 12.2, 129,150 rows 8.7 / 13.2.
+constexpr int RES_THREADS = 1024;
+constexpr int RES_ROWS = RED_TILE / RES_THREADS;  // rows per thread
+constexpr int RES_HALO_PT = 4;                    // halo entries per thread
+constexpr int RES_HALO_MAX = RES_HALO_PT * RES_THREADS;
+constexpr int RES_SMEM_MAX = 226 * 1024;
+template <class T>
+__host__ __device__ constexpr size_t res_smem_bytes(int slots, int halo) {
+    // products (double per row), z, directions of rows and halo, values, local columns
+    return RED_TILE * sizeof(double) + RED_TILE * sizeof(T) + ((size_t)(RED_TILE + halo) * sizeof(T) + 15) / 16 * 16 +
+           ((size_t)slots * sizeof(T) + 15) / 16 * 16 + (size_t)slots * sizeof(unsigned short);
+}
+
+struct ResState {
+    double gamma, beta, pNorm2, alpha, rNorm;
+    int iter, done, status, stop;
+};
+
+// the tile's sum of the products in pr (cg_persist_body's order: thread v <
+// 256 adds rows v + 256 k in k order, then block_tree), in every lane of warp
+// 0; called by the whole block after the products are visible
+__device__ __forceinline__ double res_tile_sum(const double* pr, double* sm8) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < RED_THREADS) {
+        double acc = 0.0;
+#pragma unroll
+        for (int k = 0; k < RED_ITEMS; ++k) acc = acc + pr[k * RED_THREADS + threadIdx.x];
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, off);
+        if (lane == 0) sm8[warp] = acc;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    if (warp != 0) return 0.0;
+    return ((sm8[0] + sm8[4]) + (sm8[2] + sm8[6])) + ((sm8[1] + sm8[5]) + (sm8[3] + sm8[7]));
+}
+
+// reduce_partials over the ntiles <= 256 tiles, by warp 0 of every block: tot
+// is this block's partial, written into its column of every block's row of
+// buf; the block polls its own row and leaves it unset again (release: with
+// everything the block wrote before).  false: gave up.
+__device__ __forceinline__ bool res_exchange(double tot, const TileCtx& tc, double* buf, bool release, int* err,
+                                             double& sum) {
+    const int T = tc.ntiles, lane = threadIdx.x & 31;
+    if (T == 1) {
+        sum = 0.0 + tot;
+        return true;
+    }
+    if (release) __threadfence();
+    for (int t = lane; t < T; t += 32) st_flow(buf + (size_t)t * T + tc.tile, tot);
+    double* row = buf + (size_t)tc.tile * T;
+    // every entry in flight at once; acquire loads only where data was
+    // released (they cost 0.1-1 us more per exchange)
+    double w[8];
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = 32 * j + lane < T ? flow_unset_value<double>() : 0.0;
+    for (int spins = 0;; ++spins) {
+        bool all = true;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (flow_unset(w[j])) w[j] = release ? ld_flow_acquire(row + 32 * j + lane) : ld_flow(row + 32 * j + lane);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) all = all && !flow_unset(w[j]);
+        if (__all_sync(0xffffffffu, all)) break;
+        if (spins > FLOW_SPIN_LIMIT || ((spins & 1023) == 1023 && *(volatile int*)err)) {
+            ok = false;
+            break;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (32 * j + lane < T) {
+            row[32 * j + lane] = flow_unset_value<double>();
+            w[j] = 0.0 + w[j];
+        }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) {
+        if (lane == 0) *(volatile int*)err = 1;
+        return false;
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (32 * j < T) w[j] = w[j] + __shfl_xor_sync(0xffffffffu, w[j], off);
+    sum = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+    return true;
+}
+
+// the same among the blocks of one cluster (ntiles <= 16): the partial goes
+// into every block's shared memory (mine[0 .. ntiles) of each), a hardware
+// cluster barrier makes it and the blocks' z visible.  Called by every thread;
+// the sum is valid in warp 0.
+__device__ __forceinline__ double res_exchange_cl(double tot, const TileCtx& tc, double* mine) {
+    if (tc.ntiles == 1) return 0.0 + tot;
+    if (threadIdx.x < tc.ntiles)
+        *cooperative_groups::this_cluster().map_shared_rank(mine + tc.tile, threadIdx.x) = tot;
+    cooperative_groups::this_cluster().sync();
+    double w = 0.0;
+    if (threadIdx.x < 32) {
+        w = threadIdx.x < tc.ntiles ? 0.0 + mine[threadIdx.x] : 0.0;
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) w = w + __shfl_xor_sync(0xffffffffu, w, off);
+    }
+    return w + 0.0;  // block_tree's other seven warps hold zeros
+}
+
+// CL: the system's tiles are the blocks of one thread-block cluster; z and the
+// partials travel through distributed shared memory (a halo entry is read
+// from its owner's z), with no trip to L2 in an iteration.
+template <class T, bool CL>
+__device__ __forceinline__ void cg_resident_body(const TileCtx& tc, const CSRView& A, const T* __restrict__ nz,
+                                                 const T* __restrict__ Pj, int jacobi, T* x, const T* r, T* z, const T* pg,
+                                                 KScalars* S, double* ring, int* err, int max_iters, int slots,
+                                                 int halo, unsigned char* smem) {
+    __shared__ double sm8[8];
+    __shared__ ResState st;
+    __shared__ int sh_halo;
+    double* pr = reinterpret_cast<double*>(smem);
+    T* z_s = reinterpret_cast<T*>(smem + RED_TILE * sizeof(double));
+    T* dir = z_s + RED_TILE;
+    __shared__ double cl_part[2][16];
+    T* val = reinterpret_cast<T*>((unsigned char*)dir + ((size_t)(RED_TILE + halo) * sizeof(T) + 15) / 16 * 16);
+    unsigned short* idx =
+        reinterpret_cast<unsigned short*>((unsigned char*)val + ((size_t)slots * sizeof(T) + 15) / 16 * 16);
+    const int n = A.n, row0 = tc.tile * RED_TILE, e0 = A.slice[row0 / SELL_C];
+    if (threadIdx.x == 0) {
+        st = ResState{S->gamma, S->beta, S->pNorm2, S->alpha, S->rNorm, S->iter, S->done, S->status, 0};
+        sh_halo = 0;
+    }
+    __syncthreads();
+    if (st.done) return;  // the same in every block
+    const int itmax = S->itmax;
+    const double eps = S->eps;
+    const double epsT = sizeof(T) == 8 ? 2.220446049250313e-16 : 1.1920928955078125e-07;  // eps(T)
+    // the tile's slots and this thread's rows; halo columns listed in pr (as ints)
+    int* hcol = reinterpret_cast<int*>(pr);
+    int lb[RES_ROWS], ln[RES_ROWS];
+    T xi[RES_ROWS], ri[RES_ROWS], Pi[RES_ROWS], zi[RES_ROWS], pi[RES_ROWS], qi[RES_ROWS];
+#pragma unroll
+    for (int j = 0; j < RES_ROWS; ++j) {
+        const int i = row0 + j * RES_THREADS + threadIdx.x;
+        lb[j] = ln[j] = 0;
+        xi[j] = ri[j] = zi[j] = pi[j] = qi[j] = T(0);
+        Pi[j] = T(1);
+        if (i < n) {
+            const int b = row_base(A, i);
+            lb[j] = b - e0;
+            ln[j] = A.len[i];
+            for (int t = 0; t < ln[j]; ++t) {
+                const int c = ld_stream(A.colval + b + SELL_C * t);
+                int li = c - row0;
+                if (li < 0 || li >= RED_TILE) {
+                    const int h = atomicAdd(&sh_halo, 1);
+                    hcol[h] = c;
+                    li = RED_TILE + h;
+                }
+                idx[lb[j] + SELL_C * t] = (unsigned short)li;
+                val[lb[j] + SELL_C * t] = ld_stream(nz + b + SELL_C * t);
+            }
+            xi[j] = x[i];
+            ri[j] = r[i];
+            zi[j] = z[i];
+            pi[j] = pg[i];
+            if (jacobi) Pi[j] = Pj[i];
+        }
+    }
+    __syncthreads();
+    const int nh = sh_halo;
+    int hc[RES_HALO_PT];
+#pragma unroll
+    for (int u = 0; u < RES_HALO_PT; ++u) {
+        const int h = u * RES_THREADS + threadIdx.x;
+        hc[u] = h < nh ? hcol[h] : -1;
+    }
+    __syncthreads();
+    // every block of the cluster runs before any touches another's shared memory
+    if (CL && tc.ntiles > 1) cooperative_groups::this_cluster().sync();
+    // p_k of the halo and of this thread's rows (kaxpby!, cg_dir); the first
+    // direction is what cg_start left in pg
+    T hp[RES_HALO_PT];
+#pragma unroll
+    for (int u = 0; u < RES_HALO_PT; ++u) hp[u] = hc[u] >= 0 ? __ldcg(pg + hc[u]) : T(0);
+    for (int ran = 0; ran < max_iters; ++ran) {
+        if (ran > 0) {
+            const T b = (T)st.beta;
+            T hz[RES_HALO_PT];
+#pragma unroll
+            for (int u = 0; u < RES_HALO_PT; ++u)
+                if (hc[u] >= 0)
+                    hz[u] = CL ? *cooperative_groups::this_cluster().map_shared_rank(z_s + hc[u] % RED_TILE,
+                                                                                    hc[u] / RED_TILE)
+                               : __ldcg(z + hc[u]);
+#pragma unroll
+            for (int j = 0; j < RES_ROWS; ++j) pi[j] = zi[j] + b * pi[j];
+#pragma unroll
+            for (int u = 0; u < RES_HALO_PT; ++u)
+                if (hc[u] >= 0) hp[u] = hz[u] + b * hp[u];
+        }
+#pragma unroll
+        for (int j = 0; j < RES_ROWS; ++j) dir[j * RES_THREADS + threadIdx.x] = pi[j];
+#pragma unroll
+        for (int u = 0; u < RES_HALO_PT; ++u)
+            if (hc[u] >= 0) dir[RED_TILE + u * RES_THREADS + threadIdx.x] = hp[u];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < RES_ROWS; ++j) {
+            T q = T(0);
+            for (int t = 0; t < ln[j]; ++t) q = q + val[lb[j] + SELL_C * t] * dir[idx[lb[j] + SELL_C * t]];
+            qi[j] = q;
+            pr[j * RES_THREADS + threadIdx.x] = ln[j] ? (double)pi[j] * (double)q : 0.0;
+        }
+        __syncthreads();
+        double tot = res_tile_sum(pr, sm8);
+        double pAp = 0.0;
+        if constexpr (CL) pAp = res_exchange_cl(tot, tc, cl_part[0]);
+        if (threadIdx.x < 32) {
+            const bool ok = CL || res_exchange(tot, tc, ring + (size_t)(ran & 1) * tc.ntiles * tc.ntiles, false, err, pAp);
+            if (threadIdx.x == 0) {
+                const double lim = epsT * st.pNorm2;
+                if (!ok) {
+                    st.stop = 2;
+                } else if (pAp <= lim && fabs(pAp) <= lim) {
+                    st.stop = 1;
+                    st.done = 1;
+                    st.status = KS_ZERO_CURV;
+                } else {
+                    st.alpha = st.gamma / pAp;
+                }
+            }
+        }
+        __syncthreads();
+        if (st.stop) break;
+        const T a = (T)st.alpha;
+#pragma unroll
+        for (int j = 0; j < RES_ROWS; ++j) {
+            const int i = row0 + j * RES_THREADS + threadIdx.x;
+            xi[j] = xi[j] + a * pi[j];
+            ri[j] = ri[j] + (-a) * qi[j];
+            zi[j] = jacobi ? Pi[j] * ri[j] : ri[j];
+            if constexpr (CL)
+                z_s[j * RES_THREADS + threadIdx.x] = zi[j];
+            else if (tc.ntiles > 1 && i < n)
+                z[i] = zi[j];
+            pr[j * RES_THREADS + threadIdx.x] = ln[j] ? (double)ri[j] * (double)zi[j] : 0.0;
+        }
+        __syncthreads();
+        tot = res_tile_sum(pr, sm8);
+        double g = 0.0;
+        if constexpr (CL) g = res_exchange_cl(tot, tc, cl_part[1]);
+        if (threadIdx.x < 32) {
+            const bool ok =
+                CL || res_exchange(tot, tc, ring + (size_t)(2 + (ran & 1)) * tc.ntiles * tc.ntiles, true, err, g);
+            if (threadIdx.x == 0) {  // cg_finalize on the block's copy of the state
+                const double rn = sqrt(g);
+                const bool solved = (rn <= eps) || (rn + 1.0 <= 1.0);
+                st.rNorm = rn;
+                if (!solved) {
+                    const double bt = g / st.gamma;
+                    st.beta = bt;
+                    st.pNorm2 = g + (bt * bt) * st.pNorm2;
+                    st.gamma = g;
+                }
+                st.iter = st.iter + 1;
+                if (solved) {
+                    st.done = 1;
+                    st.status = KS_SOLVED;
+                } else if (st.iter >= itmax) {
+                    st.done = 1;
+                    st.status = KS_TIRED;
+                }
+                if (st.done) st.stop = 1;
+                if (!ok) st.stop = 2;
+            }
+        }
+        __syncthreads();
+        if (st.stop) break;
+    }
+    if (st.stop == 2) return;
+#pragma unroll
+    for (int j = 0; j < RES_ROWS; ++j) {
+        const int i = row0 + j * RES_THREADS + threadIdx.x;
+        if (i < n) x[i] = xi[j];
+    }
+    if (tc.tile == 0 && threadIdx.x == 0) {
+        S->iter = st.iter;
+        S->done = st.done;
+        S->status = st.status;
+        S->gamma = st.gamma;
+        S->beta = st.beta;
+        S->pNorm2 = st.pNorm2;
+        S->alpha = st.alpha;
+        S->rNorm = st.rNorm;
     }
 }
 

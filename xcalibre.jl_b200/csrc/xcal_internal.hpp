@@ -144,6 +144,8 @@ constexpr int SELL_C = 32;
 // the second barrier when all slots (values + columns) take at most this many
 // bytes (measured: faster for a 74 MB matrix, slower for 117 and 175 MB)
 constexpr long PERSIST_PF_MAX_BYTES = 80L << 20;
+// most tiles of a system the resident CG may take (one per SM)
+constexpr int RES_TILES_MAX = 256;
 struct CSRView {
     int n;
     const int* slice;          // [ceil(n/32)+1] first slot of each slice
@@ -153,6 +155,11 @@ struct CSRView {
     const int* trans;  // slot of (col,row) per entry
     const int* cf_slot;   // slot of (cell, neighbour) per cell-face entry
     const int* fslot;     // slot of (owner, neigh) per internal face (index f - nB)
+    // most slots, and most slots whose column lies outside the tile, of any
+    // reduction tile (2048 rows); 0 where the system has too many tiles for
+    // the resident CG
+    int tile_slots;
+    int tile_halo;
 };
 // slot of entry 0 of row r (entry k is at row_base + SELL_C*k)
 __host__ __device__ __forceinline__ int row_base(const CSRView& A, int r) {

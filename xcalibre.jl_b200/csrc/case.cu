@@ -1383,10 +1383,11 @@ void Case::relax_U(int comp) {
                       U.b[comp].p, mdot.p, nueff.p, Ucp, cfg.U_solver.relax, BCR_RELAX);
 }
 
-void Case::bc_relax_U(int comp) {
+void Case::bc_relax_U(int comp, double* diag_copy) {
     const double* Ucp[3] = {Uc[0].p, Uc[1].p, Uc[2].p};
     launch_bc_relax_U(stream, mv(), U.view(), bcU.view(), comp, cfg.U_schemes.divergence, U.nz.p, U.diag0.p,
-                      U.b[comp].p, mdot.p, nueff.p, Ucp, cfg.U_solver.relax, BCR_DIAG0 | BCR_BC | BCR_RELAX);
+                      U.b[comp].p, mdot.p, nueff.p, Ucp, cfg.U_solver.relax, BCR_DIAG0 | BCR_BC | BCR_RELAX,
+                      diag_copy);
 }
 
 void Case::set_reference() {
@@ -1711,8 +1712,7 @@ void Case::krylov_iterate(Equation& E, const xcal_solver_setup& SS, const T* nz,
 // Add a conditional WHILE node at the current point of the capture running on
 // `stream`; body(h) launches the loop body (captured into the node's body
 // graph on a side stream) and must end with a kernel that sets h.
-template <class F>
-void Case::capture_while(F&& body) {
+void Case::capture_while(const std::function<void(cudaGraphConditionalHandle)>& body) {
     if (side_depth >= 2) fail(XCAL_ERR_INVALID, "graph mode: WHILE loops nest at most two deep");
     cudaStreamCaptureStatus st;
     cudaGraph_t g = nullptr;
@@ -1901,6 +1901,18 @@ Case::SolveRef Case::solve_ref(int eqn, int comp) {
 
 // solve_system! (Solve_1_api.jl:268-307)
 double Case::solve_system(int eqn, int comp, int* iters) {
+    {
+        const SolveRef R = solve_ref(eqn, comp);
+        if (use_fused(*R.E, R.SS)) {
+            double res = 0.0;
+            if (cfg.precision == XCAL_PREC_MIXED)
+                fused_solve<float, 1>(*R.E, R.SS, &R, &res);
+            else
+                fused_solve<double, 1>(*R.E, R.SS, &R, &res);
+            if (iters) *iters = last_iters[R.gk];
+            return res;
+        }
+    }
     smooth(eqn, comp);
     if (capturing) {  // graph mode: residual goes to gres
         solve_captured(eqn, comp);
@@ -2054,6 +2066,20 @@ void Case::solve_mixed(Equation& E, const xcal_solver_setup& SS, double* field, 
 
 void Case::solve_equation_U(double res[3]) {  // Solve_1_api.jl:233-266
     discretise(XCAL_EQN_U);
+    reserve_fused();
+    if (bf.ready && use_fused(U, cfg.U_solver) && components_apart()) {
+        SolveRef R[3];
+        for (int d = 0; d < 3; ++d) {
+            bc_relax_U(d, bf.diag.p + (size_t)d * U.n);
+            if (d == 0) update_precond(XCAL_EQN_U);
+            R[d] = solve_ref(XCAL_EQN_U, d);
+        }
+        if (cfg.precision == XCAL_PREC_MIXED)
+            fused_solve<float, 3>(U, cfg.U_solver, R, res);
+        else
+            fused_solve<double, 3>(U, cfg.U_solver, R, res);
+        return;
+    }
     for (int d = 0; d < 3; ++d) {
         bc_relax_U(d);
         if (d == 0) update_precond(XCAL_EQN_U);
@@ -2348,6 +2374,7 @@ void Case::piso_body(double r3[3], double& rp) {
 void Case::capture_step() {
     if (step_graph) return;
     autotune();
+    reserve_fused();
     sync();
     const long long t0 = t_launch_count;
     body_kernels_captured = 0;

@@ -1,5 +1,6 @@
 // case.hpp -- host objects behind the C ABI handles.
 #pragma once
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -158,6 +159,11 @@ struct KrylovVecs {
     T *x, *r, *z, *p, *q, *v, *s, *t;
 };
 
+// the systems of a fused BiCGSTAB solve (bicg_fused.cu)
+template <class T, int NC>
+struct BfView;
+constexpr int BF_MAX_ROWS = 524288;  // largest fused system
+
 struct Case {
     xcal_ctx* ctx = nullptr;
     const DevMesh* mesh = nullptr;
@@ -261,7 +267,7 @@ struct Case {
     void discretise(int eqn);
     void apply_bcs(int eqn, int comp);
     void relax_U(int comp);
-    void bc_relax_U(int comp);
+    void bc_relax_U(int comp, double* diag_copy = nullptr);
     void set_reference();
     void update_precond(int eqn);
     double solve_system(int eqn, int comp, int* iters);
@@ -322,6 +328,28 @@ struct Case {
     void dilu_refresh(Equation& E, bool fp32, bool cg);
     template <class T>
     T* flow_scratch(const T* out);
+    // BiCGSTAB of the three momentum components side by side, or of one scalar
+    // with fewer launches (bicg_fused.cu)
+    struct Fused {
+        bool ready = false;
+        DBuf<double> diag, dx, vec, part0, part1, res;  // diagonals of the components; vectors of components 1, 2
+        DBuf<float> diag32, vec32;
+        DBuf<KScalars> S;
+        KScalars* hS = nullptr;  // pinned
+        double* hres = nullptr;  // pinned
+        ~Fused() {
+            if (hS) cudaFreeHost(hS);
+            if (hres) cudaFreeHost(hres);
+        }
+    } bf;
+    int apart = -1;  // components_apart(), once known
+    bool use_fused(const Equation& E, const xcal_solver_setup& SS);
+    bool components_apart();
+    void reserve_fused();
+    template <class T, int NC>
+    BfView<T, NC> bf_view(Equation& E, const xcal_solver_setup& SS, const SolveRef* R);
+    template <class T, int NC>
+    void fused_solve(Equation& E, const xcal_solver_setup& SS, const SolveRef* R, double* res);
     // where the dataflow kernels report a wait that gave up: the case's own
     // flag, or the batch's while the case is resident in one
     int* batch_err = nullptr;
@@ -365,8 +393,7 @@ struct Case {
     void piso_body(double r3[3], double& rp);
     void set_graph_mode(bool on);
     void courant_to_slot();
-    template <class F>
-    void capture_while(F&& body);
+    void capture_while(const std::function<void(cudaGraphConditionalHandle)>& body);
     void solve_captured(int eqn, int comp);
     template <class T>
     void krylov_start(Equation& E, const xcal_solver_setup& SS, const T* nz, const T* P, const T* c, const T* r0,

@@ -16,7 +16,8 @@ void launch_assemble_p(cudaStream_t s, const MeshView& m, const CSRView& A, cons
                        double* nz, double* b);
 void launch_bc_relax_U(cudaStream_t s, const MeshView& m, const CSRView& A, const BCView& bc, int comp,
                        int div_scheme, double* nz, const double* diag0, double* b, const double* mdot,
-                       const double* nueff, const double* const U[3], double alpha, int flags);
+                       const double* nueff, const double* const U[3], double alpha, int flags,
+                       double* diag_copy = nullptr);  // the relaxed diagonal, once more
 void launch_bc_p(cudaStream_t s, const MeshView& m, const CSRView& A, const BCView& bc, double* nz, double* b,
                  const double* rDf, const double* p);
 void launch_set_reference(cudaStream_t s, const CSRView& A, double* nz, double* b, double pref, int row);

@@ -284,7 +284,7 @@ __global__ void k_bc_relax_U(MeshView m, CSRView A, BCView bc, int comp, int div
                              const double* __restrict__ diag0, double* b, const double* __restrict__ mdot,
                              const double* __restrict__ nueff, const double* __restrict__ Ux,
                              const double* __restrict__ Uy, const double* __restrict__ Uz, double alpha,
-                             int flags) {
+                             int flags, double* diag_copy) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.nC) return;
     int ds = A.diag[i];
@@ -342,6 +342,7 @@ __global__ void k_bc_relax_U(MeshView m, CSRView A, BCView bc, int comp, int div
     double D0 = d;
     double Dmax = jl_max(fabs(D0), sumv) / alpha;
     nz[ds] = Dmax;
+    if (diag_copy) diag_copy[i] = Dmax;
     const double* U = comp == 0 ? Ux : (comp == 1 ? Uy : Uz);
     b[i] = bi + (Dmax - D0) * U[i];
 }
@@ -1455,9 +1456,9 @@ void launch_assemble_p(cudaStream_t s, const MeshView& m, const CSRView& A, cons
 }
 void launch_bc_relax_U(cudaStream_t s, const MeshView& m, const CSRView& A, const BCView& bc, int comp,
                        int div_scheme, double* nz, const double* diag0, double* b, const double* mdot,
-                       const double* nueff, const double* const U[3], double alpha, int flags) {
+                       const double* nueff, const double* const U[3], double alpha, int flags, double* diag_copy) {
     k_bc_relax_U<<<nblk(m.nC), TPB, 0, s>>>(m, A, bc, comp, div_scheme, nz, diag0, b, mdot, nueff, U[0], U[1], U[2],
-                                            alpha, flags);
+                                            alpha, flags, diag_copy);
     XCAL_CHECK_LAUNCH();
 }
 void launch_bc_p(cudaStream_t s, const MeshView& m, const CSRView& A, const BCView& bc, double* nz, double* b,

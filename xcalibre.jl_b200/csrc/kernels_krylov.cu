@@ -600,14 +600,7 @@ __global__ void __launch_bounds__(RED_THREADS, 8) k_residual(CSRView A, const do
     if (!last_block(&S->counter2)) return;
     double sR = reduce_partials(part0, gridDim.x, sm);
     double sb = reduce_partials(part1, gridDim.x, sm);
-    if (threadIdx.x == 0) {
-        double normb = sqrt(sb);
-        double denom = normb > jl_eps(normb) ? normb : 1.0;
-        double res = sqrt(sR) / denom;
-        S->resid = res;
-        S->normb = normb;
-        if (out) *out = res;
-    }
+    if (threadIdx.x == 0) residual_scalars(S, sR, sb, out);
 }
 
 // ---------------------------------------------------------------------------

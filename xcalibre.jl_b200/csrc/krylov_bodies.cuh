@@ -288,6 +288,76 @@ __device__ __forceinline__ void cg_rz_body(const TileCtx& tc, int n, const T* __
     if (threadIdx.x == 0) cg_finalize(S, g);
 }
 
+// BiCGSTAB's scalar decisions (Krylov.jl bicgstab!), taken by one thread once
+// a reduction is complete.  The start, from ||r||^2 and <c, r>:
+__device__ __forceinline__ void bicg_start_scalars(KScalars* S, double rr, double cr) {
+    double rNorm = sqrt(rr);
+    S->rNorm = rNorm;
+    S->rNorm0 = rNorm;
+    S->iter = 0;
+    S->done = 0;
+    S->status = KS_RUNNING;
+    S->outer_conv = 0;
+    S->loops = 0;
+    if (rNorm == 0.0) {
+        S->done = 1;
+        S->status = KS_ZERO_RHS;
+        S->outer_conv = 1;
+        return;
+    }
+    start_eps(S, rNorm);
+    S->next_rho = cr;
+    if (cr == 0.0) {
+        S->done = 1;
+        S->status = KS_BREAKDOWN;
+        return;
+    }
+    if (rNorm <= S->eps) {
+        S->done = 1;
+        S->status = KS_SOLVED;
+    } else if (S->iter >= S->itmax) {
+        S->done = 1;
+        S->status = KS_TIRED;
+    }
+}
+// alpha = rho / <c, v> (the iteration counter advances)
+__device__ __forceinline__ void bicg_alpha_scalars(KScalars* S, double cv) {
+    S->iter = S->iter + 1;
+    S->rho = S->next_rho;
+    S->cv = cv;
+    S->alpha = S->rho / cv;
+}
+// beta and the stopping tests, from <c, r> and ||r||^2 of the new residual
+__device__ __forceinline__ void bicg_xr_scalars(KScalars* S, double omega, double cr, double rr) {
+    S->next_rho = cr;
+    S->beta = (cr / S->rho) * (S->alpha / omega);
+    double rNorm = sqrt(rr);
+    S->rNorm = rNorm;
+    bool mach = (rNorm + 1.0 <= 1.0);
+    bool solved = (rNorm <= S->eps) || mach;
+    bool tired = S->iter >= S->itmax;
+    bool breakdown = (S->alpha == 0.0) || isnan(S->alpha);
+    if (solved) {
+        S->done = 1;
+        S->status = KS_SOLVED;
+    } else if (tired) {
+        S->done = 1;
+        S->status = KS_TIRED;
+    } else if (breakdown) {
+        S->done = 1;
+        S->status = KS_BREAKDOWN;
+    }
+}
+// the scaled residual (Solve_1_api.jl:441-464) from ||b - A x||^2 and ||b||^2
+__device__ __forceinline__ void residual_scalars(KScalars* S, double sR, double sb, double* out) {
+    double normb = sqrt(sb);
+    double denom = normb > jl_eps(normb) ? normb : 1.0;
+    double res = sqrt(sR) / denom;
+    S->resid = res;
+    S->normb = normb;
+    if (out) *out = res;
+}
+
 template <class T>
 __device__ __forceinline__ void bicg_start_body(const TileCtx& tc, int n, const T* __restrict__ c, const T* __restrict__ r, T* p, KScalars* S,
                              double* part0, double* part1) {
@@ -311,36 +381,7 @@ __device__ __forceinline__ void bicg_start_body(const TileCtx& tc, int n, const 
     if (!last_block(&S->counter, tc.ntiles)) return;
     double rr = reduce_partials(part0, tc.ntiles, sm);
     double cr = reduce_partials(part1, tc.ntiles, sm);
-    if (threadIdx.x == 0) {
-        double rNorm = sqrt(rr);
-        S->rNorm = rNorm;
-        S->rNorm0 = rNorm;
-        S->iter = 0;
-        S->done = 0;
-        S->status = KS_RUNNING;
-        S->outer_conv = 0;
-        S->loops = 0;
-        if (rNorm == 0.0) {
-            S->done = 1;
-            S->status = KS_ZERO_RHS;
-            S->outer_conv = 1;
-            return;
-        }
-        start_eps(S, rNorm);
-        S->next_rho = cr;
-        if (cr == 0.0) {
-            S->done = 1;
-            S->status = KS_BREAKDOWN;
-            return;
-        }
-        if (rNorm <= S->eps) {
-            S->done = 1;
-            S->status = KS_SOLVED;
-        } else if (S->iter >= S->itmax) {
-            S->done = 1;
-            S->status = KS_TIRED;
-        }
-    }
+    if (threadIdx.x == 0) bicg_start_scalars(S, rr, cr);
 }
 
 template <class T>
@@ -356,12 +397,7 @@ __device__ __forceinline__ void bicg_alpha_body(const TileCtx& tc, int n, const 
     if (threadIdx.x == 0) part[tc.tile] = tot;
     if (!last_block(&S->counter, tc.ntiles)) return;
     double cv = reduce_partials(part, tc.ntiles, sm);
-    if (threadIdx.x == 0) {
-        S->iter = S->iter + 1;
-        S->rho = S->next_rho;
-        S->cv = cv;
-        S->alpha = S->rho / cv;
-    }
+    if (threadIdx.x == 0) bicg_alpha_scalars(S, cv);
 }
 
 template <class T>
@@ -432,26 +468,7 @@ __device__ __forceinline__ void bicg_xr_body(const TileCtx& tc, int n, T* x, con
     if (!last_block(&S->counter, tc.ntiles)) return;
     double cr = reduce_partials(part0, tc.ntiles, sm);
     double rr = reduce_partials(part1, tc.ntiles, sm);
-    if (threadIdx.x == 0) {
-        S->next_rho = cr;
-        S->beta = (cr / S->rho) * (S->alpha / omega);
-        double rNorm = sqrt(rr);
-        S->rNorm = rNorm;
-        bool mach = (rNorm + 1.0 <= 1.0);
-        bool solved = (rNorm <= S->eps) || mach;
-        bool tired = S->iter >= S->itmax;
-        bool breakdown = (S->alpha == 0.0) || isnan(S->alpha);
-        if (solved) {
-            S->done = 1;
-            S->status = KS_SOLVED;
-        } else if (tired) {
-            S->done = 1;
-            S->status = KS_TIRED;
-        } else if (breakdown) {
-            S->done = 1;
-            S->status = KS_BREAKDOWN;
-        }
-    }
+    if (threadIdx.x == 0) bicg_xr_scalars(S, omega, cr, rr);
 }
 
 template <class T>

@@ -873,7 +873,7 @@ void Case::fused_solve(Equation& E, const xcal_solver_setup& SS, const SolveRef*
     for (int d = 0; d < NC; ++d) {
         const int gk = R[d].gk;
         last_iters[gk] = total[d];
-        if (mixed && gk < 7) last_outer[gk] = outers[d];
+        if (mixed) last_outer[gk] = outers[d];
         note_status(gk, status[d]);
     }
 }

@@ -254,8 +254,8 @@ struct Case {
         cudaGraphExec_t exec = nullptr;
         long long launches = 0;  // kernels per replay
     };
-    ChunkGraph chunk_graph[7][2];  // [Ux, Uy, Uz, p, k, omega, wall distance][plain, profiled]
-    cudaEvent_t gev[7][12] = {};   // event nodes of the profiled graphs
+    ChunkGraph chunk_graph[8][2];  // [Ux, Uy, Uz, p, k, omega, wall distance, kl][plain, profiled]
+    cudaEvent_t gev[8][12] = {};   // event nodes of the profiled graphs
     template <class F>
     void replay_chunk(ChunkGraph& g, F&& body);
 
@@ -364,7 +364,7 @@ struct Case {
     // scaled defect in V.r (host-polled; field corrected by the kernel)
     bool use_fold(const Equation& E, const xcal_solver_setup& SS, bool captured) const;
     void fold_iterate(Equation& E, double* field, const KrylovVecs<float>& V, KScalars* S, KScalars* hS, int gk);
-    int last_outer[7] = {0, 0, 0, 0, 0, 0, 0};  // mixed: defect-correction steps of the last solve per system
+    int last_outer[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // mixed: defect-correction steps of the last solve per system
     bool tuned = false;
     void autotune();  // launch-shape autotuner (autotune.cu), once per case
 

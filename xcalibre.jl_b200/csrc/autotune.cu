@@ -4,11 +4,9 @@
 //  * the row mapping and block size of the SpMVs that carry no reduction
 //    (the BiCGSTAB SpMV): the canonical tile kernel or 1/2/4 rows per thread
 //    in blocks of 128/256/512 threads;
-//  * how a DILU application runs: rows waiting for the values they read
-//    (dataflow), or, where that may lose, one block sweeping every level
-//    (systems of up to 4,096 rows), one launch per level, or every level in
-//    one cooperative launch with a grid barrier between levels (systems of
-//    more than 524,288 rows).
+//  * how a DILU application of a system of more than 524,288 rows runs: rows
+//    waiting for the values they read (dataflow), one launch per level, or
+//    every level in one cooperative launch with a grid barrier between levels.
 // Each candidate is timed with CUDA events on the case's own matrix at first
 // use; choices are cached per size class (value size, log2 rows, entries per
 // row), so later cases of the same class reuse them without timing.
@@ -67,13 +65,14 @@ static SpmvShape tune_spmv(Case& C, Equation& E, const T* nz, const T* x, T* y) 
     return best;
 }
 
-// the fastest DILU form on this system: 1 one-block sweeps, 2 one launch per
-// level, 3 one cooperative launch over every level, 4 dataflow.  Candidates by
-// size (measured on B200, us per application, dataflow against the best other
-// form): the one-block sweeps come within reach only below some 4k rows
-// (1,518 rows FP32: 20.3 / 18.6; 3,700 rows: 31.1 / 31.6; 6,400 rows FP64:
-// 26.7 / 43.3), the level forms only above 0.5M (884,736 rows FP32: 117 / 155;
-// 2.1M rows: 233 / 192, FP64 283 / 252)
+// the fastest DILU form on this system: 2 one launch per level, 3 one
+// cooperative launch over every level, 4 dataflow.  Up to 524,288 rows dataflow
+// is taken as it is: measured on B200 (us per application, dataflow against
+// the best other form) 27,025 rows FP64 37 / 88, 262,144 rows FP32 61 / 131;
+// one-block sweeps come within reach only below some 4k rows (1,518 rows FP32
+// 20.3 / 18.6), where the fused BiCGSTAB then shares one sweep among three
+// components.  Above, both are timed (884,736 rows FP32: 117 / 155; 2.1M rows:
+// 233 / 192, FP64 283 / 252).
 template <class T>
 static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, T* out) {
     const int reps = (int)std::max(3L, std::min(20L, 20000000L / std::max(E.nnz_csr, 1L)));
@@ -81,11 +80,9 @@ static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, 
     kr_flow_unset(C.stream, C.flow_scratch<T>(out), (size_t)E.n * sizeof(T));
     int best = 4;
     float best_ms = 1e30f;
-    if (E.n > 4096 && E.n <= 524288) return best;
-    for (int form = 1; form <= 4; ++form) {
-        if (form == 1 && E.n > 4096) continue;
-        if ((form == 2 || form == 3) && E.n <= 524288) continue;
-        E.use_block = form == 1;
+    if (E.n <= 524288) return best;
+    for (int form = 2; form <= 4; ++form) {
+        E.use_block = false;
         E.use_grid = form == 3;
         E.use_flow = form == 4;
         float ms = time_ms(C.stream, C.ev[6], C.ev[7], reps, [&] { C.dilu_ldiv(E, nz, D, b, out, nullptr); });

@@ -38,33 +38,27 @@ constexpr int FOLD_SMEM_MAX = 220 * 1024;
 
 // rp[i].x = r_i = (float)(sqrt(P_i) (b_i - sum_j a_ij field_j)) -- the
 // scaled FP64 defect (row sums in the row's CSR order, FP64)
-__global__ void __launch_bounds__(RED_THREADS, 8) k_fold_defect(CSRView A, const double* __restrict__ nz,
-                                                             const double* __restrict__ b,
-                                                             const double* __restrict__ field,
-                                                             const double* __restrict__ P, float2* rp) {
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(k);
-        if (i < A.n) rp[i].x = (float)(sqrt(P[i]) * (b[i] - row_dot(A, nz, field, i)));
-    }
+__global__ void __launch_bounds__(256) k_fold_defect(CSRView A, const double* __restrict__ nz,
+                                                     const double* __restrict__ b, const double* __restrict__ field,
+                                                     const double* __restrict__ P, float2* rp) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < A.n) rp[i].x = (float)(sqrt(P[i]) * (b[i] - row_dot8(A, nz, field, i)));
 }
 
 // start of the inner solve: gamma = <r, r> over rp[].x (canonical tile
 // tree, the last block finishing), then cg!'s start tests (cg_start_scalars)
-__global__ void __launch_bounds__(RED_THREADS) k_fold_start(int n, const float2* __restrict__ rp, KScalars* S,
-                                                            double* part) {
-    __shared__ double sm[8];
-    double acc = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        const int i = tile_row(k);
-        if (i < n) {
-            const double ri = (double)rp[i].x;
-            acc = acc + ri * ri;
-        }
-    }
-    const double tot = block_tree(acc, sm);
-    if (threadIdx.x == 0) part[blockIdx.x] = tot;
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_fold_start(int n, const float2* __restrict__ rp,
+                                                                        KScalars* S, double* part) {
+    __shared__ TileSmem<NT, 1> sh;
+    double tot[1];
+    tile_reduce<NT, 1>(grid_tiles(), n, sh, tot, [&](int i, double* v) {
+        const double ri = (double)rp[i].x;
+        v[0] = ri * ri;
+    });
+    if (threadIdx.x == 0) part[blockIdx.x] = tot[0];
     if (!last_block(&S->counter)) return;
-    const double gamma = reduce_partials(part, (int)gridDim.x, sm);
+    const double gamma = reduce_partials(part, (int)gridDim.x, sh.sm);
     if (threadIdx.x == 0) cg_start_scalars(S, gamma);
 }
 
@@ -335,12 +329,16 @@ __global__ void __launch_bounds__(NT, 1)
 
 void kr_fold_defect(cudaStream_t s, const CSRView& A, const double* nz, const double* b, const double* field,
                     const double* P, float2* rp) {
-    k_fold_defect<<<(A.n + RED_TILE - 1) / RED_TILE, RED_THREADS, 0, s>>>(A, nz, b, field, P, rp);
+    k_fold_defect<<<(A.n + 255) / 256, 256, 0, s>>>(A, nz, b, field, P, rp);
     XCAL_CHECK_LAUNCH();
 }
 
 void kr_fold_start(cudaStream_t s, int n, const float2* rp, KScalars* S, double* part) {
-    k_fold_start<<<(n + RED_TILE - 1) / RED_TILE, RED_THREADS, 0, s>>>(n, rp, S, part);
+    const int nt = (n + RED_TILE - 1) / RED_TILE;
+    if (nt <= WIDE_TILES)
+        k_fold_start<WIDE_NT><<<nt, WIDE_NT, 0, s>>>(n, rp, S, part);
+    else
+        k_fold_start<RED_THREADS><<<nt, RED_THREADS, 0, s>>>(n, rp, S, part);
     XCAL_CHECK_LAUNCH();
 }
 

@@ -17,26 +17,25 @@ namespace xcal {
     const BSys<T>& B = sys[tm.x];                   \
     const TileCtx tc{tm.y, B.ntiles};
 
-template <class T>
-__global__ void __launch_bounds__(RED_THREADS, 8) kbk_spmv(const BSys<T>* __restrict__ sys, const int2* tmap, int in,
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_spmv(const BSys<T>* __restrict__ sys, const int2* tmap, int in,
                                                         int out) {
     XCAL_BSYS
-    spmv_body<T>(tc, B.A, B.nz, B.vec[in], B.vec[out], B.S);
+    spmv_body<T, NT>(tc, B.A, B.nz, B.vec[in], B.vec[out], B.S);
 }
 
-template <class T>
-__global__ void kbk_jacobi_apply(const BSys<T>* __restrict__ sys, const int2* tmap, int in, int out, int use_S) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_jacobi_apply(const BSys<T>* __restrict__ sys, const int2* tmap, int in, int out, int use_S) {
     XCAL_BSYS
     jacobi_apply_body<T>(tc, B.n, B.P, B.vec[in], B.vec[out], use_S ? B.S : nullptr);
 }
 
-template <class T>
-__global__ void kbk_copy(const BSys<T>* __restrict__ sys, const int2* tmap, int in, int out, int use_S) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_copy(const BSys<T>* __restrict__ sys, const int2* tmap, int in, int out, int use_S) {
     XCAL_BSYS
     copy_body<T>(tc, B.n, B.vec[in], B.vec[out], use_S ? B.S : nullptr);
 }
 
-// one DILU level over the rows (system, row) of every system at that level
 // DILU sweeps of every system as a dataflow (krylov_bodies.cuh): the blocks
 // draw (system, chunk of positions) items, listed in chunk order, from a
 // ticket, so whatever a chunk waits for was drawn before it by a running
@@ -62,64 +61,64 @@ __global__ void __launch_bounds__(FLOW_THREADS) kbk_dilu_flow(const BSys<T>* __r
     }
 }
 
-template <class T>
-__global__ void kbk_cg_start(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_cg_start(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
-    cg_start_body<T>(tc, B.n, B.vec[KV_R], B.vec[KV_Z], B.vec[KV_P], B.S, B.part0, B.ring);
+    cg_start_body<T, NT>(tc, B.n, B.vec[KV_R], B.vec[KV_Z], B.vec[KV_P], B.S, B.part0, B.ring);
 }
 
-template <class T>
-__global__ void __launch_bounds__(RED_THREADS, 8) kbk_cg_spmv(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_cg_spmv(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
-    cg_spmv_body<T>(tc, B.A, B.nz, B.vec[KV_Z], B.vec[KV_P], B.vec[KV_V], B.vec[KV_Q], B.S, B.part0);
+    cg_spmv_body<T, NT>(tc, B.A, B.nz, B.vec[KV_Z], B.vec[KV_P], B.vec[KV_V], B.vec[KV_Q], B.S, B.part0);
 }
 
-template <class T>
-__global__ void __launch_bounds__(RED_THREADS, sizeof(T) == 4 ? 4 : 8) kbk_cg_update(const BSys<T>* __restrict__ sys, const int2* tmap, int jacobi_fused) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, NT > RED_THREADS ? 1 : sizeof(T) == 4 ? 4 : 8) kbk_cg_update(const BSys<T>* __restrict__ sys, const int2* tmap, int jacobi_fused) {
     XCAL_BSYS
-    cg_update_body<T>(tc, B.n, B.vec[KV_X], B.vec[KV_P], B.vec[KV_V], B.vec[KV_R], B.vec[KV_Q], B.vec[KV_Z], B.P,
+    cg_update_body<T, NT>(tc, B.n, B.vec[KV_X], B.vec[KV_P], B.vec[KV_V], B.vec[KV_R], B.vec[KV_Q], B.vec[KV_Z], B.P,
                       jacobi_fused, B.S, B.part0);
 }
 
-template <class T>
-__global__ void kbk_cg_rz(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_cg_rz(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
-    cg_rz_body<T>(tc, B.n, B.vec[KV_R], B.vec[KV_Z], B.S, B.part0);
+    cg_rz_body<T, NT>(tc, B.n, B.vec[KV_R], B.vec[KV_Z], B.S, B.part0);
 }
 
-template <class T>
-__global__ void kbk_bicg_start(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_bicg_start(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
-    bicg_start_body<T>(tc, B.n, B.vec[KV_C], B.vec[KV_R], B.vec[KV_P], B.S, B.part0, B.part1);
+    bicg_start_body<T, NT>(tc, B.n, B.vec[KV_C], B.vec[KV_R], B.vec[KV_P], B.S, B.part0, B.part1);
 }
 
-template <class T>
-__global__ void kbk_bicg_alpha(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_bicg_alpha(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
-    bicg_alpha_body<T>(tc, B.n, B.vec[KV_C], B.vec[KV_V], B.S, B.part0);
+    bicg_alpha_body<T, NT>(tc, B.n, B.vec[KV_C], B.vec[KV_V], B.S, B.part0);
 }
 
-template <class T>
-__global__ void kbk_bicg_s(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_bicg_s(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
     bicg_s_body<T>(tc, B.n, B.vec[KV_R], B.vec[KV_V], B.vec[KV_P], B.vec[KV_S], B.vec[KV_X], B.S);
 }
 
-template <class T>
-__global__ void kbk_bicg_omega(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_bicg_omega(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
-    bicg_omega_body<T>(tc, B.n, B.vec[KV_T], B.vec[KV_S], B.S, B.part0, B.part1);
+    bicg_omega_body<T, NT>(tc, B.n, B.vec[KV_T], B.vec[KV_S], B.S, B.part0, B.part1);
 }
 
-template <class T>
-__global__ void kbk_bicg_xr(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_bicg_xr(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
-    bicg_xr_body<T>(tc, B.n, B.vec[KV_X], B.vec[KV_S], B.vec[KV_T], B.vec[KV_R], B.vec[KV_C], B.S, B.part0,
+    bicg_xr_body<T, NT>(tc, B.n, B.vec[KV_X], B.vec[KV_S], B.vec[KV_T], B.vec[KV_R], B.vec[KV_C], B.S, B.part0,
                     B.part1);
 }
 
-template <class T>
-__global__ void kbk_bicg_p(const BSys<T>* __restrict__ sys, const int2* tmap) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbk_bicg_p(const BSys<T>* __restrict__ sys, const int2* tmap) {
     XCAL_BSYS
     bicg_p_body<T>(tc, B.n, B.vec[KV_R], B.vec[KV_V], B.vec[KV_P], B.S);
 }
@@ -179,98 +178,61 @@ __global__ void __launch_bounds__(1024, 1) kbk_cg_persist_cl(const BSys<T>* __re
     const TileCtx tc{tm.y, B.ntiles};
 
 // r0 = b - A field, x = 0, dx = field (k_init_resid)
-__global__ void __launch_bounds__(RED_THREADS, 8) kbx_init_resid(const BAux* __restrict__ aux, const int2* tmap) {
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbx_init_resid(const BAux* __restrict__ aux, const int2* tmap) {
     XCAL_BAUX
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < B.n) {
-            B.r0[i] = B.b[i] - row_dot(B.A, B.nz, (const double*)B.field, i);
-            B.x[i] = 0.0;
-            B.dx[i] = B.field[i];
-        }
-    }
+    tile_rows(tc, B.n, [&](int i) {
+        B.r0[i] = B.b[i] - row_sum<NT>(B.A, B.nz, (const double*)B.field, i);
+        B.x[i] = 0.0;
+        B.dx[i] = B.field[i];
+    });
 }
 
 // field = x + dx (k_finish)
-__global__ void kbx_finish(const BAux* __restrict__ aux, const int2* tmap) {
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbx_finish(const BAux* __restrict__ aux, const int2* tmap) {
     XCAL_BAUX
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < B.n) B.field[i] = B.x[i] + B.dx[i];
-    }
+    tile_rows(tc, B.n, [&](int i) { B.field[i] = B.x[i] + B.dx[i]; });
 }
 
 // d32 = (float)(b - A field), x32 = 0 (k_defect)
-__global__ void __launch_bounds__(RED_THREADS, 8) kbx_defect(const BAux* __restrict__ aux, const int2* tmap) {
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbx_defect(const BAux* __restrict__ aux, const int2* tmap) {
     XCAL_BAUX
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < B.n) {
-            B.d32[i] = (float)(B.b[i] - row_dot(B.A, B.nz, (const double*)B.field, i));
-            B.x32[i] = 0.0f;
-        }
-    }
+    tile_rows(tc, B.n, [&](int i) {
+        B.d32[i] = (float)(B.b[i] - row_sum<NT>(B.A, B.nz, (const double*)B.field, i));
+        B.x32[i] = 0.0f;
+    });
 }
 
 // field += x32 unless the outer loop found the defect already at its target
 // (k_correct; the case then leaves the outer loop uncorrected)
-__global__ void kbx_correct(const BAux* __restrict__ aux, const int2* tmap) {
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbx_correct(const BAux* __restrict__ aux, const int2* tmap) {
     XCAL_BAUX
     if (B.S->outer_conv) return;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < B.n) B.field[i] = B.field[i] + (double)B.x32[i];
-    }
+    tile_rows(tc, B.n, [&](int i) { B.field[i] = B.field[i] + (double)B.x32[i]; });
 }
 
 // ||b - A field|| / max(||b||, 1 if tiny) per system (k_residual: the same
 // tile trees, the last of the system's blocks finishes)
-__global__ void __launch_bounds__(RED_THREADS, 8) kbx_residual(const BAux* __restrict__ aux, const int2* tmap) {
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbx_residual(const BAux* __restrict__ aux, const int2* tmap) {
     XCAL_BAUX
-    __shared__ double sm[8];
-    double a0 = 0.0, a1 = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < B.n) {
-            double fx = row_dot(B.A, B.nz, (const double*)B.field, i);
-            double bi = B.b[i];
-            double d = bi - fx;
-            a0 = a0 + d * d;
-            a1 = a1 + bi * bi;
-        }
-    }
-    double t0 = block_tree(a0, sm);
-    double t1 = block_tree(a1, sm);
-    if (threadIdx.x == 0) {
-        B.part0[tc.tile] = t0;
-        B.part1[tc.tile] = t1;
-    }
-    if (!last_block(&B.S->counter2, tc.ntiles)) return;
-    double sR = reduce_partials(B.part0, tc.ntiles, sm);
-    double sb = reduce_partials(B.part1, tc.ntiles, sm);
-    if (threadIdx.x == 0) {
-        double normb = sqrt(sb);
-        double denom = normb > jl_eps(normb) ? normb : 1.0;
-        double res = sqrt(sR) / denom;
-        B.S->resid = res;
-        B.S->normb = normb;
-        *B.res_out = res;
-    }
+    residual_body<NT>(tc, B.A, B.nz, (const double*)B.field, B.b, B.S, B.part0, B.part1, B.res_out);
 }
 
 // nz32 = (float) nz over the tile's slots (its rows' slices are contiguous),
 // P32 = (float) P over its rows
-__global__ void kbx_to_float(const BAux* __restrict__ aux, const int2* tmap) {
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbx_to_float(const BAux* __restrict__ aux, const int2* tmap) {
     XCAL_BAUX
     const int s0 = tc.tile * (RED_TILE / SELL_C);
     const int s1 = min(s0 + RED_TILE / SELL_C, (B.n + SELL_C - 1) / SELL_C);
     const int e1 = B.A.slice[s1];
-    for (int e = B.A.slice[s0] + threadIdx.x; e < e1; e += blockDim.x) B.nz32[e] = (float)ld_stream(B.nz + e);
-    if (B.P32)
-        for (int k = 0; k < RED_ITEMS; ++k) {
-            int i = tile_row(tc, k);
-            if (i < B.n) B.P32[i] = (float)B.P[i];
-        }
+#pragma unroll 4
+    for (int e = B.A.slice[s0] + threadIdx.x; e < e1; e += NT) B.nz32[e] = (float)ld_stream(B.nz + e);
+    if (B.P32) tile_rows(tc, B.n, [&](int i) { B.P32[i] = (float)B.P[i]; });
 }
 
 // level copies: slots of level positions in the tile (contiguous slices)
@@ -280,6 +242,7 @@ __device__ __forceinline__ void level_refresh_tile(const TileCtx& tc, int n, con
     const int s0 = tc.tile * (RED_TILE / SELL_C);
     const int s1 = min(s0 + RED_TILE / SELL_C, (n + SELL_C - 1) / SELL_C);
     const int e1 = slice[s1];
+#pragma unroll 4
     for (int e = slice[s0] + threadIdx.x; e < e1; e += blockDim.x) {
         val[e] = nz[ld_stream(src + e)];
         if (dinv) dinv[e] = T(1) / D[ld_stream(col + e)];
@@ -288,13 +251,11 @@ __device__ __forceinline__ void level_refresh_tile(const TileCtx& tc, int n, con
 
 template <class T>
 __device__ __forceinline__ void flow_unset_tile(const TileCtx& tc, int n, T* y) {
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        const int i = tile_row(tc, k);
-        if (i < n) y[i] = flow_unset_value<T>();
-    }
+    tile_rows(tc, n, [&](int i) { y[i] = flow_unset_value<T>(); });
 }
 
-__global__ void kbx_level_refresh(const BAux* __restrict__ aux, const int2* tmap, int fp32) {
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) kbx_level_refresh(const BAux* __restrict__ aux, const int2* tmap, int fp32) {
     XCAL_BAUX
     if (!B.lsrc) return;
     if (fp32) {
@@ -311,11 +272,15 @@ __global__ void kbx_level_refresh(const BAux* __restrict__ aux, const int2* tmap
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-#define XCAL_XLAUNCH(K, ...)                                     \
-    do {                                                         \
-        if (ntiles_total <= 0) return;                           \
-        K<<<ntiles_total, RED_THREADS, 0, s>>>(__VA_ARGS__);     \
-        XCAL_CHECK_LAUNCH();                                     \
+// a kernel over the batch's tiles, in the block size for that many (WIDE_TILES)
+#define XCAL_XLAUNCH(K, ...)                                                 \
+    do {                                                                     \
+        if (ntiles_total <= 0) return;                                       \
+        if (ntiles_total <= WIDE_TILES)                                      \
+            K<WIDE_NT><<<ntiles_total, WIDE_NT, 0, s>>>(__VA_ARGS__);         \
+        else                                                                 \
+            K<RED_THREADS><<<ntiles_total, RED_THREADS, 0, s>>>(__VA_ARGS__); \
+        XCAL_CHECK_LAUNCH();                                                 \
     } while (0)
 void kb_init_resid(cudaStream_t s, const BAux* aux, const int2* tmap, int ntiles_total) {
     XCAL_XLAUNCH(kbx_init_resid, aux, tmap);
@@ -338,11 +303,14 @@ void kb_to_float(cudaStream_t s, const BAux* aux, const int2* tmap, int ntiles_t
 void kb_level_refresh(cudaStream_t s, const BAux* aux, const int2* tmap, int ntiles_total, int fp32) {
     XCAL_XLAUNCH(kbx_level_refresh, aux, tmap, fp32);
 }
-#define XCAL_BLAUNCH(K, ...)                                     \
-    do {                                                         \
-        if (ntiles_total <= 0) return;                           \
-        K<T><<<ntiles_total, RED_THREADS, 0, s>>>(__VA_ARGS__);  \
-        XCAL_CHECK_LAUNCH();                                     \
+#define XCAL_BLAUNCH(K, ...)                                                    \
+    do {                                                                        \
+        if (ntiles_total <= 0) return;                                          \
+        if (ntiles_total <= WIDE_TILES)                                         \
+            K<T, WIDE_NT><<<ntiles_total, WIDE_NT, 0, s>>>(__VA_ARGS__);         \
+        else                                                                    \
+            K<T, RED_THREADS><<<ntiles_total, RED_THREADS, 0, s>>>(__VA_ARGS__); \
+        XCAL_CHECK_LAUNCH();                                                    \
     } while (0)
 
 template <class T>

@@ -29,41 +29,33 @@ namespace xcal {
 // ---------------------------------------------------------------------------
 // kernels (grid = one canonical tile per block, RED_THREADS threads)
 // ---------------------------------------------------------------------------
+// Kernels without a reduction take one row per thread.
 // r = b - A*x0, x = 0, dx = x0 (warm start: Krylov.jl kaxpby!(n,1,b,-1,r))
-__global__ void __launch_bounds__(RED_THREADS, 8) k_init_resid(CSRView A, const double* __restrict__ nz,
-                                                            const double* __restrict__ b,
-                                                            const double* __restrict__ field, double* dx, double* x,
-                                                            double* r) {
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(k);
-        if (i < A.n) {
-            r[i] = b[i] - row_dot(A, nz, field, i);
-            x[i] = 0.0;
-            dx[i] = field[i];
-        }
-    }
+__global__ void __launch_bounds__(256) k_init_resid(CSRView A, const double* __restrict__ nz,
+                                                    const double* __restrict__ b, const double* __restrict__ field,
+                                                    double* dx, double* x, double* r) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= A.n) return;
+    r[i] = b[i] - row_dot8(A, nz, field, i);
+    x[i] = 0.0;
+    dx[i] = field[i];
 }
 
 // Defect of a mixed-precision correction step: d = b - A*x in FP64, stored
 // rounded to FP32 as the inner right-hand side; the inner iterate starts at 0.
-__global__ void __launch_bounds__(RED_THREADS, 8) k_defect(CSRView A, const double* __restrict__ nz,
-                                                        const double* __restrict__ b,
-                                                        const double* __restrict__ field, float* d, float* x) {
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(k);
-        if (i < A.n) {
-            d[i] = (float)(b[i] - row_dot(A, nz, field, i));
-            x[i] = 0.0f;
-        }
-    }
+__global__ void __launch_bounds__(256) k_defect(CSRView A, const double* __restrict__ nz,
+                                                const double* __restrict__ b, const double* __restrict__ field,
+                                                float* d, float* x) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= A.n) return;
+    d[i] = (float)(b[i] - row_dot8(A, nz, field, i));
+    x[i] = 0.0f;
 }
 
 // field += correction (FP64 accumulation of the FP32 inner solution)
 __global__ void k_correct(int n, double* field, const float* __restrict__ x) {
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(k);
-        if (i < n) field[i] = field[i] + (double)x[i];
-    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) field[i] = field[i] + (double)x[i];
 }
 
 // dst = (float) src, any length
@@ -76,7 +68,7 @@ __global__ void k_to_float(long n, const double* __restrict__ src, float* dst) {
 template <class T>
 __global__ void __launch_bounds__(RED_THREADS, 8) k_spmv(CSRView A, const T* __restrict__ nz,
                                                       const T* __restrict__ x, T* y, const KScalars* S) {
-    spmv_body<T>(grid_tiles(), A, nz, x, y, S);
+    spmv_body<T, RED_THREADS>(grid_tiles(), A, nz, x, y, S);
 }
 
 // y = A*x with a free row mapping (no reduction rides on this SpMV): thread g
@@ -98,42 +90,46 @@ __global__ void k_spmv_rows(CSRView A, const T* __restrict__ nz, const T* __rest
 // z = P .* r (Jacobi: opDiagonal multiply, ldiv = false)
 template <class T>
 __global__ void k_jacobi_apply(int n, const T* __restrict__ P, const T* __restrict__ r, T* z, const KScalars* S) {
-    jacobi_apply_body<T>(grid_tiles(), n, P, r, z, S);
+    if (S && S->done) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) z[i] = P[i] * r[i];
 }
 
 template <class T>
 __global__ void k_copy(int n, const T* __restrict__ a, T* b, const KScalars* S) {
-    copy_body<T>(grid_tiles(), n, a, b, S);
+    if (S && S->done) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) b[i] = a[i];
 }
 
 // ---- CG ----
 // p = z; gamma = <r,z>; initial stopping tests
-template <class T>
-__global__ void k_cg_start(int n, const T* __restrict__ r, const T* __restrict__ z, T* p, KScalars* S,
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_cg_start(int n, const T* __restrict__ r, const T* __restrict__ z, T* p, KScalars* S,
                            double* part, double* ring) {
-    cg_start_body<T>(grid_tiles(), n, r, z, p, S, part, ring);
+    cg_start_body<T, NT>(grid_tiles(), n, r, z, p, S, part, ring);
 }
 
 // q = A p_k; pAp = <p_k,q>; zero-curvature test; alpha = gamma / pAp
-template <class T>
-__global__ void __launch_bounds__(RED_THREADS, 8) k_cg_spmv(CSRView A, const T* __restrict__ nz,
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_cg_spmv(CSRView A, const T* __restrict__ nz,
                                                          const T* __restrict__ z, T* P0, T* P1, T* q, KScalars* S,
                                                          double* part) {
-    cg_spmv_body<T>(grid_tiles(), A, nz, z, P0, P1, q, S, part);
+    cg_spmv_body<T, NT>(grid_tiles(), A, nz, z, P0, P1, q, S, part);
 }
 
 // x += alpha p_k; r -= alpha q; [Jacobi: z = P r; <r,z>; finalize]
-template <class T>
-__global__ void __launch_bounds__(RED_THREADS, sizeof(T) == 4 ? 4 : 8) k_cg_update(int n, T* x, const T* __restrict__ P0, const T* __restrict__ P1, T* r,
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, NT > RED_THREADS ? 1 : sizeof(T) == 4 ? 4 : 8) k_cg_update(int n, T* x, const T* __restrict__ P0, const T* __restrict__ P1, T* r,
                             const T* __restrict__ q, T* z, const T* __restrict__ P, int jacobi_fused, KScalars* S,
                             double* part) {
-    cg_update_body<T>(grid_tiles(), n, x, P0, P1, r, q, z, P, jacobi_fused, S, part);
+    cg_update_body<T, NT>(grid_tiles(), n, x, P0, P1, r, q, z, P, jacobi_fused, S, part);
 }
 
 // <r,z> + finalize when z came from a separate preconditioner apply
-template <class T>
-__global__ void k_cg_rz(int n, const T* __restrict__ r, const T* __restrict__ z, KScalars* S, double* part) {
-    cg_rz_body<T>(grid_tiles(), n, r, z, S, part);
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_cg_rz(int n, const T* __restrict__ r, const T* __restrict__ z, KScalars* S, double* part) {
+    cg_rz_body<T, NT>(grid_tiles(), n, r, z, S, part);
 }
 
 template <class T, int NT>
@@ -192,24 +188,22 @@ __global__ void __launch_bounds__(1024, 1)
 
 // field = x + dx (warm start shift)
 __global__ void k_finish(int n, const double* __restrict__ x, const double* __restrict__ dx, double* field) {
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(k);
-        if (i < n) field[i] = x[i] + dx[i];
-    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) field[i] = x[i] + dx[i];
 }
 
 // ---- BiCGSTAB ----
 // p = r; rNorm = ||r||; next_rho = <c,r>; initial tests
-template <class T>
-__global__ void k_bicg_start(int n, const T* __restrict__ c, const T* __restrict__ r, T* p, KScalars* S,
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_bicg_start(int n, const T* __restrict__ c, const T* __restrict__ r, T* p, KScalars* S,
                              double* part0, double* part1) {
-    bicg_start_body<T>(grid_tiles(), n, c, r, p, S, part0, part1);
+    bicg_start_body<T, NT>(grid_tiles(), n, c, r, p, S, part0, part1);
 }
 
 // alpha = rho / <c,v> (rho = next_rho; iteration counter advances)
-template <class T>
-__global__ void k_bicg_alpha(int n, const T* __restrict__ c, const T* __restrict__ v, KScalars* S, double* part) {
-    bicg_alpha_body<T>(grid_tiles(), n, c, v, S, part);
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_bicg_alpha(int n, const T* __restrict__ c, const T* __restrict__ v, KScalars* S, double* part) {
+    bicg_alpha_body<T, NT>(grid_tiles(), n, c, v, S, part);
 }
 
 // s = r - alpha v; x = x + alpha p
@@ -220,17 +214,17 @@ __global__ void k_bicg_s(int n, const T* __restrict__ r, const T* __restrict__ v
 }
 
 // omega = <t,s> / <t,t>
-template <class T>
-__global__ void k_bicg_omega(int n, const T* __restrict__ t, const T* __restrict__ s, KScalars* S, double* part0,
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_bicg_omega(int n, const T* __restrict__ t, const T* __restrict__ s, KScalars* S, double* part0,
                              double* part1) {
-    bicg_omega_body<T>(grid_tiles(), n, t, s, S, part0, part1);
+    bicg_omega_body<T, NT>(grid_tiles(), n, t, s, S, part0, part1);
 }
 
 // x = x + omega s; r = s - omega t; next_rho = <c,r>; ||r||; stopping tests
-template <class T>
-__global__ void k_bicg_xr(int n, T* x, const T* __restrict__ s, const T* __restrict__ t, T* r,
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_bicg_xr(int n, T* x, const T* __restrict__ s, const T* __restrict__ t, T* r,
                           const T* __restrict__ c, KScalars* S, double* part0, double* part1) {
-    bicg_xr_body<T>(grid_tiles(), n, x, s, t, r, c, S, part0, part1);
+    bicg_xr_body<T, NT>(grid_tiles(), n, x, s, t, r, c, S, part0, part1);
 }
 
 // p = r + beta (p - omega v)
@@ -257,13 +251,8 @@ __global__ void k_jacobi_smooth(CSRView A, const double* __restrict__ nz, const 
 // ---- preconditioners ----
 // update_Jacobi! (preconditioners_2_functions.jl:86-98)
 __global__ void k_jacobi_update(CSRView A, const double* __restrict__ nz, double* P) {
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(k);
-        if (i < A.n) {
-            double d = fabs(nz[A.diag[i]]);
-            P[i] = 1.0 / d;
-        }
-    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < A.n) P[i] = 1.0 / fabs(nz[A.diag[i]]);
 }
 
 // update_dilu_diagonal! restated per row (preconditioners_1_DILU.jl:43-82):
@@ -575,32 +564,13 @@ __global__ void k_gather_vals(long n, const int* __restrict__ src, const T* __re
         dst[e] = vals[ld_stream(src + e)];
 }
 
-// residual (src/Solve/Solve_1_api.jl:441-464): ||b - A x|| / max(||b||, 1 if tiny)
-__global__ void __launch_bounds__(RED_THREADS, 8) k_residual(CSRView A, const double* __restrict__ nz,
-                                                          const double* __restrict__ x, const double* __restrict__ b,
-                                                          KScalars* S, double* part0, double* part1, double* out) {
-    __shared__ double sm[8];
-    double a0 = 0.0, a1 = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(k);
-        if (i < A.n) {
-            double fx = row_dot(A, nz, x, i);
-            double bi = b[i];
-            double d = bi - fx;
-            a0 = a0 + d * d;
-            a1 = a1 + bi * bi;
-        }
-    }
-    double t0 = block_tree(a0, sm);
-    double t1 = block_tree(a1, sm);
-    if (threadIdx.x == 0) {
-        part0[blockIdx.x] = t0;
-        part1[blockIdx.x] = t1;
-    }
-    if (!last_block(&S->counter2)) return;
-    double sR = reduce_partials(part0, gridDim.x, sm);
-    double sb = reduce_partials(part1, gridDim.x, sm);
-    if (threadIdx.x == 0) residual_scalars(S, sR, sb, out);
+// residual (src/Solve/Solve_1_api.jl:441-464)
+template <int NT>
+__global__ void __launch_bounds__(NT, tile_min_blocks(NT)) k_residual(CSRView A, const double* __restrict__ nz,
+                                                                      const double* __restrict__ x,
+                                                                      const double* __restrict__ b, KScalars* S,
+                                                                      double* part0, double* part1, double* out) {
+    residual_body<NT>(grid_tiles(), A, nz, x, b, S, part0, part1, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -652,10 +622,8 @@ __global__ void k_outer_prep(KScalars* S) {
 // field += inner solution unless the defect already met the target
 __global__ void k_correct_masked(int n, double* field, const float* __restrict__ x, const KScalars* S) {
     if (S->outer_conv) return;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(k);
-        if (i < n) field[i] = field[i] + (double)x[i];
-    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) field[i] = field[i] + (double)x[i];
 }
 
 // end of a defect-correction step (the host loop's exit tests, on the device)
@@ -778,19 +746,29 @@ bool kr_cluster_capture_ok(bool in_while) {
 
 static inline int tiles(int n) { return n <= 0 ? 1 : (n + RED_TILE - 1) / RED_TILE; }
 #define TILE_LAUNCH(n) tiles(n), RED_THREADS, 0
+// one thread per row
+#define ROW_LAUNCH(n) ((n) <= 0 ? 1 : ((n) + 255) / 256), 256, 0
+// a tile kernel K<T.., NT> in the block size for n rows (WIDE_TILES)
+#define TILE_KERNEL(K, n, ...)                                                    \
+    do {                                                                          \
+        if (tiles(n) <= WIDE_TILES)                                               \
+            K(WIDE_NT)<<<tiles(n), WIDE_NT, 0, s>>>(__VA_ARGS__);                 \
+        else                                                                      \
+            K(RED_THREADS)<<<tiles(n), RED_THREADS, 0, s>>>(__VA_ARGS__);         \
+    } while (0)
 
 void kr_init_resid(cudaStream_t s, const CSRView& A, const double* nz, const double* b, const double* field,
                    double* dx, double* x, double* r) {
-    k_init_resid<<<TILE_LAUNCH(A.n), s>>>(A, nz, b, field, dx, x, r);
+    k_init_resid<<<ROW_LAUNCH(A.n), s>>>(A, nz, b, field, dx, x, r);
     XCAL_CHECK_LAUNCH();
 }
 void kr_defect(cudaStream_t s, const CSRView& A, const double* nz, const double* b, const double* field, float* d,
                float* x) {
-    k_defect<<<TILE_LAUNCH(A.n), s>>>(A, nz, b, field, d, x);
+    k_defect<<<ROW_LAUNCH(A.n), s>>>(A, nz, b, field, d, x);
     XCAL_CHECK_LAUNCH();
 }
 void kr_correct(cudaStream_t s, int n, double* field, const float* x) {
-    k_correct<<<TILE_LAUNCH(n), s>>>(n, field, x);
+    k_correct<<<ROW_LAUNCH(n), s>>>(n, field, x);
     XCAL_CHECK_LAUNCH();
 }
 void kr_to_float(cudaStream_t s, long n, const double* src, float* dst) {
@@ -823,23 +801,27 @@ void kr_spmv_shaped(cudaStream_t s, const SpmvShape& sh, const CSRView& A, const
 }
 template <class T>
 void kr_jacobi_apply(cudaStream_t s, int n, const T* P, const T* r, T* z, const KScalars* S) {
-    k_jacobi_apply<T><<<TILE_LAUNCH(n), s>>>(n, P, r, z, S);
+    k_jacobi_apply<T><<<ROW_LAUNCH(n), s>>>(n, P, r, z, S);
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
 void kr_copy(cudaStream_t s, int n, const T* a, T* b, const KScalars* S) {
-    k_copy<T><<<TILE_LAUNCH(n), s>>>(n, a, b, S);
+    k_copy<T><<<ROW_LAUNCH(n), s>>>(n, a, b, S);
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
 void kr_cg_start(cudaStream_t s, int n, const T* r, const T* z, T* p, KScalars* S, double* part, double* ring) {
-    k_cg_start<T><<<TILE_LAUNCH(n), s>>>(n, r, z, p, S, part, ring);
+#define K(NT) k_cg_start<T, NT>
+    TILE_KERNEL(K, n, n, r, z, p, S, part, ring);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
 void kr_cg_spmv(cudaStream_t s, const CSRView& A, const T* nz, const T* z, T* P0, T* P1, T* q, KScalars* S,
                 double* part) {
-    k_cg_spmv<T><<<TILE_LAUNCH(A.n), s>>>(A, nz, z, P0, P1, q, S, part);
+#define K(NT) k_cg_spmv<T, NT>
+    TILE_KERNEL(K, A.n, A, nz, z, P0, P1, q, S, part);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 static_assert(PERSIST_WIDTHS[2] == RED_THREADS, "narrow persistent form is one canonical tile row set per thread");
@@ -1094,27 +1076,35 @@ bool kr_cg_persist(cudaStream_t s, const CSRView& A, const T* nz, const T* P, in
 template <class T>
 void kr_cg_update(cudaStream_t s, int n, T* x, const T* P0, const T* P1, T* r, const T* q, T* z, const T* P,
                   int jacobi_fused, KScalars* S, double* part) {
-    k_cg_update<T><<<TILE_LAUNCH(n), s>>>(n, x, P0, P1, r, q, z, P, jacobi_fused, S, part);
+#define K(NT) k_cg_update<T, NT>
+    TILE_KERNEL(K, n, n, x, P0, P1, r, q, z, P, jacobi_fused, S, part);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
 void kr_cg_rz(cudaStream_t s, int n, const T* r, const T* z, KScalars* S, double* part) {
-    k_cg_rz<T><<<TILE_LAUNCH(n), s>>>(n, r, z, S, part);
+#define K(NT) k_cg_rz<T, NT>
+    TILE_KERNEL(K, n, n, r, z, S, part);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 void kr_finish(cudaStream_t s, int n, const double* x, const double* dx, double* field) {
-    k_finish<<<TILE_LAUNCH(n), s>>>(n, x, dx, field);
+    k_finish<<<ROW_LAUNCH(n), s>>>(n, x, dx, field);
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
 void kr_bicg_start(cudaStream_t s, int n, const T* c, const T* r, T* p, KScalars* S, double* part0,
                    double* part1) {
-    k_bicg_start<T><<<TILE_LAUNCH(n), s>>>(n, c, r, p, S, part0, part1);
+#define K(NT) k_bicg_start<T, NT>
+    TILE_KERNEL(K, n, n, c, r, p, S, part0, part1);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
 void kr_bicg_alpha(cudaStream_t s, int n, const T* c, const T* v, KScalars* S, double* part) {
-    k_bicg_alpha<T><<<TILE_LAUNCH(n), s>>>(n, c, v, S, part);
+#define K(NT) k_bicg_alpha<T, NT>
+    TILE_KERNEL(K, n, n, c, v, S, part);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
@@ -1123,14 +1113,18 @@ void kr_bicg_s(cudaStream_t s_, int n, const T* r, const T* v, const T* p, T* s,
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
-void kr_bicg_omega(cudaStream_t s_, int n, const T* t, const T* s, KScalars* S, double* part0, double* part1) {
-    k_bicg_omega<T><<<TILE_LAUNCH(n), s_>>>(n, t, s, S, part0, part1);
+void kr_bicg_omega(cudaStream_t s, int n, const T* t, const T* sv, KScalars* S, double* part0, double* part1) {
+#define K(NT) k_bicg_omega<T, NT>
+    TILE_KERNEL(K, n, n, t, sv, S, part0, part1);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
-void kr_bicg_xr(cudaStream_t s_, int n, T* x, const T* s, const T* t, T* r, const T* c, KScalars* S,
+void kr_bicg_xr(cudaStream_t s, int n, T* x, const T* sv, const T* t, T* r, const T* c, KScalars* S,
                 double* part0, double* part1) {
-    k_bicg_xr<T><<<TILE_LAUNCH(n), s_>>>(n, x, s, t, r, c, S, part0, part1);
+#define K(NT) k_bicg_xr<T, NT>
+    TILE_KERNEL(K, n, n, x, sv, t, r, c, S, part0, part1);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 template <class T>
@@ -1147,7 +1141,7 @@ void kr_jacobi_smooth(cudaStream_t s, const CSRView& A, const double* nz, const 
     }
 }
 void kr_jacobi_update(cudaStream_t s, const CSRView& A, const double* nz, double* P) {
-    k_jacobi_update<<<TILE_LAUNCH(A.n), s>>>(A, nz, P);
+    k_jacobi_update<<<ROW_LAUNCH(A.n), s>>>(A, nz, P);
     XCAL_CHECK_LAUNCH();
 }
 void kr_dilu_D(cudaStream_t s, const int* rows, int nrows, const CSRView& A, const double* nz, double* D) {
@@ -1334,7 +1328,9 @@ template bool kr_dilu_grid<float>(cudaStream_t, const LevelView<float>&, const L
 
 void kr_residual(cudaStream_t s, const CSRView& A, const double* nz, const double* x, const double* b, KScalars* S,
                  double* part0, double* part1, double* out) {
-    k_residual<<<TILE_LAUNCH(A.n), s>>>(A, nz, x, b, S, part0, part1, out);
+#define K(NT) k_residual<NT>
+    TILE_KERNEL(K, A.n, A, nz, x, b, S, part0, part1, out);
+#undef K
     XCAL_CHECK_LAUNCH();
 }
 
@@ -1356,7 +1352,7 @@ void kr_outer_prep(cudaStream_t s, KScalars* S) {
     XCAL_CHECK_LAUNCH();
 }
 void kr_correct_masked(cudaStream_t s, int n, double* field, const float* x, const KScalars* S) {
-    k_correct_masked<<<TILE_LAUNCH(n), s>>>(n, field, x, S);
+    k_correct_masked<<<ROW_LAUNCH(n), s>>>(n, field, x, S);
     XCAL_CHECK_LAUNCH();
 }
 void kr_outer_cond(cudaStream_t s, cudaGraphConditionalHandle h, KScalars* S, int max_outer, int body_kernels,

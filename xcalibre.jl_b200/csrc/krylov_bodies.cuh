@@ -26,6 +26,100 @@ __device__ __forceinline__ T row_dot(const CSRView& A, const T* __restrict__ nz,
     return acc;
 }
 
+// the same sum with the first 8 slots' loads issued together (wide tile
+// kernels: two rows per thread and registers to spare)
+template <class T>
+__device__ __forceinline__ T row_dot8(const CSRView& A, const T* __restrict__ nz, const T* __restrict__ x, int i) {
+    const int rb = row_base(A, i), rl = A.len[i];
+    T v[8], xv[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (k < rl) {
+            v[k] = ld_stream(nz + rb + SELL_C * k);
+            xv[k] = x[ld_stream(A.colval + rb + SELL_C * k)];
+        }
+    T acc = T(0);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (k < rl) acc = acc + v[k] * xv[k];
+    for (int k = 8; k < rl; ++k) {
+        const int e = rb + SELL_C * k;
+        acc = acc + ld_stream(nz + e) * x[ld_stream(A.colval + e)];
+    }
+    return acc;
+}
+template <int NT, class T>
+__device__ __forceinline__ T row_sum(const CSRView& A, const T* __restrict__ nz, const T* __restrict__ x, int i) {
+    return NT > RED_THREADS ? row_dot8(A, nz, x, i) : row_dot(A, nz, x, i);
+}
+
+// The tile kernels run in two block sizes.  NT = RED_THREADS: thread t takes
+// the tile's rows t + 256 k one after the other.  NT = WIDE_NT (launches of at
+// most WIDE_TILES tiles, which leave the chip short of threads): two rows per
+// thread, the rows' products through shared memory, threads 0..255 adding them
+// in k order -- the same partials, bit for bit.  Measured on B200: residual of
+// 27,025 rows 43 -> 12 us; CG SpMV, update and <r, z> of 116,440 rows together
+// 58 -> 34 us per DILU-CG iteration; 16 batched cases' steps around the solves
+// (95 tiles) 1.4 -> 0.9 ms per batch iteration.
+constexpr int WIDE_NT = 1024;
+constexpr int WIDE_TILES = 296;  // two per SM
+__host__ __device__ constexpr int tile_min_blocks(int nt) { return nt > RED_THREADS ? 1 : 8; }
+
+// f(i) for the rows i < n of the tile
+template <class F>
+__device__ __forceinline__ void tile_rows(const TileCtx& tc, int n, F&& f) {
+    for (int l = threadIdx.x; l < RED_TILE; l += blockDim.x) {
+        const int i = tc.tile * RED_TILE + l;
+        if (i < n) f(i);
+    }
+}
+
+template <int NT, int NV>
+struct TileSmem {
+    double pr[NT > RED_THREADS ? NV : 1][NT > RED_THREADS ? RED_TILE : 1];
+    double sm[8];
+};
+// the tile's canonical partials of the NV products f(i, v) gives for each row,
+// in tot of thread 0
+template <int NT, int NV, class F>
+__device__ __forceinline__ void tile_reduce(const TileCtx& tc, int n, TileSmem<NT, NV>& sh, double (&tot)[NV], F&& f) {
+    double acc[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) acc[q] = 0.0;
+    if constexpr (NT == RED_THREADS) {
+        for (int k = 0; k < RED_ITEMS; ++k) {
+            const int i = tile_row(tc, k);
+            if (i < n) {
+                double v[NV];
+                f(i, v);
+#pragma unroll
+                for (int q = 0; q < NV; ++q) acc[q] = acc[q] + v[q];
+            }
+        }
+    } else {
+        // rows past n add 0.0, which leaves every partial sum as it is (they
+        // start at +0.0 and are never -0.0)
+#pragma unroll
+        for (int j = 0; j < RED_TILE / NT; ++j) {
+            const int l = j * NT + threadIdx.x, i = tc.tile * RED_TILE + l;
+            double v[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) v[q] = 0.0;
+            if (i < n) f(i, v);
+#pragma unroll
+            for (int q = 0; q < NV; ++q) sh.pr[q][l] = v[q];
+        }
+        __syncthreads();
+        if (threadIdx.x < RED_THREADS)
+#pragma unroll
+            for (int k = 0; k < RED_ITEMS; ++k)
+#pragma unroll
+                for (int q = 0; q < NV; ++q) acc[q] = acc[q] + sh.pr[q][k * RED_THREADS + threadIdx.x];
+    }
+#pragma unroll
+    for (int q = 0; q < NV; ++q) tot[q] = block_tree(acc[q], sh.sm);
+}
+
 // CG stopping decisions after gamma_next = <r,z> (Krylov.jl cg!)
 __device__ __forceinline__ void cg_finalize(KScalars* S, double gamma_next) {
     double rNorm = sqrt(gamma_next);
@@ -75,32 +169,51 @@ __device__ __forceinline__ T cg_dir(const T* __restrict__ z, const T* __restrict
     return z[j] + beta * pold[j];
 }
 
-template <class T>
-__device__ __forceinline__ void spmv_body(const TileCtx& tc, CSRView A, const T* __restrict__ nz,
-                                                      const T* __restrict__ x, T* y, const KScalars* S) {
-    if (S && S->done) return;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < A.n) y[i] = row_dot(A, nz, x, i);
+// q_i = sum_k nz[i,k] * d[col(i,k)] in slot order, d = p (first iteration) or
+// z + beta p_old gathered on the fly: the first 8 slots' loads are issued
+// together, the products are then added in slot order (wide forms only; the
+// narrow forms keep the plain loop, which needs fewer registers).
+template <class T, bool FIRST>
+__device__ __forceinline__ T cg_row_q(const CSRView& A, const T* __restrict__ nz, const T* z, const T* pold,
+                                      const T* pk, T b, int i) {
+    const int rb = row_base(A, i), ln = A.len[i];
+    T qi = T(0);
+    int c[8];
+    T v[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+        if (t < ln) {
+            c[t] = ld_stream(A.colval + rb + SELL_C * t);
+            v[t] = ld_stream(nz + rb + SELL_C * t);
+        }
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+        if (t < ln) qi = qi + v[t] * (FIRST ? pk[c[t]] : cg_dir(z, pold, b, c[t]));
+    for (int t = 8; t < ln; ++t) {
+        const int s = rb + SELL_C * t;
+        const int cc = ld_stream(A.colval + s);
+        qi = qi + ld_stream(nz + s) * (FIRST ? pk[cc] : cg_dir(z, pold, b, cc));
     }
+    return qi;
+}
+
+template <class T, int NT>
+__device__ __forceinline__ void spmv_body(const TileCtx& tc, CSRView A, const T* __restrict__ nz,
+                                          const T* __restrict__ x, T* y, const KScalars* S) {
+    if (S && S->done) return;
+    tile_rows(tc, A.n, [&](int i) { y[i] = row_sum<NT>(A, nz, x, i); });
 }
 
 template <class T>
 __device__ __forceinline__ void jacobi_apply_body(const TileCtx& tc, int n, const T* __restrict__ P, const T* __restrict__ r, T* z, const KScalars* S) {
     if (S && S->done) return;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) z[i] = P[i] * r[i];
-    }
+    tile_rows(tc, n, [&](int i) { z[i] = P[i] * r[i]; });
 }
 
 template <class T>
 __device__ __forceinline__ void copy_body(const TileCtx& tc, int n, const T* __restrict__ a, T* b, const KScalars* S) {
     if (S && S->done) return;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) b[i] = a[i];
-    }
+    tile_rows(tc, n, [&](int i) { b[i] = a[i]; });
 }
 
 // the start of a cg! solve from gamma = <r0, z0> (Krylov.jl cg!): norms,
@@ -132,46 +245,50 @@ __device__ __forceinline__ void cg_start_scalars(KScalars* S, double gamma) {
     }
 }
 
-template <class T>
+template <class T, int NT>
 __device__ __forceinline__ void cg_start_body(const TileCtx& tc, int n, const T* __restrict__ r, const T* __restrict__ z, T* p, KScalars* S,
                            double* part, double* ring) {
-    __shared__ double sm[8];
-    double acc = 0.0;
+    __shared__ TileSmem<NT, 1> sh;
     // the resident CG's exchange buffers start unset (cg_resident_body)
     if (tc.ntiles <= RES_TILES_MAX)
         for (int k = threadIdx.x; k < 4 * tc.ntiles; k += blockDim.x)
             ring[((size_t)(k / tc.ntiles) * tc.ntiles + tc.tile) * tc.ntiles + k % tc.ntiles] =
                 __longlong_as_double(-1LL);
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) {
-            T zi = z[i];
-            p[i] = zi;
-            acc = acc + (double)r[i] * (double)zi;
-        }
-    }
-    double tot = block_tree(acc, sm);
-    if (threadIdx.x == 0) part[tc.tile] = tot;
+    double tot[1];
+    tile_reduce<NT, 1>(tc, n, sh, tot, [&](int i, double* v) {
+        T zi = z[i];
+        p[i] = zi;
+        v[0] = (double)r[i] * (double)zi;
+    });
+    if (threadIdx.x == 0) part[tc.tile] = tot[0];
     if (!last_block(&S->counter, tc.ntiles)) return;
-    double gamma = reduce_partials(part, tc.ntiles, sm);
+    double gamma = reduce_partials(part, tc.ntiles, sh.sm);
     if (threadIdx.x == 0) cg_start_scalars(S, gamma);
 }
 
-template <class T>
+template <class T, int NT>
 __device__ __forceinline__ void cg_spmv_body(const TileCtx& tc, CSRView A, const T* __restrict__ nz,
                                                          const T* __restrict__ z, T* P0, T* P1, T* q, KScalars* S,
                                                          double* part) {
     if (S->done) return;
-    __shared__ double sm[8];
+    __shared__ TileSmem<NT, 1> sh;
     const int it = S->iter;
     const T beta = (T)S->beta;
     T* pk = (it & 1) ? P1 : P0;
     const T* pold = (it & 1) ? P0 : P1;
-    double acc = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < A.n) {
-            T qi = T(0), pi;
+    double tot[1];
+    tile_reduce<NT, 1>(tc, A.n, sh, tot, [&](int i, double* v) {
+        T qi = T(0), pi;
+        if constexpr (NT > RED_THREADS) {
+            if (it == 0) {
+                qi = cg_row_q<T, true>(A, nz, z, pold, pk, beta, i);
+                pi = pk[i];
+            } else {
+                qi = cg_row_q<T, false>(A, nz, z, pold, pk, beta, i);
+                pi = cg_dir(z, pold, beta, i);
+                pk[i] = pi;
+            }
+        } else {
             const int rb = row_base(A, i), e1 = rb + SELL_C * A.len[i];
             if (it == 0) {
                 for (int e = rb; e < e1; e += SELL_C) qi = qi + ld_stream(nz + e) * pk[ld_stream(A.colval + e)];
@@ -182,14 +299,13 @@ __device__ __forceinline__ void cg_spmv_body(const TileCtx& tc, CSRView A, const
                 pi = cg_dir(z, pold, beta, i);
                 pk[i] = pi;
             }
-            q[i] = qi;
-            acc = acc + (double)pi * (double)qi;
         }
-    }
-    double tot = block_tree(acc, sm);
-    if (threadIdx.x == 0) part[tc.tile] = tot;
+        q[i] = qi;
+        v[0] = (double)pi * (double)qi;
+    });
+    if (threadIdx.x == 0) part[tc.tile] = tot[0];
     if (!last_block(&S->counter, tc.ntiles)) return;
-    double pAp = reduce_partials(part, tc.ntiles, sm);
+    double pAp = reduce_partials(part, tc.ntiles, sh.sm);
     if (threadIdx.x == 0) {
         const double epsT = sizeof(T) == 8 ? 2.220446049250313e-16 : 1.1920928955078125e-07;  // eps(T)
         double lim = epsT * S->pNorm2;
@@ -202,16 +318,17 @@ __device__ __forceinline__ void cg_spmv_body(const TileCtx& tc, CSRView A, const
     }
 }
 
-template <class T>
+template <class T, int NT>
 __device__ __forceinline__ void cg_update_body(const TileCtx& tc, int n, T* x, const T* __restrict__ P0, const T* __restrict__ P1, T* r,
                             const T* __restrict__ q, T* z, const T* __restrict__ P, int jacobi_fused, KScalars* S,
                             double* part) {
     if (S->done) return;
-    __shared__ double sm[8];
+    __shared__ TileSmem<NT, 1> sh;
+    double* sm = sh.sm;
     const T* p = (S->iter & 1) ? P1 : P0;
     const T alpha = (T)S->alpha;
     double acc = 0.0;
-    if constexpr (sizeof(T) == 4) {
+    if constexpr (sizeof(T) == 4 && NT == RED_THREADS) {
         // FP32: 4-byte elements leave too few bytes in flight per thread when
         // each row waits for its loads; issue all rows' loads first (same
         // arithmetic, same order of the sums).  Measured 18.4 -> 14.4 us on
@@ -249,42 +366,40 @@ __device__ __forceinline__ void cg_update_body(const TileCtx& tc, int n, T* x, c
             return;
         }
     }
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) {
-            // x, q and P are not read again before the next update: evict-first
-            // keeps L2 for z and p, which the next SpMV gathers
-            __stcs(x + i, ld_stream(x + i) + alpha * p[i]);
-            T ri = r[i] + (-alpha) * ld_stream(q + i);
-            r[i] = ri;
-            if (jacobi_fused) {
-                T zi = ld_stream(P + i) * ri;
-                z[i] = zi;
-                acc = acc + (double)ri * (double)zi;
-            }
-        }
+    // x, q and P are not read again before the next update: evict-first keeps
+    // L2 for z and p, which the next SpMV gathers
+    auto row = [&](int i) {
+        __stcs(x + i, ld_stream(x + i) + alpha * p[i]);
+        T ri = r[i] + (-alpha) * ld_stream(q + i);
+        r[i] = ri;
+        return ri;
+    };
+    if (!jacobi_fused) {
+        tile_rows(tc, n, [&](int i) { row(i); });
+        return;
     }
-    if (!jacobi_fused) return;
-    double tot = block_tree(acc, sm);
-    if (threadIdx.x == 0) part[tc.tile] = tot;
+    double tot[1];
+    tile_reduce<NT, 1>(tc, n, sh, tot, [&](int i, double* v) {
+        T ri = row(i);
+        T zi = ld_stream(P + i) * ri;
+        z[i] = zi;
+        v[0] = (double)ri * (double)zi;
+    });
+    if (threadIdx.x == 0) part[tc.tile] = tot[0];
     if (!last_block(&S->counter, tc.ntiles)) return;
     double g = reduce_partials(part, tc.ntiles, sm);
     if (threadIdx.x == 0) cg_finalize(S, g);
 }
 
-template <class T>
+template <class T, int NT>
 __device__ __forceinline__ void cg_rz_body(const TileCtx& tc, int n, const T* __restrict__ r, const T* __restrict__ z, KScalars* S, double* part) {
     if (S->done) return;
-    __shared__ double sm[8];
-    double acc = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) acc = acc + (double)r[i] * (double)z[i];
-    }
-    double tot = block_tree(acc, sm);
-    if (threadIdx.x == 0) part[tc.tile] = tot;
+    __shared__ TileSmem<NT, 1> sh;
+    double tot[1];
+    tile_reduce<NT, 1>(tc, n, sh, tot, [&](int i, double* v) { v[0] = (double)r[i] * (double)z[i]; });
+    if (threadIdx.x == 0) part[tc.tile] = tot[0];
     if (!last_block(&S->counter, tc.ntiles)) return;
-    double g = reduce_partials(part, tc.ntiles, sm);
+    double g = reduce_partials(part, tc.ntiles, sh.sm);
     if (threadIdx.x == 0) cg_finalize(S, g);
 }
 
@@ -358,45 +473,36 @@ __device__ __forceinline__ void residual_scalars(KScalars* S, double sR, double 
     if (out) *out = res;
 }
 
-template <class T>
+template <class T, int NT>
 __device__ __forceinline__ void bicg_start_body(const TileCtx& tc, int n, const T* __restrict__ c, const T* __restrict__ r, T* p, KScalars* S,
                              double* part0, double* part1) {
-    __shared__ double sm[8];
-    double a0 = 0.0, a1 = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) {
-            T ri = r[i];
-            p[i] = ri;
-            a0 = a0 + (double)ri * (double)ri;
-            a1 = a1 + (double)c[i] * (double)ri;
-        }
-    }
-    double t0 = block_tree(a0, sm);
-    double t1 = block_tree(a1, sm);
+    __shared__ TileSmem<NT, 2> sh;
+    double tot[2];
+    tile_reduce<NT, 2>(tc, n, sh, tot, [&](int i, double* v) {
+        T ri = r[i];
+        p[i] = ri;
+        v[0] = (double)ri * (double)ri;
+        v[1] = (double)c[i] * (double)ri;
+    });
     if (threadIdx.x == 0) {
-        part0[tc.tile] = t0;
-        part1[tc.tile] = t1;
+        part0[tc.tile] = tot[0];
+        part1[tc.tile] = tot[1];
     }
     if (!last_block(&S->counter, tc.ntiles)) return;
-    double rr = reduce_partials(part0, tc.ntiles, sm);
-    double cr = reduce_partials(part1, tc.ntiles, sm);
+    double rr = reduce_partials(part0, tc.ntiles, sh.sm);
+    double cr = reduce_partials(part1, tc.ntiles, sh.sm);
     if (threadIdx.x == 0) bicg_start_scalars(S, rr, cr);
 }
 
-template <class T>
+template <class T, int NT>
 __device__ __forceinline__ void bicg_alpha_body(const TileCtx& tc, int n, const T* __restrict__ c, const T* __restrict__ v, KScalars* S, double* part) {
     if (S->done) return;
-    __shared__ double sm[8];
-    double acc = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) acc = acc + (double)c[i] * (double)v[i];
-    }
-    double tot = block_tree(acc, sm);
-    if (threadIdx.x == 0) part[tc.tile] = tot;
+    __shared__ TileSmem<NT, 1> sh;
+    double tot[1];
+    tile_reduce<NT, 1>(tc, n, sh, tot, [&](int i, double* o) { o[0] = (double)c[i] * (double)v[i]; });
+    if (threadIdx.x == 0) part[tc.tile] = tot[0];
     if (!last_block(&S->counter, tc.ntiles)) return;
-    double cv = reduce_partials(part, tc.ntiles, sm);
+    double cv = reduce_partials(part, tc.ntiles, sh.sm);
     if (threadIdx.x == 0) bicg_alpha_scalars(S, cv);
 }
 
@@ -405,69 +511,56 @@ __device__ __forceinline__ void bicg_s_body(const TileCtx& tc, int n, const T* _
                          T* x, const KScalars* S) {
     if (S->done) return;
     const T alpha = (T)S->alpha;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) {
-            s[i] = r[i] + (-alpha) * v[i];
-            x[i] = x[i] + alpha * p[i];
-        }
-    }
+    tile_rows(tc, n, [&](int i) {
+        s[i] = r[i] + (-alpha) * v[i];
+        x[i] = x[i] + alpha * p[i];
+    });
 }
 
-template <class T>
+template <class T, int NT>
 __device__ __forceinline__ void bicg_omega_body(const TileCtx& tc, int n, const T* __restrict__ t, const T* __restrict__ s, KScalars* S, double* part0,
                              double* part1) {
     if (S->done) return;
-    __shared__ double sm[8];
-    double a0 = 0.0, a1 = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) {
-            double ti = (double)t[i];
-            a0 = a0 + ti * (double)s[i];
-            a1 = a1 + ti * ti;
-        }
-    }
-    double t0 = block_tree(a0, sm);
-    double t1 = block_tree(a1, sm);
+    __shared__ TileSmem<NT, 2> sh;
+    double tot[2];
+    tile_reduce<NT, 2>(tc, n, sh, tot, [&](int i, double* v) {
+        double ti = (double)t[i];
+        v[0] = ti * (double)s[i];
+        v[1] = ti * ti;
+    });
     if (threadIdx.x == 0) {
-        part0[tc.tile] = t0;
-        part1[tc.tile] = t1;
+        part0[tc.tile] = tot[0];
+        part1[tc.tile] = tot[1];
     }
     if (!last_block(&S->counter, tc.ntiles)) return;
-    double ts = reduce_partials(part0, tc.ntiles, sm);
-    double tt = reduce_partials(part1, tc.ntiles, sm);
+    double ts = reduce_partials(part0, tc.ntiles, sh.sm);
+    double tt = reduce_partials(part1, tc.ntiles, sh.sm);
     if (threadIdx.x == 0) S->omega = ts / tt;
 }
 
-template <class T>
+template <class T, int NT>
 __device__ __forceinline__ void bicg_xr_body(const TileCtx& tc, int n, T* x, const T* __restrict__ s, const T* __restrict__ t, T* r,
                           const T* __restrict__ c, KScalars* S, double* part0, double* part1) {
     if (S->done) return;
-    __shared__ double sm[8];
+    __shared__ TileSmem<NT, 2> sh;
     const double omega = S->omega;
     const T om = (T)omega;
-    double a0 = 0.0, a1 = 0.0;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) {
-            T si = s[i];
-            x[i] = x[i] + om * si;
-            T ri = si + (-om) * t[i];
-            r[i] = ri;
-            a0 = a0 + (double)c[i] * (double)ri;
-            a1 = a1 + (double)ri * (double)ri;
-        }
-    }
-    double t0 = block_tree(a0, sm);
-    double t1 = block_tree(a1, sm);
+    double tot[2];
+    tile_reduce<NT, 2>(tc, n, sh, tot, [&](int i, double* v) {
+        T si = s[i];
+        x[i] = x[i] + om * si;
+        T ri = si + (-om) * t[i];
+        r[i] = ri;
+        v[0] = (double)c[i] * (double)ri;
+        v[1] = (double)ri * (double)ri;
+    });
     if (threadIdx.x == 0) {
-        part0[tc.tile] = t0;
-        part1[tc.tile] = t1;
+        part0[tc.tile] = tot[0];
+        part1[tc.tile] = tot[1];
     }
     if (!last_block(&S->counter, tc.ntiles)) return;
-    double cr = reduce_partials(part0, tc.ntiles, sm);
-    double rr = reduce_partials(part1, tc.ntiles, sm);
+    double cr = reduce_partials(part0, tc.ntiles, sh.sm);
+    double rr = reduce_partials(part1, tc.ntiles, sh.sm);
     if (threadIdx.x == 0) bicg_xr_scalars(S, omega, cr, rr);
 }
 
@@ -475,10 +568,31 @@ template <class T>
 __device__ __forceinline__ void bicg_p_body(const TileCtx& tc, int n, const T* __restrict__ r, const T* __restrict__ v, T* p, const KScalars* S) {
     if (S->done) return;
     const T beta = (T)S->beta, omega = (T)S->omega;
-    for (int k = 0; k < RED_ITEMS; ++k) {
-        int i = tile_row(tc, k);
-        if (i < n) p[i] = r[i] + beta * (p[i] + (-omega) * v[i]);
+    tile_rows(tc, n, [&](int i) { p[i] = r[i] + beta * (p[i] + (-omega) * v[i]); });
+}
+
+// residual (src/Solve/Solve_1_api.jl:441-464): ||b - A x|| / max(||b||, 1 if tiny)
+template <int NT>
+__device__ __forceinline__ void residual_body(const TileCtx& tc, const CSRView& A, const double* __restrict__ nz,
+                                              const double* __restrict__ x, const double* __restrict__ b, KScalars* S,
+                                              double* part0, double* part1, double* out) {
+    __shared__ TileSmem<NT, 2> sh;
+    double tot[2];
+    tile_reduce<NT, 2>(tc, A.n, sh, tot, [&](int i, double* v) {
+        double fx = row_sum<NT>(A, nz, x, i);
+        double bi = b[i];
+        double d = bi - fx;
+        v[0] = d * d;
+        v[1] = bi * bi;
+    });
+    if (threadIdx.x == 0) {
+        part0[tc.tile] = tot[0];
+        part1[tc.tile] = tot[1];
     }
+    if (!last_block(&S->counter2, tc.ntiles)) return;
+    double sR = reduce_partials(part0, tc.ntiles, sh.sm);
+    double sb = reduce_partials(part1, tc.ntiles, sh.sm);
+    if (threadIdx.x == 0) residual_scalars(S, sR, sb, out);
 }
 
 // A DILU application of a small system as one
@@ -822,34 +936,6 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* count, int nblocks, u
     ++nb;
     __syncthreads();
     return *sh_err == 0;
-}
-
-// q_i = sum_k nz[i,k] * d[col(i,k)] in slot order, d = p (first iteration) or
-// z + beta p_old gathered on the fly: the first 8 slots' loads are issued
-// together, the products are then added in slot order (wide form only; the
-// narrow form keeps the plain loop, which needs fewer registers).
-template <class T, bool FIRST>
-__device__ __forceinline__ T cg_row_q(const CSRView& A, const T* __restrict__ nz, const T* z, const T* pold,
-                                      const T* pk, T b, int i) {
-    const int rb = row_base(A, i), ln = A.len[i];
-    T qi = T(0);
-    int c[8];
-    T v[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t)
-        if (t < ln) {
-            c[t] = ld_stream(A.colval + rb + SELL_C * t);
-            v[t] = ld_stream(nz + rb + SELL_C * t);
-        }
-#pragma unroll
-    for (int t = 0; t < 8; ++t)
-        if (t < ln) qi = qi + v[t] * (FIRST ? pk[c[t]] : cg_dir(z, pold, b, c[t]));
-    for (int t = 8; t < ln; ++t) {
-        const int s = rb + SELL_C * t;
-        const int cc = ld_stream(A.colval + s);
-        qi = qi + ld_stream(nz + s) * (FIRST ? pk[cc] : cg_dir(z, pold, b, cc));
-    }
-    return qi;
 }
 
 // Bulk prefetch of [p, p + bytes) into L2 (no data reaches the SM; p and

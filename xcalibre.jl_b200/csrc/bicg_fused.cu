@@ -695,8 +695,6 @@ void Case::reserve_fused() {
     bf.S.alloc(3);
     bf.S.zero(stream);
     bf.res.alloc(3);
-    XCAL_CUDA(cudaMallocHost(&bf.hS, 3 * sizeof(KScalars)));
-    XCAL_CUDA(cudaMallocHost(&bf.hres, 3 * sizeof(double)));
     bf.ready = true;
 }
 
@@ -819,8 +817,8 @@ void Case::fused_solve(Equation& E, const xcal_solver_setup& SS, const SolveRef*
         for (int d = 0; d < NC; ++d) res[d] = 0.0;
         return;
     }
-    KScalars* hS = NC == 1 ? h_S + R[0].kslot : bf.hS;
-    double* hres = NC == 1 ? h_res : bf.hres;
+    KScalars* hS = NC == 1 ? h_S + R[0].kslot : h_S + 2;
+    double* hres = h_res;
     std::memset(hS, 0, NC * sizeof(KScalars));
     for (int d = 0; d < NC; ++d) {
         hS[d].atol = SS.atol;

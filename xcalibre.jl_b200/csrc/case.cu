@@ -56,6 +56,10 @@ CSRView Equation::view() const {
     v.cf_slot = d_cf_slot.p;
     v.tile_slots = tile_slots;
     v.tile_halo = tile_halo;
+    v.hoff = d_hoff.p;
+    v.hdst = d_hdst.p;
+    v.hrow = d_hrow.p;
+    v.rowh = d_rowh.p;
     v.fslot = d_fslot.p;
     return v;
 }
@@ -477,19 +481,6 @@ void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& b
     }
     rows_s.clear();
     rows_s.shrink_to_fit();
-    constexpr int TILE = 2048;
-    E.tile_slots = E.tile_halo = 0;
-    for (int r0 = 0; r0 < n && n <= RES_TILES_MAX * TILE; r0 += TILE) {
-        const int r1 = std::min(n, r0 + TILE);
-        int halo = 0;
-        for (int r = r0; r < r1; ++r)
-            for (int k = 0; k < E.len[r]; ++k) {
-                const int c = E.colval[E.base(r) + SELL_C * k];
-                halo += c < r0 || c >= r1;
-            }
-        E.tile_slots = std::max(E.tile_slots, E.slice[(r1 + SELL_C - 1) / SELL_C] - E.slice[r0 / SELL_C]);
-        E.tile_halo = std::max(E.tile_halo, halo);
-    }
     E.diag.resize(n);
     for (int c = 0; c < n; ++c) E.diag[c] = E.find(c, c);
     std::vector<int> trans(E.nnz, 0), cf_slot(m.cf_face.size()), fslot(m.nI);
@@ -516,6 +507,40 @@ void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& b
                 const int e = b + SELL_C * k;
                 if (!set[e]) trans[e] = E.find(E.colval[e], i);
             }
+    }
+    // what the resident CG keeps per tile, and its halo entries (CSRView)
+    constexpr int TILE = 2048;
+    E.tile_slots = E.tile_halo = 0;
+    if (n <= RES_TILES_MAX * TILE) {
+        std::vector<int> hoff(1, 0), hslot, entry(E.nnz, -1);
+        std::vector<unsigned short> hrow, rowh(n);
+        bool ok = true;
+        for (int r0 = 0; r0 < n; r0 += TILE) {
+            const int r1 = std::min(n, r0 + TILE);
+            for (int r = r0; r < r1; ++r) {
+                rowh[r] = (unsigned short)std::min((int)hslot.size() - hoff.back(), 65535);
+                for (int k = 0; k < E.len[r]; ++k) {
+                    const int e = E.base(r) + SELL_C * k, c = E.colval[e];
+                    if (c >= r0 && c < r1) continue;
+                    ok = ok && trans[e] >= 0;
+                    entry[e] = (int)hslot.size();
+                    hslot.push_back(e);
+                    hrow.push_back((unsigned short)(r - r0));
+                }
+            }
+            E.tile_halo = std::max(E.tile_halo, (int)hslot.size() - hoff.back());
+            E.tile_slots = std::max(E.tile_slots, E.slice[(r1 + SELL_C - 1) / SELL_C] - E.slice[r0 / SELL_C]);
+            hoff.push_back((int)hslot.size());
+        }
+        std::vector<int> hdst(hslot.size());
+        for (size_t g = 0; ok && g < hslot.size(); ++g) hdst[g] = entry[trans[hslot[g]]];
+        E.n_halo = (long)hslot.size();
+        if (!ok) E.tile_slots = 0;  // an entry without its transposed one: not this form
+        E.d_hoff.upload(hoff, s);
+        E.d_hdst.upload(hdst, s);
+        E.d_hrow.upload(hrow, s);
+        E.d_rowh.upload(rowh, s);
+        XCAL_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
     }
     E.d_slice.upload(E.slice, s);
     E.d_len.upload(E.len, s);
@@ -766,7 +791,7 @@ Case::Case(xcal_ctx* c, const DevMesh* m, const xcal_config* cf) : ctx(c), mesh(
     }
     XCAL_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     for (auto& e : ev) XCAL_CUDA(cudaEventCreate(&e));
-    XCAL_CUDA(cudaMallocHost(&h_S, 2 * sizeof(KScalars)));
+    XCAL_CUDA(cudaMallocHost(&h_S, 5 * sizeof(KScalars)));
     XCAL_CUDA(cudaMallocHost(&h_res, 16 * sizeof(double)));
     int nC = m->nC, nF = m->nF;
     std::vector<xcal_bc> bU(cfg.bc_U, cfg.bc_U + cfg.n_bc_U), bP(cfg.bc_p, cfg.bc_p + cfg.n_bc_p);

@@ -89,6 +89,9 @@ struct Equation {
     DBuf<int> d_slice, d_colval, d_diag, d_trans, d_cf_slot, d_fslot;
     DBuf<unsigned char> d_len;
     int tile_slots = 0, tile_halo = 0;  // CSRView: what the resident CG keeps per tile
+    long n_halo = 0;                    // its halo entries over all tiles
+    DBuf<int> d_hoff, d_hdst;
+    DBuf<unsigned short> d_hrow, d_rowh;
     int base(int r) const { return slice[r / SELL_C] + r % SELL_C; }
     DBuf<double> nz, nz0, diag0, P;
     DBuf<float> nz32, P32;  // mixed precision: FP32 copies for the inner solves
@@ -218,7 +221,7 @@ struct Case {
     double ms[6] = {0, 0, 0, 0, 0, 0};
     long long launches = 0;
     cudaEvent_t ev[8];
-    KScalars* h_S = nullptr;  // pinned host mirror (2 entries)
+    KScalars* h_S = nullptr;  // pinned host mirror (2 entries; then the fused momentum solve's 3)
     double* h_res = nullptr;  // pinned
     // optional per-kernel event timing (xcal_case_set_profiling)
     bool profiling = false;
@@ -335,12 +338,6 @@ struct Case {
         DBuf<double> diag, dx, vec, part0, part1, res;  // diagonals of the components; vectors of components 1, 2
         DBuf<float> diag32, vec32;
         DBuf<KScalars> S;
-        KScalars* hS = nullptr;  // pinned
-        double* hres = nullptr;  // pinned
-        ~Fused() {
-            if (hS) cudaFreeHost(hS);
-            if (hres) cudaFreeHost(hres);
-        }
     } bf;
     int apart = -1;  // components_apart(), once known
     bool use_fused(const Equation& E, const xcal_solver_setup& SS);

@@ -1415,8 +1415,8 @@ constexpr int RES_HALO_MAX = RES_HALO_PT * RES_THREADS;
 constexpr int RES_SMEM_MAX = 226 * 1024;
 template <class T>
 __host__ __device__ constexpr size_t res_smem_bytes(int slots, int halo) {
-    // products (double per row), z, directions of rows and halo, values, local columns
-    return RED_TILE * sizeof(double) + RED_TILE * sizeof(T) + ((size_t)(RED_TILE + halo) * sizeof(T) + 15) / 16 * 16 +
+    // products (double per row), z of rows and halo, directions of both, values, local columns
+    return RED_TILE * sizeof(double) + 2 * (((size_t)(RED_TILE + halo) * sizeof(T) + 15) / 16 * 16) +
            ((size_t)slots * sizeof(T) + 15) / 16 * 16 + (size_t)slots * sizeof(unsigned short);
 }
 
@@ -1515,8 +1515,12 @@ __device__ __forceinline__ double res_exchange_cl(double tot, const TileCtx& tc,
 }
 
 // CL: the system's tiles are the blocks of one thread-block cluster; z and the
-// partials travel through distributed shared memory (a halo entry is read
-// from its owner's z), with no trip to L2 in an iteration.
+// partials travel through distributed shared memory, with no trip to L2 in an
+// iteration.  The owner of a row writes its z into the halo entries that read
+// it (27,025 rows: 6.6 us per iteration; 7.7 us when the entries were read
+// from their owners at the start of the next iteration).  The same through L2,
+// with a tag beside each z, measured slower than a coalesced z array behind
+// the <r, z> exchange's release (62,403 rows: 19.4 against 18.5 ms per pass).
 template <class T, bool CL>
 __device__ __forceinline__ void cg_resident_body(const TileCtx& tc, const CSRView& A, const T* __restrict__ nz,
                                                  const T* __restrict__ Pj, int jacobi, T* x, const T* r, T* z, const T* pg,
@@ -1524,10 +1528,9 @@ __device__ __forceinline__ void cg_resident_body(const TileCtx& tc, const CSRVie
                                                  int halo, unsigned char* smem) {
     __shared__ double sm8[8];
     __shared__ ResState st;
-    __shared__ int sh_halo;
     double* pr = reinterpret_cast<double*>(smem);
     T* z_s = reinterpret_cast<T*>(smem + RED_TILE * sizeof(double));
-    T* dir = z_s + RED_TILE;
+    T* dir = reinterpret_cast<T*>((unsigned char*)z_s + ((size_t)(RED_TILE + halo) * sizeof(T) + 15) / 16 * 16);
     __shared__ double cl_part[2][16];
     T* val = reinterpret_cast<T*>((unsigned char*)dir + ((size_t)(RED_TILE + halo) * sizeof(T) + 15) / 16 * 16);
     unsigned short* idx =
@@ -1535,82 +1538,90 @@ __device__ __forceinline__ void cg_resident_body(const TileCtx& tc, const CSRVie
     const int n = A.n, row0 = tc.tile * RED_TILE, e0 = A.slice[row0 / SELL_C];
     if (threadIdx.x == 0) {
         st = ResState{S->gamma, S->beta, S->pNorm2, S->alpha, S->rNorm, S->iter, S->done, S->status, 0};
-        sh_halo = 0;
     }
     __syncthreads();
     if (st.done) return;  // the same in every block
     const int itmax = S->itmax;
     const double eps = S->eps;
     const double epsT = sizeof(T) == 8 ? 2.220446049250313e-16 : 1.1920928955078125e-07;  // eps(T)
-    // the tile's slots and this thread's rows; halo columns listed in pr (as ints)
+    const int h0 = tc.ntiles > 1 ? A.hoff[tc.tile] : 0, nh = tc.ntiles > 1 ? A.hoff[tc.tile + 1] - h0 : 0;
+    // the tile's slots and this thread's rows; the halo entries' first
+    // directions, p_0, straight into dir, their columns into pr (as ints)
     int* hcol = reinterpret_cast<int*>(pr);
     int lb[RES_ROWS], ln[RES_ROWS];
-    T xi[RES_ROWS], ri[RES_ROWS], Pi[RES_ROWS], zi[RES_ROWS], pi[RES_ROWS], qi[RES_ROWS];
+    T xi[RES_ROWS], ri[RES_ROWS], Pi[RES_ROWS], pi[RES_ROWS], qi[RES_ROWS];
 #pragma unroll
     for (int j = 0; j < RES_ROWS; ++j) {
         const int i = row0 + j * RES_THREADS + threadIdx.x;
         lb[j] = ln[j] = 0;
-        xi[j] = ri[j] = zi[j] = pi[j] = qi[j] = T(0);
+        xi[j] = ri[j] = pi[j] = qi[j] = T(0);
         Pi[j] = T(1);
         if (i < n) {
             const int b = row_base(A, i);
             lb[j] = b - e0;
             ln[j] = A.len[i];
+            int h = A.rowh[i];
             for (int t = 0; t < ln[j]; ++t) {
                 const int c = ld_stream(A.colval + b + SELL_C * t);
                 int li = c - row0;
                 if (li < 0 || li >= RED_TILE) {
-                    const int h = atomicAdd(&sh_halo, 1);
                     hcol[h] = c;
-                    li = RED_TILE + h;
+                    li = RED_TILE + h++;
+                    dir[li] = __ldcg(pg + c);
                 }
                 idx[lb[j] + SELL_C * t] = (unsigned short)li;
                 val[lb[j] + SELL_C * t] = ld_stream(nz + b + SELL_C * t);
             }
             xi[j] = x[i];
             ri[j] = r[i];
-            zi[j] = z[i];
             pi[j] = pg[i];
             if (jacobi) Pi[j] = Pj[i];
         }
     }
     __syncthreads();
-    const int nh = sh_halo;
-    int hc[RES_HALO_PT];
+    // this thread's halo entries.  CL: where each one's z goes (the row whose z
+    // it takes, the rank and entry it is written to); else the column it reads
+    int hto[RES_HALO_PT], hrow[RES_HALO_PT];
 #pragma unroll
     for (int u = 0; u < RES_HALO_PT; ++u) {
         const int h = u * RES_THREADS + threadIdx.x;
-        hc[u] = h < nh ? hcol[h] : -1;
+        hto[u] = -1;
+        hrow[u] = 0;
+        if (h < nh) {
+            if constexpr (CL) {
+                const int g = A.hdst[h0 + h];
+                int k = 0;
+                while (g >= A.hoff[k + 1]) ++k;
+                hto[u] = k << 16 | (g - A.hoff[k]);
+                hrow[u] = A.hrow[h0 + h];
+            } else {
+                hto[u] = hcol[h];
+            }
+        }
     }
     __syncthreads();
     // every block of the cluster runs before any touches another's shared memory
     if (CL && tc.ntiles > 1) cooperative_groups::this_cluster().sync();
     // p_k of the halo and of this thread's rows (kaxpby!, cg_dir); the first
-    // direction is what cg_start left in pg
-    T hp[RES_HALO_PT];
-#pragma unroll
-    for (int u = 0; u < RES_HALO_PT; ++u) hp[u] = hc[u] >= 0 ? __ldcg(pg + hc[u]) : T(0);
+    // directions are in place
     for (int ran = 0; ran < max_iters; ++ran) {
         if (ran > 0) {
             const T b = (T)st.beta;
             T hz[RES_HALO_PT];
 #pragma unroll
             for (int u = 0; u < RES_HALO_PT; ++u)
-                if (hc[u] >= 0)
-                    hz[u] = CL ? *cooperative_groups::this_cluster().map_shared_rank(z_s + hc[u] % RED_TILE,
-                                                                                    hc[u] / RED_TILE)
-                               : __ldcg(z + hc[u]);
+                if (hto[u] >= 0) hz[u] = CL ? z_s[RED_TILE + u * RES_THREADS + threadIdx.x] : __ldcg(z + hto[u]);
 #pragma unroll
-            for (int j = 0; j < RES_ROWS; ++j) pi[j] = zi[j] + b * pi[j];
+            for (int j = 0; j < RES_ROWS; ++j) pi[j] = z_s[j * RES_THREADS + threadIdx.x] + b * pi[j];
 #pragma unroll
             for (int u = 0; u < RES_HALO_PT; ++u)
-                if (hc[u] >= 0) hp[u] = hz[u] + b * hp[u];
+                if (hto[u] >= 0) {
+                    const int l = RED_TILE + u * RES_THREADS + threadIdx.x;
+                    dir[l] = hz[u] + b * dir[l];
+                }
         }
 #pragma unroll
         for (int j = 0; j < RES_ROWS; ++j) dir[j * RES_THREADS + threadIdx.x] = pi[j];
-#pragma unroll
-        for (int u = 0; u < RES_HALO_PT; ++u)
-            if (hc[u] >= 0) dir[RED_TILE + u * RES_THREADS + threadIdx.x] = hp[u];
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < RES_ROWS; ++j) {
@@ -1646,14 +1657,19 @@ __device__ __forceinline__ void cg_resident_body(const TileCtx& tc, const CSRVie
             const int i = row0 + j * RES_THREADS + threadIdx.x;
             xi[j] = xi[j] + a * pi[j];
             ri[j] = ri[j] + (-a) * qi[j];
-            zi[j] = jacobi ? Pi[j] * ri[j] : ri[j];
-            if constexpr (CL)
-                z_s[j * RES_THREADS + threadIdx.x] = zi[j];
-            else if (tc.ntiles > 1 && i < n)
-                z[i] = zi[j];
-            pr[j * RES_THREADS + threadIdx.x] = ln[j] ? (double)ri[j] * (double)zi[j] : 0.0;
+            const T zi = jacobi ? Pi[j] * ri[j] : ri[j];
+            z_s[j * RES_THREADS + threadIdx.x] = zi;
+            if (!CL && tc.ntiles > 1 && i < n) z[i] = zi;
+            pr[j * RES_THREADS + threadIdx.x] = ln[j] ? (double)ri[j] * (double)zi : 0.0;
         }
         __syncthreads();
+        if constexpr (CL) {
+#pragma unroll
+            for (int u = 0; u < RES_HALO_PT; ++u)
+                if (hto[u] >= 0)
+                    *cooperative_groups::this_cluster().map_shared_rank(z_s + RED_TILE + (hto[u] & 0xffff),
+                                                                        hto[u] >> 16) = z_s[hrow[u]];
+        }
         tot = res_tile_sum(pr, sm8);
         double g = 0.0;
         if constexpr (CL) g = res_exchange_cl(tot, tc, cl_part[1]);

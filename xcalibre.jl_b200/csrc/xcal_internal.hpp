@@ -160,6 +160,14 @@ struct CSRView {
     // the resident CG
     int tile_slots;
     int tile_halo;
+    // the off-tile slots ("halo entries"), tile by tile in row and slot order:
+    // tile t's are hoff[t] .. hoff[t+1]; rowh[r] of them precede row r in its
+    // tile; entry g sits in local row hrow[g], its transposed slot is entry
+    // hdst[g] (of another tile)
+    const int* hoff;
+    const int* hdst;
+    const unsigned short* hrow;
+    const unsigned short* rowh;
 };
 // slot of entry 0 of row r (entry k is at row_base + SELL_C*k)
 __host__ __device__ __forceinline__ int row_base(const CSRView& A, int r) {

@@ -593,7 +593,9 @@ int32_t xcal_case_stream(const xcal_case* cs, void** stream);
  * the steady-state CUDA-graph chunks only sampled iterations are timed. */
 int32_t xcal_case_set_profiling(xcal_case* cs, int32_t enable);
 /* graph mode (off by default): each xcal_simple_iterate iteration /
- * xcal_piso_step step replays one CUDA graph captured on first use.  The
+ * xcal_piso_step step replays one CUDA graph captured on first use; when off,
+ * the library drives a step from the host or, where that is faster (FP64 cases
+ * of at most 524,288 cells, from their third step on), replays it too.  The
  * Krylov loops run as conditional WHILE nodes whose stopping tests are taken
  * on the device (at most itmax/4 + 2 loop bodies), so a step needs one host
  * synchronisation.  Results are identical to the default mode.  Per-kernel

@@ -568,9 +568,10 @@ __global__ void k_bf_loop_cond(cudaGraphConditionalHandle h, KScalars* S, int ca
     cudaGraphSetConditional(h, any ? 1u : 0u);
 }
 template <int NC>
-__global__ void k_bf_record(const KScalars* S, int* out) {
+__global__ void k_bf_record(const KScalars* S, int* out, int* hits) {
     const int d = threadIdx.x;
     if (blockIdx.x != 0 || d >= NC) return;
+    if (S[d].status == KS_TIRED) atomicAdd(hits, 1);
     out[2 * d] = S[d].iter;
     out[2 * d + 1] = S[d].status;
 }
@@ -812,7 +813,7 @@ void Case::fused_solve(Equation& E, const xcal_solver_setup& SS, const SolveRef*
             XCAL_CHECK_LAUNCH();
         });
         bf_finish(stream, V);
-        k_bf_record<NC><<<1, 32, 0, stream>>>(V.S, giters.p + 2 * R[0].slot);
+        k_bf_record<NC><<<1, 32, 0, stream>>>(V.S, giters.p + 2 * R[0].slot, giters.p + 2 * GRES_N);
         XCAL_CHECK_LAUNCH();
         for (int d = 0; d < NC; ++d) res[d] = 0.0;
         return;

@@ -446,7 +446,13 @@ int32_t xcal_case_set_persistent(xcal_case* cs, int32_t mode) {
     if (mode != 0 && mode != 1 && mode != 2 && mode != PERSIST_MT1024 && mode != PERSIST_MT512 && mode != 256 &&
         mode != 512 && mode != 1024)
         return XCAL_ERR_INVALID;
-    cs->c->persistent_cg = mode;
+    Case* c = cs->c.get();
+    if (mode != c->persistent_cg && c->step_graph) {  // a captured step holds the previous form
+        c->sync();
+        cudaGraphExecDestroy(c->step_graph);
+        c->step_graph = nullptr;
+    }
+    c->persistent_cg = mode;
     return XCAL_OK;
 }
 

@@ -943,11 +943,11 @@ Case::Case(xcal_ctx* c, const DevMesh* m, const xcal_config* cf) : ctx(c), mesh(
     cmax_ctr.zero(stream);
     gres.alloc(GRES_N);
     gres.zero(stream);
-    giters.alloc(2 * GRES_N);
+    giters.alloc(2 * GRES_N + 1);
     giters.zero(stream);
     dlaunch.alloc(1);
     dlaunch.zero(stream);
-    XCAL_CUDA(cudaMallocHost(&h_iters, 2 * GRES_N * sizeof(int)));
+    XCAL_CUDA(cudaMallocHost(&h_iters, (2 * GRES_N + 1) * sizeof(int)));
     XCAL_CUDA(cudaMallocHost(&h_launch, sizeof(unsigned long long)));
     XCAL_CUDA(cudaMallocHost(&h_perr, sizeof(int)));
     // host-side per-cell constants: V^(1/3) (Courant) and the LES filter
@@ -1883,7 +1883,7 @@ void Case::solve_captured(int eqn, int comp) {
         });
     }
     kr_residual(stream, A, E.nz.p, field, b, S, ws.part0.p, ws.part1.p, gres.p + slot);
-    kr_record(stream, S, giters.p + 2 * slot);
+    kr_record(stream, S, giters.p + 2 * slot, giters.p + 2 * GRES_N);
 }
 
 // apply_smoother!(setup.smoother, values, A, b) (Solve_1_api.jl:284): the
@@ -2332,23 +2332,23 @@ double Case::max_courant() {
 }
 
 // One SIMPLE iteration's launches (Solvers_1_SIMPLE.jl:164-240).  Eager:
-// residuals returned, phases timed with events.  Under capture: residuals
-// land in gres, no events.
-void Case::simple_body(double r3[3], double& rp, bool timed) {
+// residuals returned.  Under capture: residuals land in gres.  Phases timed
+// with events either way (event nodes in a graph).
+void Case::simple_body(double r3[3], double& rp) {
     NvtxRange range("SIMPLE iteration");
-    if (timed) XCAL_CUDA(cudaEventRecord(ev[0], stream));
+    mark(0);
     {
         NvtxRange r("momentum predictor");
         solve_equation_U(r3);
     }
-    if (timed) XCAL_CUDA(cudaEventRecord(ev[1], stream));
+    mark(1);
     {
         NvtxRange r("pressure predictor + flux divergence");
         pressure_predictor(true);
         flux_divergence();
     }
     XCAL_CUDA(cudaMemcpyAsync(prev.p, p.p, mesh->nC * sizeof(double), cudaMemcpyDeviceToDevice, stream));
-    if (timed) XCAL_CUDA(cudaEventRecord(ev[2], stream));
+    mark(2);
     {
         NvtxRange r("pressure equation");
         rp = solve_equation_p();
@@ -2356,13 +2356,13 @@ void Case::simple_body(double r3[3], double& rp, bool timed) {
         grad_p();
         nonorth_correctors(rp);
     }
-    if (timed) XCAL_CUDA(cudaEventRecord(ev[3], stream));
+    mark(3);
     {
         NvtxRange r("correction + turbulence");
         correct();
         turbulence();
     }
-    if (timed) XCAL_CUDA(cudaEventRecord(ev[4], stream));
+    mark(4);
 }
 
 // One PISO time step's launches (Solvers_2_PISO.jl:108-187); the Courant
@@ -2417,11 +2417,12 @@ void Case::capture_step() {
     XCAL_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     try {
         XCAL_CUDA(cudaMemsetAsync(ws.err.p, 0, sizeof(int), stream));
+        XCAL_CUDA(cudaMemsetAsync(giters.p + 2 * GRES_N, 0, sizeof(int), stream));
         double r3[3], rp;
         if (cfg.algorithm == XCAL_ALGO_PISO)
             piso_body(r3, rp);
         else
-            simple_body(r3, rp, false);
+            simple_body(r3, rp);
     } catch (...) {
         capturing = false;
         cudaStreamEndCapture(stream, &g);
@@ -2443,11 +2444,12 @@ void Case::capture_step() {
 // Courant number, the solves' iteration counts and the body-kernel count.
 void Case::run_step_graph(double res[4], double* courant) {
     capture_step();
-    XCAL_CUDA(cudaEventRecord(ev[0], stream));
+    const bool simple = cfg.algorithm != XCAL_ALGO_PISO;  // its graph times its own phases
+    if (!simple) XCAL_CUDA(cudaEventRecord(ev[0], stream));
     XCAL_CUDA(cudaGraphLaunch(step_graph, stream));
-    XCAL_CUDA(cudaEventRecord(ev[1], stream));
+    if (!simple) XCAL_CUDA(cudaEventRecord(ev[1], stream));
     XCAL_CUDA(cudaMemcpyAsync(h_res, gres.p, GRES_N * sizeof(double), cudaMemcpyDeviceToHost, stream));
-    XCAL_CUDA(cudaMemcpyAsync(h_iters, giters.p, 2 * GRES_N * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    XCAL_CUDA(cudaMemcpyAsync(h_iters, giters.p, (2 * GRES_N + 1) * sizeof(int), cudaMemcpyDeviceToHost, stream));
     XCAL_CUDA(cudaMemcpyAsync(h_launch, dlaunch.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
     XCAL_CUDA(cudaMemsetAsync(dlaunch.p, 0, sizeof(unsigned long long), stream));
     XCAL_CUDA(cudaMemcpyAsync(h_perr, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
@@ -2456,17 +2458,70 @@ void Case::run_step_graph(double res[4], double* courant) {
     long long nk = step_top_kernels + (long long)h_launch[0];
     g_launch_count.fetch_add(nk, std::memory_order_relaxed);
     t_launch_count += nk;
-    float t = 0;
-    cudaEventElapsedTime(&t, ev[0], ev[1]);
-    ms[5] += t;
-    for (int k = 0; k < 4; ++k) {
-        res[k] = h_res[k];
-        last_iters[k] = h_iters[2 * k];
-        if (h_iters[2 * k + 1] == KS_LOOP_CAP)
-            fail(XCAL_ERR_TIMEOUT, "a Krylov solve did not finish within its loop-body cap");
-        note_status(k, h_iters[2 * k + 1]);
+    if (simple) {
+        add_phases();
+    } else {
+        float t = 0;
+        cudaEventElapsedTime(&t, ev[0], ev[1]);
+        ms[5] += t;
     }
+    // (result slot, system index) of the step's solves
+    const int solved[][2] = {{0, 0}, {1, 1}, {2, 2}, {GRES_P, 3}, {GRES_K, 4}, {GRES_OMEGA, 5}, {GRES_KL, 7}};
+    const int nsolved = !has_k() ? 4 : !rans_kw() ? 5 : !lke() ? 6 : 7;
+    for (int q = 0; q < nsolved; ++q) {
+        const int slot = solved[q][0], gk = solved[q][1];
+        if (h_iters[2 * slot + 1] == KS_LOOP_CAP)
+            fail(XCAL_ERR_TIMEOUT, "a Krylov solve did not finish within its loop-body cap");
+        last_iters[gk] = h_iters[2 * slot];
+        last_status[gk] = h_iters[2 * slot + 1];
+    }
+    itmax_hits += h_iters[2 * GRES_N];  // every solve of the step, correctors included
+    for (int k = 0; k < 4; ++k) res[k] = h_res[k];
+    if (has_k()) res_k = h_res[GRES_K];
+    if (rans_kw()) res_omega = h_res[GRES_OMEGA];
+    if (lke()) res_kl = h_res[GRES_KL];
     if (courant) *courant = h_res[GRES_CO];
+}
+
+// phase event k of a SIMPLE iteration
+void Case::mark(int k) {
+    if (capturing)
+        XCAL_CUDA(cudaEventRecordWithFlags(ev[k], stream, cudaEventRecordExternal));
+    else
+        XCAL_CUDA(cudaEventRecord(ev[k], stream));
+}
+void Case::add_phases() {
+    float a = 0, b = 0, c = 0, d = 0;
+    cudaEventElapsedTime(&a, ev[0], ev[1]);
+    cudaEventElapsedTime(&b, ev[1], ev[2]);
+    cudaEventElapsedTime(&c, ev[2], ev[3]);
+    cudaEventElapsedTime(&d, ev[3], ev[4]);
+    ms[1] += a;
+    ms[3] += b + d;
+    ms[2] += c;
+    ms[5] += a + b + c + d;
+}
+
+// Whether this iteration replays the step graph: in graph mode, and otherwise
+// from the third iteration on where launches and host round trips are a good
+// part of it.  Measured on B200 (ms per pass, host-driven / graph): 1,073 cells
+// 5.6 / 4.7 (10 iterations), 7,500 cells with k, omega and kl 10.4 / 8.9 (5),
+// 116,440 cells DILU-CG 25.5 / 22.8 (3); the capture costs about 1 ms once.  Not
+// in mixed precision, whose captured momentum solves are not fused (262,144
+// cells 18.9 / 20.3), nor above BF_MAX_ROWS (no difference at 2.1M cells).
+bool Case::replay_step() {
+    if (graph_mode) return true;
+    if (no_auto_graph || profiling || batch_err || iteration < 3 || cfg.precision != XCAL_PREC_FP64 ||
+        mesh->nC > BF_MAX_ROWS || !kr_coop_capture_ok(false) || !kr_cluster_capture_ok(false))
+        return false;
+    try {
+        capture_step();
+    } catch (const Error&) {  // what cannot be captured runs host-driven
+        cudaGetLastError();
+        no_auto_graph = true;
+        return false;
+    }
+    return true;
 }
 
 bool Case::simple_iteration(double res[4]) {  // Solvers_1_SIMPLE.jl:164-240
@@ -2474,7 +2529,7 @@ bool Case::simple_iteration(double res[4]) {  // Solvers_1_SIMPLE.jl:164-240
     autotune();
     iteration += 1;
     double r3[3], rp;
-    if (graph_mode) {
+    if (replay_step()) {
         double r[4];
         run_step_graph(r, nullptr);
         r3[0] = r[0];
@@ -2482,17 +2537,9 @@ bool Case::simple_iteration(double res[4]) {  // Solvers_1_SIMPLE.jl:164-240
         r3[2] = r[2];
         rp = r[3];
     } else {
-        simple_body(r3, rp, true);
+        simple_body(r3, rp);
         sync();
-        float a = 0, b = 0, c = 0, d = 0;
-        cudaEventElapsedTime(&a, ev[0], ev[1]);
-        cudaEventElapsedTime(&b, ev[1], ev[2]);
-        cudaEventElapsedTime(&c, ev[2], ev[3]);
-        cudaEventElapsedTime(&d, ev[3], ev[4]);
-        ms[1] += a;
-        ms[3] += b + d;
-        ms[2] += c;
-        ms[5] += a + b + c + d;
+        add_phases();
     }
     res[0] = r3[0];
     res[1] = r3[1];
@@ -2513,7 +2560,7 @@ double Case::piso_step(double res[4]) {  // Solvers_2_PISO.jl:108-187
     iteration += 1;
     time = time + cfg.dt;
     double r3[3], rp, co;
-    if (graph_mode) {
+    if (replay_step()) {
         double r[4];
         run_step_graph(r, &co);
         r3[0] = r[0];

@@ -371,7 +371,7 @@ struct Case {
     // round trip until its residuals are read.
     enum { GRES_U = 0, GRES_P = 3, GRES_CO = 4, GRES_K = 5, GRES_OMEGA = 6, GRES_KL = 7, GRES_N = 8 };
     DBuf<double> gres;          // per-step results: U x,y,z and p residuals, max Courant
-    DBuf<int> giters;           // (iterations, status) of the step's 4 solves
+    DBuf<int> giters;           // (iterations, status) per result slot; then how many solves stopped at itmax
     DBuf<unsigned int> cmax_ctr;
     DBuf<unsigned long long> dlaunch;  // kernels run inside WHILE bodies (graph mode)
     long long step_top_kernels = 0;    // kernels of a step graph outside WHILE bodies
@@ -386,7 +386,11 @@ struct Case {
     int* h_perr = nullptr;      // pinned: persistent CG error flag after a graph replay
     long long body_kernels_captured = 0;
     long long last_body_kernels = 0;  // kernels captured into the last WHILE body
-    void simple_body(double r3[3], double& rp, bool timed);
+    void simple_body(double r3[3], double& rp);
+    void mark(int k);
+    void add_phases();
+    bool replay_step();
+    bool no_auto_graph = false;  // a capture failed: replay_step() leaves this case host-driven
     void piso_body(double r3[3], double& rp);
     void set_graph_mode(bool on);
     void courant_to_slot();

@@ -336,7 +336,7 @@ void kr_outer_prep(cudaStream_t s, KScalars* S);
 void kr_correct_masked(cudaStream_t s, int n, double* field, const float* x, const KScalars* S);
 void kr_outer_cond(cudaStream_t s, cudaGraphConditionalHandle h, KScalars* S, int max_outer, int body_kernels,
                    unsigned long long* launches);
-void kr_record(cudaStream_t s, const KScalars* S, int* out);
+void kr_record(cudaStream_t s, const KScalars* S, int* out, int* hits);
 
 // ---- mixed precision: FP32 inner CG on the Jacobi-scaled system (cg_folded.cu)
 // Off-diagonal entries of Ahat = M^1/2 A M^1/2 (M = diag(1/|a_ii|)) in

@@ -643,9 +643,11 @@ __global__ void k_outer_cond(cudaGraphConditionalHandle h, KScalars* S, int max_
     cudaGraphSetConditional(h, stop ? 0u : 1u);
 }
 
-// iterations and status of the finished solve into out[0..1]
-__global__ void k_record(const KScalars* S, int* out) {
+// iterations and status of the finished solve into out[0..1]; hits counts the
+// solves that stopped at itmax
+__global__ void k_record(const KScalars* S, int* out, int* hits) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    if (S->status == KS_TIRED) *hits += 1;
     out[0] = S->mixed ? S->total : S->iter;
     out[1] = S->status;
 }
@@ -1360,8 +1362,8 @@ void kr_outer_cond(cudaStream_t s, cudaGraphConditionalHandle h, KScalars* S, in
     k_outer_cond<<<1, 32, 0, s>>>(h, S, max_outer, body_kernels, launches);
     XCAL_CHECK_LAUNCH();
 }
-void kr_record(cudaStream_t s, const KScalars* S, int* out) {
-    k_record<<<1, 32, 0, s>>>(S, out);
+void kr_record(cudaStream_t s, const KScalars* S, int* out, int* hits) {
+    k_record<<<1, 32, 0, s>>>(S, out, hits);
     XCAL_CHECK_LAUNCH();
 }
 

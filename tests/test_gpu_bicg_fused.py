@@ -68,13 +68,15 @@ def test_fused_mixed(x, ctx, name, pre, rtol):
     mesh = x.build_mesh3(MESHES[name](x))
     cfg, keep = _config(x, mesh, getattr(x, pre), rtol, "mixed")
     outs = []
-    for separate in (True, False):
+    for separate, graph in ((True, False), (False, False), (False, True)):
         dm = x.DeviceMesh(ctx, mesh)
         c = x.Case(dm, cfg)
         c.set_inner_cg(1)
         c.set_profiling(separate)
+        c.set_graph_mode(graph)
         outs.append(_run(x, c, mesh) + (c.solve_report()["iterations"],))
         c.close()
         dm.close()
-    for a, b in zip(*outs):
-        assert np.array_equal(a, b)
+    for out in outs[1:]:
+        for a, b in zip(outs[0], out):
+            assert np.array_equal(a, b)

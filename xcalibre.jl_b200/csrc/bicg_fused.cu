@@ -3,10 +3,9 @@
 // in the diagonal alone), or one transported scalar.
 //
 // A momentum solve to a tenth of its residual takes one or two BiCGSTAB
-// iterations (Krylov.jl bicgstab!, Solve_1_api.jl:268-307), so on meshes up to
-// some 500k cells its cost is latency: about 25 launches, three dependent
-// DILU applications and several host round trips per component, one component
-// after the other.  Here
+// iterations (Krylov.jl bicgstab!, Solve_1_api.jl:268-307), so its cost is
+// latency: about 25 launches, three dependent DILU applications and several
+// host round trips per component, one component after the other.  Here
 //   * the components run side by side: a row's slots are read once for all
 //     three, and their DILU dataflows (krylov_bodies.cuh) overlap;
 //   * an iteration is five launches: A p with M^-1 (k_bf_flow), alpha,
@@ -29,7 +28,9 @@
 // between them.  Measured on B200, momentum solve per SIMPLE iteration (one
 // BiCGSTAB iteration per component, DILU), this against the components one by
 // one: 1,073 cells FP64 0.25 / 0.55 ms, 27,025 cells 0.40 / 0.80 ms, 262,144
-// cells mixed 0.67 / 1.19 ms.
+// cells mixed 0.67 / 1.19 ms, 2.1M cells mixed 2.24 / 3.50 ms.  Captured (graph
+// mode; mixed: an outer WHILE over the defect-correction steps), LES at 884,736
+// cells, a step: 7.6 -> 6.3 ms.
 #include <algorithm>
 #include <cstring>
 
@@ -122,14 +123,19 @@ __global__ void k_bf_refresh(BfRefresh R) {
         }
 }
 
-// the components whose solve goes on (bit mask); the same in every block: no
-// kernel that reads it changes it
+// whether component d takes part, and the components that do (or, running: whose
+// solve goes on) as a bit mask; the same in every block: no kernel that reads
+// them changes them
 template <class T, int NC>
-__device__ __forceinline__ int bf_running(const BfView<T, NC>& V) {
+__device__ __forceinline__ bool bf_active(const BfView<T, NC>& V, int d) {
+    return (V.active >> d & 1) && !V.S[d].off;
+}
+template <class T, int NC>
+__device__ __forceinline__ int bf_mask(const BfView<T, NC>& V, bool running) {
     int m = 0;
 #pragma unroll
     for (int d = 0; d < NC; ++d)
-        if ((V.active >> d & 1) && !V.S[d].done) m |= 1 << d;
+        if (bf_active(V, d) && !(running && V.S[d].done)) m |= 1 << d;
     return m;
 }
 
@@ -188,7 +194,7 @@ __device__ __forceinline__ bool bf_wait(T* const (&ys)[NC], int run, const int* 
 template <class T, int NC, int PRE, int MODE>
 __global__ void __launch_bounds__(FLOW_THREADS) k_bf_flow(const __grid_constant__ BfView<T, NC> V) {
     __shared__ int sh_err;
-    const int run = MODE == 0 ? V.active : bf_running(V);
+    const int run = bf_mask(V, MODE != 0);
     if (!run) return;
     const int n = V.A.n;
     const int start = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -366,7 +372,7 @@ __global__ void __launch_bounds__(BF_NT) k_bf_start(const __grid_constant__ BfVi
     __shared__ double sm[8];
     const int d = blockIdx.y, n = V.A.n, nt = gridDim.x;
     if (blockIdx.x == 0 && d == 0 && threadIdx.x == 0) V.bar[0] = 0u;
-    if (!(V.active >> d & 1)) return;
+    if (!bf_active(V, d)) return;
 #pragma unroll
     for (int j = 0; j < BF_IPT; ++j) {
         const int l = j * BF_NT + threadIdx.x, i = blockIdx.x * RED_TILE + l;
@@ -399,7 +405,7 @@ __global__ void __launch_bounds__(BF_NT) k_bf_alpha(const __grid_constant__ BfVi
     __shared__ double sm[8];
     const int d = blockIdx.y, n = V.A.n, nt = gridDim.x;
     if (blockIdx.x == 0 && d == 0 && threadIdx.x == 0) V.bar[0] = 0u;
-    if (!(V.active >> d & 1) || V.S[d].done) return;
+    if (!bf_active(V, d) || V.S[d].done) return;
 #pragma unroll
     for (int j = 0; j < BF_IPT; ++j) {
         const int l = j * BF_NT + threadIdx.x, i = blockIdx.x * RED_TILE + l;
@@ -420,7 +426,7 @@ __global__ void __launch_bounds__(BF_NT) k_bf_omega(const __grid_constant__ BfVi
     __shared__ double pr[2][RED_TILE];
     __shared__ double sm[8];
     const int d = blockIdx.y, n = V.A.n, nt = gridDim.x;
-    if (!(V.active >> d & 1) || V.S[d].done) return;
+    if (!bf_active(V, d) || V.S[d].done) return;
 #pragma unroll
     for (int j = 0; j < BF_IPT; ++j) {
         const int l = j * BF_NT + threadIdx.x, i = blockIdx.x * RED_TILE + l;
@@ -446,7 +452,7 @@ __global__ void __launch_bounds__(BF_NT) k_bf_xr(const __grid_constant__ BfView<
     __shared__ double pr[2][RED_TILE];
     __shared__ double sm[8];
     const int d = blockIdx.y, n = V.A.n, nt = gridDim.x;
-    if (!(V.active >> d & 1) || V.S[d].done) return;
+    if (!bf_active(V, d) || V.S[d].done) return;
     const double omega = V.S[d].omega;
     const T om = (T)omega;
 #pragma unroll
@@ -481,7 +487,7 @@ template <class T, int NC>
 __global__ void __launch_bounds__(BF_NT) k_bf_p(const __grid_constant__ BfView<T, NC> V) {
     const int d = blockIdx.y, n = V.A.n;
     if (blockIdx.x == 0 && d == 0 && threadIdx.x == 0) V.bar[0] = 0u;
-    if (!(V.active >> d & 1) || V.S[d].done || V.S[d].iter == 0) return;
+    if (!bf_active(V, d) || V.S[d].done || V.S[d].iter == 0) return;
     const T beta = (T)V.S[d].beta, omega = (T)V.S[d].omega;
 #pragma unroll
     for (int j = 0; j < BF_IPT; ++j) {
@@ -499,7 +505,7 @@ __global__ void __launch_bounds__(BF_NT) k_bf_finish(const __grid_constant__ BfV
     __shared__ double pr[2][RED_TILE];
     __shared__ double sm[8];
     const int d = blockIdx.y, n = V.A.n, nt = gridDim.x;
-    if (!(V.active >> d & 1) || !V.S[d].done) return;
+    if (!bf_active(V, d) || !V.S[d].done) return;
     const bool apply = sizeof(T) == 8 || !V.S[d].outer_conv;
     const T* x = V.x[d];
     const double* dx = V.dx[d];
@@ -558,6 +564,7 @@ __global__ void k_bf_loop_cond(cudaGraphConditionalHandle h, KScalars* S, int ca
     atomicAdd(launches, (unsigned long long)body_kernels);
     bool any = false;
     for (int d = 0; d < NC; ++d) {
+        if (S[d].off) continue;
         S[d].loops = S[d].loops + 1;
         if (!S[d].done && S[d].loops >= cap) {
             S[d].done = 1;
@@ -567,12 +574,48 @@ __global__ void k_bf_loop_cond(cudaGraphConditionalHandle h, KScalars* S, int ca
     }
     cudaGraphSetConditional(h, any ? 1u : 0u);
 }
+// one defect-correction step of the components still in it (solve_mixed's
+// loop, on the device): its start, and its exit tests
+template <int NC>
+__global__ void k_bf_outer_prep(KScalars* S, unsigned int* bar) {
+    const int d = threadIdx.x;
+    if (blockIdx.x != 0 || d >= NC) return;
+    if (d == 0) bar[0] = 0u;
+    if (S[d].off) return;
+    S[d].iter = 0;
+    S[d].done = 0;
+    S[d].status = KS_RUNNING;
+}
+template <int NC>
+__global__ void k_bf_outer_cond(cudaGraphConditionalHandle h, KScalars* S, int max_outer, int body_kernels,
+                                unsigned long long* launches) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    atomicAdd(launches, (unsigned long long)body_kernels);
+    bool any = false;
+    for (int d = 0; d < NC; ++d) {
+        KScalars& K = S[d];
+        if (K.off) continue;
+        bool stop = K.outer_conv != 0;
+        if (!stop) {
+            K.total = K.total + K.iter;
+            const int st = K.status;
+            stop = st == KS_ZERO_CURV || st == KS_BREAKDOWN || st == KS_TIRED || st == KS_LOOP_CAP ||
+                   (st == KS_SOLVED && K.eps <= K.eps_outer);
+        }
+        K.outer = K.outer + 1;
+        if (stop || K.outer >= max_outer)
+            K.off = 1;
+        else
+            any = true;
+    }
+    cudaGraphSetConditional(h, any ? 1u : 0u);
+}
 template <int NC>
 __global__ void k_bf_record(const KScalars* S, int* out, int* hits) {
     const int d = threadIdx.x;
     if (blockIdx.x != 0 || d >= NC) return;
     if (S[d].status == KS_TIRED) atomicAdd(hits, 1);
-    out[2 * d] = S[d].iter;
+    out[2 * d] = S[d].mixed ? S[d].total : S[d].iter;
     out[2 * d + 1] = S[d].status;
 }
 
@@ -647,17 +690,17 @@ static void bf_finish(cudaStream_t s, const BfView<T, NC>& V) {
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// The fused solve applies where a solve is latency-bound and its form is one
-// the kernels cover: BiCGSTAB without a smoother, on systems up to
-// BF_MAX_ROWS (at 2.1M rows the sweeps' level form is faster, and the matrix
-// streams dominate), DILU as dataflow sweeps.  Profiling times the separate
-// kernels, a batch runs its own batched ones.
+// The fused solve covers BiCGSTAB without a smoother at every size (momentum
+// solve per SIMPLE iteration, components in turn with the fastest DILU form
+// against this, ms: 884,736 cells mixed 2.35 / 1.08, FP64 2.45 / 1.17; 2.1M cells
+// mixed 3.50 / 2.24, FP64 3.95 / 2.74).  A chosen DILU form, and profiling, which
+// times the separate kernels, keep those; a batch runs its own batched ones.
 bool Case::use_fused(const Equation& E, const xcal_solver_setup& SS) {
-    if (SS.solver != XCAL_SOLVER_BICGSTAB || SS.smoother_loops > 0 || profiling || batch_err) return false;
-    if (E.n > BF_MAX_ROWS || dilu_mode != 0) return false;
-    if (capturing && cfg.precision == XCAL_PREC_MIXED) return false;  // its defect correction is a WHILE node
-    if (SS.precond == XCAL_PRECOND_DILU) return E.use_flow && E.flow_D && !E.lower_off.empty() && coop_ok_here();
-    return true;
+    if (SS.solver != XCAL_SOLVER_BICGSTAB || SS.smoother_loops > 0 || profiling || batch_err || dilu_mode != 0)
+        return false;
+    if (SS.precond != XCAL_PRECOND_DILU) return true;
+    // the sweeps are cooperative launches, under capture inside WHILE bodies
+    return E.flow_D && !E.lower_off.empty() && (capturing ? kr_coop_capture_ok(true) : coop_ok_here());
 }
 
 // Components may be solved side by side when no boundary condition of one
@@ -677,25 +720,45 @@ bool Case::components_apart() {
     return apart == 1;
 }
 
-// work vectors of components 1 and 2, and the three diagonals (allocated at the
-// first fused momentum solve, never under capture)
+// work vectors of components 1 and 2, and the three diagonals, allocated at the
+// first fused momentum solve (a case in a batch has none), never under capture;
+// where they would take more than a quarter of the free memory the components
+// are solved in turn
 void Case::reserve_fused() {
-    if (bf.ready || capturing || !use_fused(U, cfg.U_solver) || !components_apart()) return;
+    if (bf.ready || bf.refused || capturing || !use_fused(U, cfg.U_solver) || !components_apart()) return;
     const size_t n = U.n, T = (n + RED_TILE - 1) / RED_TILE;
-    AllocScope acc(&bytes);
-    bf.diag.alloc(3 * n);
-    bf.dx.alloc(2 * n);
-    if (cfg.precision == XCAL_PREC_MIXED) {
-        bf.diag32.alloc(3 * n);
-        bf.vec32.alloc(2 * 9 * n);
-    } else {
-        bf.vec.alloc(2 * 8 * n);
+    const size_t need = n * (cfg.precision == XCAL_PREC_MIXED ? 124 : 168);
+    size_t free_b = 0, total_b = 0, held = 0;
+    XCAL_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (need > free_b / 4) {
+        bf.refused = true;
+        return;
     }
-    bf.part0.alloc(3 * T);
-    bf.part1.alloc(3 * T);
-    bf.S.alloc(3);
-    bf.S.zero(stream);
-    bf.res.alloc(3);
+    try {
+        AllocScope acc(&held);
+        bf.diag.alloc(3 * n);
+        bf.dx.alloc(2 * n);
+        if (cfg.precision == XCAL_PREC_MIXED) {
+            bf.diag32.alloc(3 * n);
+            bf.vec32.alloc(2 * 9 * n);
+        } else {
+            bf.vec.alloc(2 * 8 * n);
+        }
+        bf.part0.alloc(3 * T);
+        bf.part1.alloc(3 * T);
+        bf.S.alloc(3);
+        bf.S.zero(stream);
+        bf.res.alloc(3);
+    } catch (const Error&) {
+        cudaGetLastError();
+        for (DBuf<double>* b : {&bf.diag, &bf.dx, &bf.vec, &bf.part0, &bf.part1, &bf.res}) b->release();
+        bf.diag32.release();
+        bf.vec32.release();
+        bf.S.release();
+        bf.refused = true;
+        return;
+    }
+    bytes += held;
     bf.ready = true;
 }
 
@@ -803,16 +866,31 @@ void Case::fused_solve(Equation& E, const xcal_solver_setup& SS, const SolveRef*
     BfView<T, NC> V = bf_view<T, NC>(E, SS, R);
     bf_refresh<T, NC>(stream, E, V, pre);
     if (capturing) {
-        k_bf_init<NC><<<1, 32, 0, stream>>>(V.S, SS.atol, SS.rtol, itmax, 0, inner_rtol);
+        k_bf_init<NC><<<1, 32, 0, stream>>>(V.S, SS.atol, SS.rtol, itmax, mixed ? 1 : 0, inner_rtol);
         XCAL_CHECK_LAUNCH();
-        bf_start(stream, V, pre);
-        capture_while([&](cudaGraphConditionalHandle h) {
-            const long long k0 = t_launch_count;
-            bf_iterate(stream, V, pre, false);
-            k_bf_loop_cond<NC><<<1, 32, 0, stream>>>(h, V.S, itmax + 2, (int)(t_launch_count - k0) + 1, dlaunch.p);
-            XCAL_CHECK_LAUNCH();
-        });
-        bf_finish(stream, V);
+        auto solve = [&] {
+            bf_start(stream, V, pre);
+            capture_while([&](cudaGraphConditionalHandle h) {
+                const long long k0 = t_launch_count;
+                bf_iterate(stream, V, pre, false);
+                k_bf_loop_cond<NC><<<1, 32, 0, stream>>>(h, V.S, itmax + 2, (int)(t_launch_count - k0) + 1, dlaunch.p);
+                XCAL_CHECK_LAUNCH();
+            });
+            bf_finish(stream, V);
+        };
+        if (mixed)
+            capture_while([&](cudaGraphConditionalHandle h) {
+                const long long k0 = t_launch_count;
+                k_bf_outer_prep<NC><<<1, 32, 0, stream>>>(V.S, V.bar);
+                XCAL_CHECK_LAUNCH();
+                solve();
+                // this body's own kernels (the iterations' bodies count themselves)
+                const int own = (int)(t_launch_count - k0 - last_body_kernels) + 1;
+                k_bf_outer_cond<NC><<<1, 32, 0, stream>>>(h, V.S, 64, own, dlaunch.p);
+                XCAL_CHECK_LAUNCH();
+            });
+        else
+            solve();
         k_bf_record<NC><<<1, 32, 0, stream>>>(V.S, giters.p + 2 * R[0].slot, giters.p + 2 * GRES_N);
         XCAL_CHECK_LAUNCH();
         for (int d = 0; d < NC; ++d) res[d] = 0.0;

@@ -2508,11 +2508,11 @@ void Case::add_phases() {
 // 5.6 / 4.7 (10 iterations), 7,500 cells with k, omega and kl 10.4 / 8.9 (5),
 // 116,440 cells DILU-CG 25.5 / 22.8 (3); the capture costs about 1 ms once.  Not
 // in mixed precision, whose captured momentum solves are not fused (262,144
-// cells 18.9 / 20.3), nor above BF_MAX_ROWS (no difference at 2.1M cells).
+// cells 18.9 / 20.3), nor above REPLAY_MAX_CELLS (no difference at 2.1M cells).
 bool Case::replay_step() {
     if (graph_mode) return true;
     if (no_auto_graph || profiling || batch_err || iteration < 3 || cfg.precision != XCAL_PREC_FP64 ||
-        mesh->nC > BF_MAX_ROWS || !kr_coop_capture_ok(false) || !kr_cluster_capture_ok(false))
+        mesh->nC > REPLAY_MAX_CELLS || !kr_coop_capture_ok(false) || !kr_cluster_capture_ok(false))
         return false;
     try {
         capture_step();

@@ -165,7 +165,8 @@ struct KrylovVecs {
 // the systems of a fused BiCGSTAB solve (bicg_fused.cu)
 template <class T, int NC>
 struct BfView;
-constexpr int BF_MAX_ROWS = 524288;  // largest fused system
+// largest case whose steps are replayed as a graph without being asked
+constexpr int REPLAY_MAX_CELLS = 524288;
 
 struct Case {
     xcal_ctx* ctx = nullptr;
@@ -335,6 +336,7 @@ struct Case {
     // with fewer launches (bicg_fused.cu)
     struct Fused {
         bool ready = false;
+        bool refused = false;  // no memory for it
         DBuf<double> diag, dx, vec, part0, part1, res;  // diagonals of the components; vectors of components 1, 2
         DBuf<float> diag32, vec32;
         DBuf<KScalars> S;

@@ -210,6 +210,7 @@ struct alignas(128) KScalars {
     int iter, itmax, done, status;
     unsigned int counter;                             // last-block ticket
     unsigned int counter2;
+    int off;  // fused solves, graph mode: the component has left the defect-correction loop
 };
 enum {
     KS_RUNNING = 0,

@@ -585,6 +585,7 @@ int32_t xcal_get_launch_count(const xcal_case* cs, int64_t* count);
  * its own CUDA events around library calls */
 int32_t xcal_case_stream(const xcal_case* cs, void** stream);
 /* per-kernel CUDA-event timing of the dominant kernels (off by default).
+ * While on, BiCGSTAB runs as separate kernels, so that each can be timed.
  * which: 0 = CG SpMV (+ p.Ap), 1 = BiCGSTAB SpMV, 2 = DILU sweep levels,
  *        3 = CG vector update (+ Jacobi apply and r.z when fused),
  *        4 = count only: every CG SpMV launch that did work (ms = 0),
@@ -602,13 +603,14 @@ int32_t xcal_case_set_profiling(xcal_case* cs, int32_t enable);
  * profiling does not apply inside the graph. */
 int32_t xcal_case_set_graph_mode(xcal_case* cs, int32_t enable);
 /* persistent CG (on by default): a CG solve with Jacobi or no preconditioner
- * runs as one cooperative launch (grid barriers between the SpMV and update
- * phases, q kept on chip) whenever the system's tiles fit the GPU at once;
- * otherwise, and in graph mode, the two-kernel loop runs.  Same results.
- * mode: 0 off; 1 on: a system of at most 16 tiles of 2048 rows runs as one
- * thread-block cluster (hardware cluster barriers), a larger one in the
+ * runs as one launch whenever the system's tiles fit the GPU at once;
+ * otherwise the two-kernel loop runs.  Same results.
+ * mode: 0 off; 1 on: a system of at most one tile of 2048 rows per SM whose
+ * matrix fits in shared memory keeps it there for the whole solve (up to 16
+ * tiles as one thread-block cluster); otherwise one of at most 16 tiles runs
+ * as one thread-block cluster (hardware cluster barriers), a larger one in the
  * widest cooperative block form whose blocks are co-resident (1024, 512 or
- * 256 threads); 2 = the cluster form only, 256 / 512 / 1024 = that
+ * 256 threads; grid barriers between the SpMV and update phases, q on chip); 2 = the cluster form only, 256 / 512 / 1024 = that
  * cooperative form only, 4 / 5 = one block of 1024 / 512 threads per SM,
  * each owning every 148th tile (its q in shared memory: up to 12 FP64 / 25
  * FP32 tiles per block) (each falls back to the two-kernel loop when it
@@ -640,10 +642,11 @@ int32_t xcal_case_solve_report(const xcal_case* cs, int32_t* iters7, int32_t* st
 int32_t xcal_case_set_inner_cg(xcal_case* cs, int32_t mode);
 /* launch-shape autotuner (runs on first use, or now): out6 = for U then p,
  * (SpMV rows per thread [0 = canonical tile kernel], SpMV block size, DILU
- * form [0 one launch per level, 1 one-block sweeps, 2 one cooperative launch
- * over every level]).  The choices never change a result. */
+ * form [0 one launch per level, 1 one-block sweeps, 2 one cooperative launch:
+ * rows that wait for the values they read, or every level with a barrier]).  The choices never change a result. */
 int32_t xcal_case_tuning(xcal_case* cs, int32_t* out6);
-/* DILU execution: 0 = autotuned (default), 1 = one-block sweeps,
+/* DILU execution: 0 = chosen by size and timing (default; rows that wait for
+ * the values they read, or one of the forms below), 1 = one-block sweeps,
  * 2 = one launch per level over level-ordered triangles, 3 = every level of
  * an application in one cooperative launch (a grid barrier between levels).
  * Same results, bit for bit. */

@@ -890,7 +890,8 @@ class Case:
         """Launch shapes chosen by the autotuner (tuning runs now if it has
         not yet): per equation the BiCGSTAB SpMV rows per thread (0 = tile
         kernel) and block size, and the DILU form (one-block sweeps, or one
-        cooperative launch over every level)."""
+        cooperative launch: rows that wait for the values they read, or
+        every level with a barrier)."""
         a = np.zeros(6, dtype=np.int32)
         self._chk(lib().xcal_case_tuning(self.h, _abi.ptr(a, C.c_int32)))
         return {eq: {"spmv_rows_per_thread": int(a[3 * k]), "spmv_block": int(a[3 * k + 1]),
@@ -898,7 +899,7 @@ class Case:
                 for k, eq in enumerate(("U", "p"))}
 
     def set_dilu_mode(self, mode: int):
-        """0 = autotuned, 1 = one-block sweeps, 2 = per-level kernels,
+        """0 = chosen by size and timing, 1 = one-block sweeps, 2 = per-level kernels,
         3 = every level in one cooperative launch (same results)."""
         self._chk(lib().xcal_case_set_dilu_mode(self.h, int(mode)))
 

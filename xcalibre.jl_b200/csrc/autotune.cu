@@ -6,7 +6,9 @@
 //    in blocks of 128/256/512 threads;
 //  * how a DILU application of a system of more than 524,288 rows runs: rows
 //    waiting for the values they read (dataflow), one launch per level, or
-//    every level in one cooperative launch with a grid barrier between levels.
+//    every level in one cooperative launch with a grid barrier between levels
+//    (the fused BiCGSTAB, which shares the waits among components, is always
+//    a dataflow).
 // Each candidate is timed with CUDA events on the case's own matrix at first
 // use; choices are cached per size class (value size, log2 rows, entries per
 // row), so later cases of the same class reuse them without timing.

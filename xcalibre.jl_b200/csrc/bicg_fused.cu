@@ -722,42 +722,56 @@ bool Case::components_apart() {
 
 // work vectors of components 1 and 2, and the three diagonals, allocated at the
 // first fused momentum solve (a case in a batch has none), never under capture;
-// where they would take more than a quarter of the free memory the components
-// are solved in turn
+// where they (above 64 MB) would take more than a quarter of the free memory the
+// components are solved in turn
 void Case::reserve_fused() {
     if (bf.ready || bf.refused || capturing || !use_fused(U, cfg.U_solver) || !components_apart()) return;
+    const bool mixed = cfg.precision == XCAL_PREC_MIXED;
     const size_t n = U.n, T = (n + RED_TILE - 1) / RED_TILE;
-    const size_t need = n * (cfg.precision == XCAL_PREC_MIXED ? 124 : 168);
-    size_t free_b = 0, total_b = 0, held = 0;
-    XCAL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if (need > free_b / 4) {
-        bf.refused = true;
-        return;
+    // one allocation: seven cost a new case's first step 0.1-0.2 ms (1,073 and
+    // 27,025 cells: 0.66 -> 0.57 and 2.04 -> 1.90 ms)
+    size_t need = 0;
+    auto take = [&](size_t b) {
+        const size_t at = need;
+        need += (b + 255) & ~size_t(255);
+        return at;
+    };
+    const size_t o_diag = take(3 * n * sizeof(double)), o_dx = take(2 * n * sizeof(double));
+    const size_t o_part0 = take(3 * T * sizeof(double)), o_part1 = take(3 * T * sizeof(double));
+    const size_t o_res = take(3 * sizeof(double)), o_S = take(3 * sizeof(KScalars));
+    const size_t o_vec = take(mixed ? 2 * 9 * n * sizeof(float) : 2 * 8 * n * sizeof(double));
+    const size_t o_diag32 = take(mixed ? 3 * n * sizeof(float) : 0);
+    size_t held = 0;
+    if (need > (size_t)64 << 20) {
+        size_t free_b = 0, total_b = 0;
+        XCAL_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        if (need > free_b / 4) {
+            bf.refused = true;
+            return;
+        }
     }
     try {
         AllocScope acc(&held);
-        bf.diag.alloc(3 * n);
-        bf.dx.alloc(2 * n);
-        if (cfg.precision == XCAL_PREC_MIXED) {
-            bf.diag32.alloc(3 * n);
-            bf.vec32.alloc(2 * 9 * n);
-        } else {
-            bf.vec.alloc(2 * 8 * n);
-        }
-        bf.part0.alloc(3 * T);
-        bf.part1.alloc(3 * T);
-        bf.S.alloc(3);
-        bf.S.zero(stream);
-        bf.res.alloc(3);
+        bf.mem.alloc(need);
     } catch (const Error&) {
         cudaGetLastError();
-        for (DBuf<double>* b : {&bf.diag, &bf.dx, &bf.vec, &bf.part0, &bf.part1, &bf.res}) b->release();
-        bf.diag32.release();
-        bf.vec32.release();
-        bf.S.release();
         bf.refused = true;
         return;
     }
+    unsigned char* m = bf.mem.p;
+    bf.diag = reinterpret_cast<double*>(m + o_diag);
+    bf.dx = reinterpret_cast<double*>(m + o_dx);
+    bf.part0 = reinterpret_cast<double*>(m + o_part0);
+    bf.part1 = reinterpret_cast<double*>(m + o_part1);
+    bf.res = reinterpret_cast<double*>(m + o_res);
+    bf.S = reinterpret_cast<KScalars*>(m + o_S);
+    if (mixed) {
+        bf.vec32 = reinterpret_cast<float*>(m + o_vec);
+        bf.diag32 = reinterpret_cast<float*>(m + o_diag32);
+    } else {
+        bf.vec = reinterpret_cast<double*>(m + o_vec);
+    }
+    XCAL_CUDA(cudaMemsetAsync(bf.S, 0, 3 * sizeof(KScalars), stream));
     bytes += held;
     bf.ready = true;
 }
@@ -772,9 +786,9 @@ BfView<T, NC> Case::bf_view(Equation& E, const xcal_solver_setup& SS, const Solv
     V.bar = ws.bar.p;
     V.err = ws.err.p;
     V.active = (1 << NC) - 1;
-    V.S = NC == 1 ? ws.S.p + R[0].kslot : bf.S.p;
-    V.part0 = NC == 1 ? ws.part0.p : bf.part0.p;
-    V.part1 = NC == 1 ? ws.part1.p : bf.part1.p;
+    V.S = NC == 1 ? ws.S.p + R[0].kslot : bf.S;
+    V.part0 = NC == 1 ? ws.part0.p : bf.part0;
+    V.part1 = NC == 1 ? ws.part1.p : bf.part1;
     if (SS.precond == XCAL_PRECOND_DILU) {
         V.lo = level_view<T>(E, 0);
         V.up = level_view<T>(E, 1);
@@ -789,18 +803,18 @@ BfView<T, NC> Case::bf_view(Equation& E, const xcal_solver_setup& SS, const Solv
     for (int d = 0; d < NC; ++d) {
         V.b[d] = R[d].b;
         V.field[d] = R[d].field;
-        V.res[d] = capturing ? gres.p + R[d].slot : NC == 1 ? resbuf.p : bf.res.p + d;
-        V.dg64[d] = NC == 1 ? nullptr : bf.diag.p + d * n;
-        V.dx[d] = d == 0 ? ws.dx.p : bf.dx.p + (d - 1) * n;
+        V.res[d] = capturing ? gres.p + R[d].slot : NC == 1 ? resbuf.p : bf.res + d;
+        V.dg64[d] = NC == 1 ? nullptr : bf.diag + d * n;
+        V.dx[d] = d == 0 ? ws.dx.p : bf.dx + (d - 1) * n;
         T* w[9];
         if constexpr (F) {
             T* first[9] = {ws.fx.p, ws.fr.p, ws.fp.p, ws.fv.p, ws.fs.p, ws.ft.p, ws.fq.p, ws.fz.p, ws.fd.p};
-            for (int k = 0; k < 9; ++k) w[k] = d == 0 ? first[k] : bf.vec32.p + ((d - 1) * 9 + k) * n;
-            V.dg[d] = NC == 1 ? nullptr : bf.diag32.p + d * n;
+            for (int k = 0; k < 9; ++k) w[k] = d == 0 ? first[k] : bf.vec32 + ((d - 1) * 9 + k) * n;
+            V.dg[d] = NC == 1 ? nullptr : bf.diag32 + d * n;
             V.c[d] = w[8];
         } else {
             T* first[8] = {ws.x.p, ws.r.p, ws.p.p, ws.v.p, ws.s.p, ws.t.p, ws.q.p, ws.z.p};
-            for (int k = 0; k < 8; ++k) w[k] = d == 0 ? first[k] : bf.vec.p + ((d - 1) * 8 + k) * n;
+            for (int k = 0; k < 8; ++k) w[k] = d == 0 ? first[k] : bf.vec + ((d - 1) * 8 + k) * n;
             V.dg[d] = V.dg64[d];
             V.c[d] = R[d].b;
         }

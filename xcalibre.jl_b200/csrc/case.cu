@@ -2095,7 +2095,7 @@ void Case::solve_equation_U(double res[3]) {  // Solve_1_api.jl:233-266
     if (bf.ready && use_fused(U, cfg.U_solver) && components_apart()) {
         SolveRef R[3];
         for (int d = 0; d < 3; ++d) {
-            bc_relax_U(d, bf.diag.p + (size_t)d * U.n);
+            bc_relax_U(d, bf.diag + (size_t)d * U.n);
             if (d == 0) update_precond(XCAL_EQN_U);
             R[d] = solve_ref(XCAL_EQN_U, d);
         }

@@ -337,9 +337,11 @@ struct Case {
     struct Fused {
         bool ready = false;
         bool refused = false;  // no memory for it
-        DBuf<double> diag, dx, vec, part0, part1, res;  // diagonals of the components; vectors of components 1, 2
-        DBuf<float> diag32, vec32;
-        DBuf<KScalars> S;
+        DBuf<unsigned char> mem;  // holds all of:
+        double *diag = nullptr, *dx = nullptr, *vec = nullptr;  // diagonals of the components; vectors of components 1, 2
+        double *part0 = nullptr, *part1 = nullptr, *res = nullptr;
+        float *diag32 = nullptr, *vec32 = nullptr;
+        KScalars* S = nullptr;
     } bf;
     int apart = -1;  // components_apart(), once known
     bool use_fused(const Equation& E, const xcal_solver_setup& SS);

@@ -572,6 +572,13 @@ int32_t xcal_residual_noalloc(int32_t n, const int32_t* rowptr, const int32_t* c
  * kernel launched after it still ran (the context stayed usable). */
 int32_t xcal_check_bounded_wait(xcal_ctx* ctx, int64_t spin_limit, int32_t* gave_up, int32_t* flag_set,
                                 int32_t* ran_after);
+/* the same for the kernels whose rows or blocks wait for values of others:
+ * `which` runs on a small system one of whose values is never written, giving
+ * up after spin_limit polls (1 .. 2,097,152).  gave_up = 1 when the kernel
+ * ended without that value; flag_set and ran_after as above. */
+enum { XCAL_WAIT_DILU_FACTOR = 0 };
+int32_t xcal_check_wait(xcal_ctx* ctx, int32_t which, int64_t spin_limit, int32_t* gave_up, int32_t* flag_set,
+                        int32_t* ran_after);
 
 /* ---- timers --------------------------------------------------------------*/
 /* cumulative device time (ms) per phase since case creation:

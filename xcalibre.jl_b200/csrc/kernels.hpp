@@ -320,9 +320,10 @@ int flow_grid(const void* kernel);
 // marks values as not yet computed (all bits one)
 void kr_flow_unset(cudaStream_t s, void* p, size_t bytes);
 // the DILU factor in the same way (D is set to unset values first; ticket:
-// one word, zeroed here), an ordinary launch
+// one word, zeroed here), an ordinary launch; spin_limit: polls before a wait
+// gives up (0: the usual limit)
 void kr_dilu_D_flow(cudaStream_t s, int n, const LevelDView& L, const double* nz, double* D, unsigned int* ticket,
-                    int* err);
+                    int* err, int spin_limit = 0);
 void kr_residual(cudaStream_t s, const CSRView& A, const double* nz, const double* x, const double* b, KScalars* S,
                  double* part0, double* part1, double* out);
 // device-driven solve control of graph mode (conditional WHILE nodes)

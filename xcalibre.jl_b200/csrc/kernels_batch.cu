@@ -48,16 +48,15 @@ __global__ void __launch_bounds__(FLOW_THREADS) kbk_dilu_flow(const BSys<T>* __r
                                                               unsigned int* ticket, int* err, int in, int out,
                                                               int use_S) {
     __shared__ int sh_item;
-    for (;;) {
-        const int t = flow_ticket(ticket, &sh_item);
+    for (bool ok = true;;) {
+        const int t = flow_ticket(ticket, &sh_item, ok);
         if (t >= n_items) return;
         const int2 it = items[t];
         const BSys<T>& B = sys[it.x];
         if (use_S && B.S->done) continue;
         const int k0 = it.y * FLOW_THREADS + (threadIdx.x & ~31);
-        const bool ok = LOWER ? flow_lower_rows(B.n, B.lo, (const T*)B.vec[in], B.flow_y, B.vec[out], k0, err)
-                              : flow_upper_rows(B.n, B.up, B.P, B.flow_y, B.vec[out], k0, err);
-        if (__syncthreads_or(!ok)) return;
+        ok = LOWER ? flow_lower_rows(B.n, B.lo, (const T*)B.vec[in], B.flow_y, B.vec[out], k0, err)
+                   : flow_upper_rows(B.n, B.up, B.P, B.flow_y, B.vec[out], k0, err);
     }
 }
 

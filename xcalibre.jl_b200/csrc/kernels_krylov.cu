@@ -469,11 +469,12 @@ __global__ void __launch_bounds__(FLOW_THREADS) k_dilu_flow(int n, LevelView<T> 
 // belong to chunks already drawn by running blocks, and the kernel needs no
 // co-residency (it also runs inside a batch's per-case graphs).
 __global__ void __launch_bounds__(FLOW_THREADS) k_dilu_D_flow(int n, LevelDView L, const double* __restrict__ nz,
-                                                              double* D, unsigned int* ticket, int* err) {
+                                                              double* D, unsigned int* ticket, int* err,
+                                                              int spin_limit) {
     __shared__ int sh_chunk;
     const int chunks = (n + FLOW_THREADS - 1) / FLOW_THREADS;
-    for (;;) {
-        const int chunk = flow_ticket(ticket, &sh_chunk);
+    for (bool ok = true;;) {
+        const int chunk = flow_ticket(ticket, &sh_chunk, ok);
         if (chunk >= chunks) return;
         const int k = chunk * FLOW_THREADS + threadIdx.x;
         int i = 0, c = -1, base = 0;
@@ -498,17 +499,16 @@ __global__ void __launch_bounds__(FLOW_THREADS) k_dilu_D_flow(int n, LevelDView 
             for (int j = 0; j < FLOW_U; ++j)
                 if (j < c) pj[j] = nz[tj[j]] * nz[sj[j]];
         }
-        if (!flow_wait((const double*)D, L.col, base, c, cj, yv, err, [&] {
+        ok = flow_wait((const double*)D, L.col, base, c, cj, yv, err, [&] {
 #pragma unroll
-                for (int j = 0; j < FLOW_U; ++j)
-                    if (j < c) d = d - pj[j] / yv[j];
-                for (int j = FLOW_U; j < c; ++j) {
-                    const int e = base + SELL_C * j;
-                    d = d - (nz[ld_stream(L.tsrc + e)] * nz[ld_stream(L.src + e)]) / ld_flow(D + ld_stream(L.col + e));
-                }
-                st_flow(D + i, d);
-            }))
-            return;
+            for (int j = 0; j < FLOW_U; ++j)
+                if (j < c) d = d - pj[j] / yv[j];
+            for (int j = FLOW_U; j < c; ++j) {
+                const int e = base + SELL_C * j;
+                d = d - (nz[ld_stream(L.tsrc + e)] * nz[ld_stream(L.src + e)]) / ld_flow(D + ld_stream(L.col + e));
+            }
+            st_flow(D + i, d);
+        }, spin_limit);
     }
 }
 
@@ -1315,12 +1315,13 @@ template bool kr_dilu_flow<float>(cudaStream_t, int, const LevelView<float>&, co
                                   const float*, float*, float*, unsigned int*, int*, const KScalars*);
 void kr_flow_unset(cudaStream_t s, void* p, size_t bytes) { XCAL_CUDA(cudaMemsetAsync(p, 0xff, bytes, s)); }
 void kr_dilu_D_flow(cudaStream_t s, int n, const LevelDView& L, const double* nz, double* D, unsigned int* ticket,
-                    int* err) {
+                    int* err, int spin_limit) {
     if (n <= 0) return;
     kr_flow_unset(s, D, (size_t)n * sizeof(double));
     XCAL_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s));
     const int blocks = std::min(flow_grid((const void*)k_dilu_D_flow), (n + FLOW_THREADS - 1) / FLOW_THREADS);
-    k_dilu_D_flow<<<std::max(blocks, 1), FLOW_THREADS, 0, s>>>(n, L, nz, D, ticket, err);
+    k_dilu_D_flow<<<std::max(blocks, 1), FLOW_THREADS, 0, s>>>(n, L, nz, D, ticket, err,
+                                                              spin_limit > 0 ? spin_limit : FLOW_SPIN_LIMIT);
     XCAL_CHECK_LAUNCH();
 }
 template bool kr_dilu_grid<double>(cudaStream_t, const LevelView<double>&, const LevelView<double>&, const double*,

@@ -751,6 +751,15 @@ __device__ __forceinline__ double flow_unset_value<double>() { return __longlong
 template <>
 __device__ __forceinline__ float flow_unset_value<float>() { return __int_as_float(-1); }
 
+// whether a warp that has polled `spins` times stops waiting (the same answer
+// in every lane): past the limit, or as another warp gave up
+__device__ __forceinline__ bool flow_give_up(int spins, int spin_limit, int* err) {
+    if (spins < spin_limit && (spins & 1023) != 1023) return false;
+    if (!__any_sync(0xffffffffu, spins >= spin_limit || *(volatile int*)err)) return false;
+    *(volatile int*)err = 1;
+    return true;
+}
+
 // Polls the values ys[col] of one row's c slots (the first FLOW_U's columns
 // in cj, values landing in yv) until all are set, then runs `finish` --
 // inside the loop, so that a row another lane of the warp waits for is
@@ -758,7 +767,8 @@ __device__ __forceinline__ float flow_unset_value<float>() { return __int_as_flo
 // the warp calls it (c < 0: no row).  false: gave up.
 template <class T, class F>
 __device__ __forceinline__ bool flow_wait(const T* ys, const int* __restrict__ col, int base, int c,
-                                          const int (&cj)[FLOW_U], T (&yv)[FLOW_U], int* err, F&& finish) {
+                                          const int (&cj)[FLOW_U], T (&yv)[FLOW_U], int* err, F&& finish,
+                                          int spin_limit = FLOW_SPIN_LIMIT) {
     bool fin = c < 0;
 #pragma unroll
     for (int j = 0; j < FLOW_U; ++j)
@@ -777,10 +787,7 @@ __device__ __forceinline__ bool flow_wait(const T* ys, const int* __restrict__ c
             }
         }
         if (__all_sync(0xffffffffu, fin)) return true;
-        if (spins > FLOW_SPIN_LIMIT || ((spins & 1023) == 1023 && *(volatile int*)err)) {
-            *(volatile int*)err = 1;
-            return false;
-        }
+        if (flow_give_up(spins, spin_limit, err)) return false;
         if (!fin) {
 #pragma unroll
             for (int j = 0; j < FLOW_U; ++j)
@@ -791,9 +798,13 @@ __device__ __forceinline__ bool flow_wait(const T* ys, const int* __restrict__ c
 
 // a block's next chunk of work, drawn from a counter that only grows: chunks
 // are handed out in order to blocks that run, so waiting on an earlier chunk
-// always ends
-__device__ __forceinline__ int flow_ticket(unsigned int* ticket, int* sh) {
-    __syncthreads();
+// always ends.  Called by every thread of the block; ok: whether the thread's
+// last chunk went well.  Where one warp gave up the whole block gets no more
+// work: a warp that left alone could be the one that draws, and the others
+// would go on with its last ticket for good
+constexpr int FLOW_NO_CHUNK = 0x7fffffff;
+__device__ __forceinline__ int flow_ticket(unsigned int* ticket, int* sh, bool ok) {
+    if (__syncthreads_or(!ok)) return FLOW_NO_CHUNK;
     if (threadIdx.x == 0) *sh = (int)atomicAdd(ticket, 1u);
     __syncthreads();
     return *sh;

@@ -154,3 +154,39 @@ def test_serving_same_alone_and_in_mix(x, ctx):
         assert np.array_equal(m.U, solo.U) and np.array_equal(m.p, solo.p)
     s = serve.summarize(mix, server.wall)
     assert s["cases"] == 5 and s["p99_ms"] >= s["p50_ms"] > 0
+
+
+def test_case_carries_on_after_its_batch(x, ctx):
+    """A case whose k and omega solves captured their chunks inside a batch
+    goes on alone once the batch is gone, equal to a case never in one.
+    (Profiling keeps those solves on the chunked loop.)"""
+    from test_gpu_komega import komega_channel_case
+    from test_komega import set_komega_fields
+    mesh = x.build_mesh3(x.channel_polymesh(40, 16, 15, seed=4))
+    out = []
+    for batched in (False, True):
+        model, config = komega_channel_case(x, mesh, 6, "DILU")
+        for name in ("k", "omega"):
+            config.solvers[name].rtol = 1e-13
+            config.solvers[name].relax = 1.0
+        cfg, keep = x.build_config(model, config)
+        dm = x.DeviceMesh(ctx, mesh)
+        c = x.Case(dm, cfg)
+        set_komega_fields(x, c, model)
+        c.set_profiling(True)
+        if batched:
+            batch = x.api.Batch(ctx, 2, 1 << 32)
+            assert batch.add(c)
+            for _ in range(2):
+                batch.simple_iterate()
+            batch.remove(c)
+            batch.close()
+        else:
+            c.simple_iterate(2)
+        assert c.solve_report()["iterations"][4] > 7  # a chunk of 8 iterations was captured
+        c.simple_iterate(2)
+        out.append([c.get_field(getattr(x._abi, f)) for f in ("FIELD_U", "FIELD_P", "FIELD_K", "FIELD_OMEGA")])
+        c.close()
+        dm.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

@@ -1438,7 +1438,7 @@ void Case::update_precond_E(Equation& E, int pt) {
         kr_jacobi_update(stream, E.view(), E.nz.p, E.P.p);
     } else if (pt == XCAL_PRECOND_DILU) {
         if (E.flow_D) {
-            kr_dilu_D_flow(stream, E.n, level_d_view(E), E.nz.p, E.P.p, ws.bar.p, flow_err());
+            kr_dilu_D_flow(stream, E.n, level_d_view(E), E.nz.p, E.P.p, ws.bar.p, factor_err());
             return;
         }
         if (E.dilu_block()) {
@@ -1473,7 +1473,7 @@ void Case::dilu_ldiv(Equation& E, const T* nz, const T* D, const T* b, T* out, c
     (void)nz;
     if (E.use_flow && coop_ok_here() &&
         kr_dilu_flow(stream, E.n, level_view<T>(E, 0), level_view<T>(E, 1), D, b, flow_scratch<T>(out), out,
-                     ws.bar.p, flow_err(), S))
+                     ws.bar.p, ws.err.p, S))
         return;
     if (E.dilu_block()) {
         kr_dilu_block(stream, E.n, level_view<T>(E, 0), level_view<T>(E, 1), D, b, out, S);

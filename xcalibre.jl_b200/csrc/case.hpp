@@ -351,10 +351,12 @@ struct Case {
     BfView<T, NC> bf_view(Equation& E, const xcal_solver_setup& SS, const SolveRef* R);
     template <class T, int NC>
     void fused_solve(Equation& E, const xcal_solver_setup& SS, const SolveRef* R, double* res);
-    // where the dataflow kernels report a wait that gave up: the case's own
-    // flag, or the batch's while the case is resident in one
+    // where the DILU factor reports a wait that gave up: the case's own flag,
+    // or the batch's while the case is resident in one (whose graphs of the
+    // factor go when the case leaves).  Applications report to the case's own:
+    // its solves read that, and the graphs of their chunks outlive a batch
     int* batch_err = nullptr;
-    int* flow_err() { return batch_err ? batch_err : ws.err.p; }
+    int* factor_err() { return batch_err ? batch_err : ws.err.p; }
     template <class T>
     void krylov_iterate(Equation& E, const xcal_solver_setup& SS, const T* nz, const T* P, const T* c, const T* r0,
                         const KrylovVecs<T>& V, KScalars* S, KScalars* hS, int gk);

@@ -579,6 +579,10 @@ int32_t xcal_check_bounded_wait(xcal_ctx* ctx, int64_t spin_limit, int32_t* gave
 enum { XCAL_WAIT_DILU_FACTOR = 0 };
 int32_t xcal_check_wait(xcal_ctx* ctx, int32_t which, int64_t spin_limit, int32_t* gave_up, int32_t* flag_set,
                         int32_t* ran_after);
+/* that barrier on a case's stream, with the error flag of its DILU solves: the
+ * case's next DILU-preconditioned solve returns XCAL_ERR_TIMEOUT, what runs
+ * after it is as usual. */
+int32_t xcal_case_check_wait(xcal_case* cs, int64_t spin_limit);
 
 /* ---- timers --------------------------------------------------------------*/
 /* cumulative device time (ms) per phase since case creation:

@@ -70,6 +70,7 @@ SIGNATURES = {
     "xcal_case_solve_report": (_i32, [_vp, _pi, _pi, _pi64]),
     "xcal_check_bounded_wait": (_i32, [_vp, _i64, _pi, _pi, _pi]),
     "xcal_check_wait": (_i32, [_vp, _i32, _i64, _pi, _pi, _pi]),
+    "xcal_case_check_wait": (_i32, [_vp, _i64]),
     "xcal_det_math": (_i32, [_i32, _pd, _pd, _i64]),
     "xcal_equation_create": (_i32, [_vp, _i32, C.POINTER(_abi.TermDesc), _i32, C.POINTER(_abi.SourceDesc), _i32,
                                     C.POINTER(_abi.BCDesc), C.POINTER(_vp)]),

@@ -942,7 +942,7 @@ void Case::fused_solve(Equation& E, const xcal_solver_setup& SS, const SolveRef*
             if (pre == XCAL_PRECOND_DILU)
                 XCAL_CUDA(cudaMemcpyAsync(h_perr, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
             sync();
-            if (pre == XCAL_PRECOND_DILU && *h_perr) fail(XCAL_ERR_TIMEOUT, "DILU sweep: a wait gave up");
+            if (pre == XCAL_PRECOND_DILU) report_wait(*h_perr, "DILU sweep: a wait gave up");
             bool all = true;
             for (int d = 0; d < NC; ++d) all = all && (!(V.active >> d & 1) || hS[d].done);
             if (all) break;

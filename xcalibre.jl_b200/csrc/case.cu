@@ -1016,6 +1016,14 @@ Case::~Case() {
 
 void Case::sync() { XCAL_CUDA(cudaStreamSynchronize(stream)); }
 
+// a wait that gave up is reported once: the flag is clear again for what runs
+// after it
+void Case::report_wait(int flag, const char* what) {
+    if (!flag) return;
+    XCAL_CUDA(cudaMemsetAsync(ws.err.p, 0, sizeof(int), stream));
+    fail(XCAL_ERR_TIMEOUT, what);
+}
+
 // Capture `body` (a fixed sequence of launches on the case stream) once,
 // then replay it.  Launch counts follow the replays, not the capture.
 template <class F>
@@ -1648,7 +1656,7 @@ void Case::krylov_iterate(Equation& E, const xcal_solver_setup& SS, const T* nz,
             XCAL_CUDA(cudaMemcpyAsync(hS, S, sizeof(KScalars), cudaMemcpyDeviceToHost, stream));
             XCAL_CUDA(cudaMemcpyAsync(&errflag, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
             sync();
-            if (errflag) fail(XCAL_ERR_TIMEOUT, "persistent CG: a grid barrier wait gave up");
+            report_wait(errflag, "persistent CG: a grid barrier wait gave up");
             if (!hS->done) fail(XCAL_ERR_TIMEOUT, "persistent CG did not report completion");
             if (profiling) {
                 float t = 0;
@@ -1992,7 +2000,7 @@ double Case::solve_system_ref(const SolveRef& R, int* iters, bool fp64) {
     XCAL_CUDA(cudaMemcpyAsync(h_res, resbuf.p, sizeof(double), cudaMemcpyDeviceToHost, stream));
     if (grid_dilu) XCAL_CUDA(cudaMemcpyAsync(h_perr, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
     sync();
-    if (grid_dilu && *h_perr) fail(XCAL_ERR_TIMEOUT, "DILU sweep: a grid barrier wait gave up");
+    if (grid_dilu) report_wait(*h_perr, "DILU sweep: a wait gave up");
     return h_res[0];
 }
 
@@ -2016,7 +2024,7 @@ void Case::fold_iterate(Equation& E, double* field, const KrylovVecs<float>& V, 
     XCAL_CUDA(cudaMemcpyAsync(hS, S, sizeof(KScalars), cudaMemcpyDeviceToHost, stream));
     XCAL_CUDA(cudaMemcpyAsync(&errflag, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
     sync();
-    if (errflag) fail(XCAL_ERR_TIMEOUT, "folded CG: a grid barrier wait gave up");
+    report_wait(errflag, "folded CG: a grid barrier wait gave up");
     if (!hS->done) fail(XCAL_ERR_TIMEOUT, "folded CG did not report completion");
     if (profiling) {
         float t = 0;
@@ -2454,7 +2462,7 @@ void Case::run_step_graph(double res[4], double* courant) {
     XCAL_CUDA(cudaMemsetAsync(dlaunch.p, 0, sizeof(unsigned long long), stream));
     XCAL_CUDA(cudaMemcpyAsync(h_perr, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
     sync();
-    if (*h_perr) fail(XCAL_ERR_TIMEOUT, "persistent CG: a grid barrier wait gave up (graph mode)");
+    report_wait(*h_perr, "a kernel's bounded wait gave up (graph mode)");
     long long nk = step_top_kernels + (long long)h_launch[0];
     g_launch_count.fetch_add(nk, std::memory_order_relaxed);
     t_launch_count += nk;

@@ -324,6 +324,7 @@ struct Case {
     MeshView mv() const { return mesh->view(); }
     double* field_comp(int field, int comp, long& count);
     void sync();
+    void report_wait(int flag, const char* what);
     template <class T>
     void dilu_ldiv(Equation& E, const T* nz, const T* D, const T* b, T* out, const KScalars* S);
     template <class T>

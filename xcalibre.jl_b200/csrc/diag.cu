@@ -8,7 +8,9 @@
 //   xcal_check_bounded_wait  the grid barrier: one block waits for a second
 //                            that is never launched;
 //   xcal_check_wait          the kernel named by `which`, on a system one of
-//                            whose rows waits for a value nothing writes.
+//                            whose rows waits for a value nothing writes;
+//   xcal_case_check_wait     that barrier with a case's own flag, which the
+//                            case's next solve reports.
 #include <cmath>
 #include <vector>
 
@@ -124,6 +126,26 @@ extern "C" int32_t xcal_check_wait(xcal_ctx* ctx, int32_t which, int64_t spin_li
         return XCAL_OK;
     } catch (const Error& e) {
         ctx->set_error(e.msg);
+        return e.code;
+    }
+}
+
+extern "C" int32_t xcal_case_check_wait(xcal_case* cs, int64_t spin_limit) {
+    if (!cs || spin_limit < 1 || spin_limit > BAR_SPIN_LIMIT) return XCAL_ERR_INVALID;
+    Case* c = cs->c.get();
+    try {
+        XCAL_CUDA(cudaSetDevice(c->ctx->device));
+        DBuf<unsigned int> count;
+        DBuf<int> out;
+        count.alloc(2);
+        count.zero(c->stream);
+        out.alloc(4);
+        k_wait_check<<<1, 32, 0, c->stream>>>(count.p, c->ws.err.p, (long)spin_limit, out.p);
+        XCAL_CHECK_LAUNCH();
+        c->sync();
+        return XCAL_OK;
+    } catch (const Error& e) {
+        c->ctx->set_error(e.msg);
         return e.code;
     }
 }

@@ -133,3 +133,33 @@ def test_dilu_flow_mixed_and_batch(x, ctx, name):
     for c, dm, _ in members:
         c.close()
         dm.close()
+
+
+@pytest.mark.parametrize("modes", [(0, 2), (0, 1), (3, 1), (0, 3, 2)])
+def test_dilu_form_changed_between_steps(x, ctx, modes):
+    """A DILU-CG whose solves run captured chunks of iterations takes another
+    form between host-driven steps: the same results as without the change."""
+    mesh = x.build_mesh3(MESHES["4620"](x))
+    out = []
+    for ms in ((0,) * len(modes), modes):
+        cfg, keep = _config(x, mesh)
+        cfg.p_solver.rtol = 1e-12
+        dm = x.DeviceMesh(ctx, mesh)
+        c = x.Case(dm, cfg)
+        _start(x, c, mesh)
+        its = []
+        for m in ms:
+            c.set_dilu_mode(m)
+            # U, then p: the step calls are host-driven whatever the iteration
+            c.initial_calculations()
+            c.solve_equation(x._abi.EQN_U)
+            c.pressure_predictor()
+            c.flux_divergence()
+            c.solve_equation(x._abi.EQN_P)
+            its.append(int(c.solve_report()["iterations"][3]))
+        assert min(its) > 60, its  # chunks of 4, 8, 16 and captured ones of 32
+        out.append((its, c.get_field(x._abi.FIELD_U), c.get_field(x._abi.FIELD_P)))
+        c.close()
+        dm.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

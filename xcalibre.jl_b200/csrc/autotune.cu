@@ -144,6 +144,7 @@ void Case::autotune() {
                 lk.lock();
                 g_dilu_choice[k] = form;
             }
+            if (E.use_flow != (form == 4)) drop_graphs();  // chunks of earlier solves hold the other form
             E.use_block = form == 1;
             E.use_grid = form == 3;
             E.use_flow = form == 4;

@@ -993,11 +993,23 @@ Case::Case(xcal_ctx* c, const DevMesh* m, const xcal_config* cf) : ctx(c), mesh(
     if (has_y()) wall_distance();
 }
 
-Case::~Case() {
+// The captured step and the captured chunks of iterations.  Both hold the DILU
+// form they were captured with, and the dataflow form relies on scratch that
+// only its own refresh resets: a form may change only with the graphs gone.
+void Case::drop_graphs() {
     if (stream) cudaStreamSynchronize(stream);
     for (auto& row : chunk_graph)
         for (auto& g : row)
-            if (g.exec) cudaGraphExecDestroy(g.exec);
+            if (g.exec) {
+                cudaGraphExecDestroy(g.exec);
+                g.exec = nullptr;
+            }
+    if (step_graph) cudaGraphExecDestroy(step_graph);
+    step_graph = nullptr;
+}
+
+Case::~Case() {
+    drop_graphs();
     for (auto& row : gev)
         for (auto& e : row)
             if (e) cudaEventDestroy(e);
@@ -1008,7 +1020,6 @@ Case::~Case() {
     if (h_iters) cudaFreeHost(h_iters);
     if (h_perr) cudaFreeHost(h_perr);
     if (h_launch) cudaFreeHost(h_launch);
-    if (step_graph) cudaGraphExecDestroy(step_graph);
     for (cudaStream_t& sd : side)
         if (sd) cudaStreamDestroy(sd);
     if (stream && own_stream) cudaStreamDestroy(stream);

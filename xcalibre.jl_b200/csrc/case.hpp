@@ -325,6 +325,7 @@ struct Case {
     double* field_comp(int field, int comp, long& count);
     void sync();
     void report_wait(int flag, const char* what);
+    void drop_graphs();
     template <class T>
     void dilu_ldiv(Equation& E, const T* nz, const T* D, const T* b, T* out, const KScalars* S);
     template <class T>

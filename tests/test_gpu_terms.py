@@ -282,3 +282,19 @@ def test_poisson_solve_from_terms(x, ctx, solver, pre):
     assert its > 0 and res < 1e-10, (res, its)
     assert np.linalg.norm(sol - exact) / np.linalg.norm(exact) < 1e-8
     E.close()
+
+
+@pytest.mark.parametrize("name", ["test_poisson_solve_from_terms", "test_dilu_form_changed_between_steps"])
+def test_first_dilu_solve_of_a_process(name):
+    """A process whose first work is a DILU solve long enough for captured
+    chunks, with no step driven before it."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    arg = {"test_poisson_solve_from_terms": "test_gpu_terms.py::test_poisson_solve_from_terms[bicgstab-dilu]",
+           "test_dilu_form_changed_between_steps":
+               "test_gpu_dilu_flow.py::test_dilu_form_changed_between_steps[modes0]"}[name]
+    r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-m", "gpu", os.path.join(here, arg)],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:]

@@ -102,10 +102,6 @@ static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, 
 void Case::autotune() {
     if (tuned || capturing) return;
     tuned = true;
-    // whether cooperative kernels run inside captured graphs: found here,
-    // before any capture (the checks run graphs of their own)
-    kr_coop_capture_ok(false);
-    kr_coop_capture_ok(true);
     const bool mixed = cfg.precision == XCAL_PREC_MIXED;
     const int tsz = mixed ? 4 : 8;
     for (int e = 0; e < 2; ++e) {

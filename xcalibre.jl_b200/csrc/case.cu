@@ -789,6 +789,9 @@ Case::Case(xcal_ctx* c, const DevMesh* m, const xcal_config* cf) : ctx(c), mesh(
         if (ss->precond < XCAL_PRECOND_NONE || ss->precond > XCAL_PRECOND_DILU)
             fail(XCAL_ERR_UNSUPPORTED, "unknown preconditioner");
     }
+    // which launch forms run inside captured graphs: the check runs graphs of
+    // its own, which no capture may be open for
+    kr_probe_capture();
     XCAL_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     for (auto& e : ev) XCAL_CUDA(cudaEventCreate(&e));
     XCAL_CUDA(cudaMallocHost(&h_S, 5 * sizeof(KScalars)));
@@ -2424,15 +2427,8 @@ void Case::capture_step() {
     body_kernels_captured = 0;
     capturing = true;
     cudaGraph_t g = nullptr;
-    // decided before the capture (the check runs graphs of its own)
-    kr_coop_capture_ok(false);
-    kr_cluster_capture_ok(false);
-    if (cfg.precision == XCAL_PREC_MIXED) {
-        kr_coop_capture_ok(true);
-        kr_cluster_capture_ok(true);
-        // the folded inner CG's storage (uploads) cannot be made under capture
-        if (use_fold(P, cfg.p_solver, true)) build_fold(P, stream, fold_uniform_ok());
-    }
+    // the folded inner CG's storage (uploads) cannot be made under capture
+    if (use_fold(P, cfg.p_solver, true)) build_fold(P, stream, fold_uniform_ok());
     XCAL_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     try {
         XCAL_CUDA(cudaMemsetAsync(ws.err.p, 0, sizeof(int), stream));

@@ -192,7 +192,9 @@ constexpr int PERSIST_MT512 = 5;
 constexpr int PERSIST_MT_SMEM = 200 * 1024;
 // whether this device and driver run a cooperative kernel captured into a
 // CUDA graph (in_while: inside the body of a conditional WHILE node); found
-// out once per process by capturing and running a one-block no-op that way
+// out once per process by capturing and running a one-block no-op that way --
+// by kr_probe_capture, before the first capture: a probe during one breaks it
+void kr_probe_capture();
 bool kr_coop_capture_ok(bool in_while);
 // the same for a kernel launched as thread-block clusters
 bool kr_cluster_capture_ok(bool in_while);

@@ -14,6 +14,7 @@
 // products accumulated in FP64 and the step scalars kept in FP64 on the
 // device and rounded to FP32 where they scale a vector.
 #include <algorithm>
+#include <array>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -732,19 +733,16 @@ static bool capture_probe(bool in_while, bool cluster) {
     return ok;
 }
 
-bool kr_coop_capture_ok(bool in_while) {
-    static int state[2] = {-1, -1};
-    int& st = state[in_while ? 1 : 0];
-    if (st < 0) st = capture_probe(in_while, false) ? 1 : 0;
-    return st == 1;
+// [cluster][in a WHILE body], probed once per process
+static const std::array<std::array<bool, 2>, 2>& capture_probes() {
+    static const std::array<std::array<bool, 2>, 2> ok = {
+        {{capture_probe(false, false), capture_probe(true, false)},
+         {capture_probe(false, true), capture_probe(true, true)}}};
+    return ok;
 }
-
-bool kr_cluster_capture_ok(bool in_while) {
-    static int state[2] = {-1, -1};
-    int& st = state[in_while ? 1 : 0];
-    if (st < 0) st = capture_probe(in_while, true) ? 1 : 0;
-    return st == 1;
-}
+void kr_probe_capture() { (void)capture_probes(); }
+bool kr_coop_capture_ok(bool in_while) { return capture_probes()[0][in_while ? 1 : 0]; }
+bool kr_cluster_capture_ok(bool in_while) { return capture_probes()[1][in_while ? 1 : 0]; }
 
 static inline int tiles(int n) { return n <= 0 ? 1 : (n + RED_TILE - 1) / RED_TILE; }
 #define TILE_LAUNCH(n) tiles(n), RED_THREADS, 0

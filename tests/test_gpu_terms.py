@@ -298,3 +298,44 @@ def test_first_dilu_solve_of_a_process(name):
     r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-m", "gpu", os.path.join(here, arg)],
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout[-2000:]
+
+
+def test_equations_solved_in_turn_on_one_case(x, ctx):
+    """Two equations of one case, each solved with every solver in turn (long
+    enough for captured chunks of iterations), then a third in the place of
+    the closed first: every solution is its own system's."""
+    import scipy.sparse as sp
+    import scipy.sparse.linalg as spl
+    D = _dsl(x)
+    mesh = x.build_mesh3(x.box_polymesh(20, 16, 14, seed=4))
+    case, keep = _laplace_case_generic(x, ctx, mesh)
+    rng = np.random.default_rng(3)
+    T = np.zeros(mesh.n_cells)
+    bcs = [x.Dirichlet("xmin", 1.0), x.Dirichlet("xmax", 0.0), x.Zerogradient("ymin"), x.Zerogradient("ymax"),
+           x.Zerogradient("zmin"), x.Zerogradient("zmax")]
+
+    def equation(k):
+        src = rng.uniform(0.0, 1.0, mesh.n_cells)
+        E = D.Equation(case, (-D.Laplacian[x.Linear](k, T) == D.Source(src)) >> D.ScalarEquation(T, bcs))
+        E.discretise()
+        E.apply_boundary_conditions(T)
+        rp, cv, nz, b = E.system()
+        return E, spl.spsolve(sp.csr_matrix((nz, cv, rp), shape=(mesh.n_cells, mesh.n_cells)).tocsc(), b)
+
+    def check(E, exact, solver, pre):
+        setup = x.SolverSetup(solver=solver(), preconditioner=pre(), convergence=1e-10, relax=1.0, rtol=1e-12,
+                              atol=1e-14, itmax=5000)
+        sol, res, its = E.solve(setup, T)
+        assert its > (28 if solver is x.Cg else 7) and res < 1e-10, (res, its)
+        assert np.linalg.norm(sol - exact) / np.linalg.norm(exact) < 1e-8
+
+    eqns = [equation(1.0), equation(7.0)]
+    for solver, pre in ((x.Bicgstab, x.DILU), (x.Bicgstab, x.Jacobi), (x.Cg, x.DILU), (x.Bicgstab, x.DILU)):
+        for E, exact in eqns:
+            check(E, exact, solver, pre)
+    eqns[0][0].close()
+    E, exact = equation(3.0)
+    check(E, exact, x.Bicgstab, x.DILU)
+    check(*eqns[1], x.Bicgstab, x.DILU)
+    E.close()
+    eqns[1][0].close()

@@ -1642,11 +1642,12 @@ void Case::krylov_step(Equation& E, const xcal_solver_setup& SS, const T* nz, co
 
 // Host-polled Krylov loop: chunks of iterations (4 -> 32 CG, 1 -> 8
 // BiCGSTAB), the steady-state chunk replayed as a cached CUDA graph, the
-// host reading the device's `done` flag after each chunk.  gk selects the
-// cached chunk graphs.
+// host reading the device's `done` flag after each chunk.  chunks: the cached
+// graphs [plain, profiled] of this system and solver.
 template <class T>
 void Case::krylov_iterate(Equation& E, const xcal_solver_setup& SS, const T* nz, const T* P, const T* c,
-                          const T* r0, const KrylovVecs<T>& V, KScalars* S, KScalars* hS, int gk) {
+                          const T* r0, const KrylovVecs<T>& V, KScalars* S, KScalars* hS, int gk,
+                          ChunkGraph* chunks) {
     const bool cg = SS.solver == XCAL_SOLVER_CG;
     const int pt = SS.precond;
     if (profiling)
@@ -1699,7 +1700,7 @@ void Case::krylov_iterate(Equation& E, const xcal_solver_setup& SS, const T* nz,
         if (graphed) {
             if (profiling)
                 for (int c8 = 4; c8 < CHUNK; c8 += 8) samples.push_back({c8, &gev[gk][nev * (c8 / 8)]});
-            replay_chunk(chunk_graph[gk][profiling ? 1 : 0], [&] {
+            replay_chunk(chunks[profiling ? 1 : 0], [&] {
                 for (int ci = 0; ci < CHUNK; ++ci)
                     krylov_step(E, SS, nz, P, c, V, S, profiling && ci % 8 == 4 ? &gev[gk][nev * (ci / 8)] : nullptr,
                                 true);
@@ -1988,6 +1989,7 @@ double Case::solve_system_ref(const SolveRef& R, int* iters, bool fp64) {
     hS->rtol = SS.rtol;
     hS->itmax = SS.itmax == 0 ? 2 * n : SS.itmax;
     const int gk = R.gk;
+    ChunkGraph* chunks = R.chunks ? R.chunks : chunk_graph[gk];
     // the DILU factor and applications as cooperative launches report a
     // barrier wait that gave up through ws.err, read back with the residual
     // below (it stays 0 otherwise)
@@ -2000,10 +2002,10 @@ double Case::solve_system_ref(const SolveRef& R, int* iters, bool fp64) {
         KrylovVecs<double> V{ws.x.p, ws.r.p, ws.z.p, ws.p.p, ws.q.p, ws.v.p, ws.s.p, ws.t.p};
         if (SS.solver == XCAL_SOLVER_CG) {
             kr_init_resid(stream, A, nz, b, field, ws.dx.p, V.x, V.r);
-            krylov_iterate<double>(E, SS, nz, E.P.p, b, V.r, V, S, hS, gk);
+            krylov_iterate<double>(E, SS, nz, E.P.p, b, V.r, V, S, hS, gk, chunks);
         } else {
             kr_init_resid(stream, A, nz, b, field, ws.dx.p, V.x, V.q);  // r0 in q
-            krylov_iterate<double>(E, SS, nz, E.P.p, b, V.q, V, S, hS, gk);
+            krylov_iterate<double>(E, SS, nz, E.P.p, b, V.q, V, S, hS, gk, chunks);
         }
         kr_finish(stream, n, V.x, ws.dx.p, field);
         if (iters) *iters = hS->iter;
@@ -2093,10 +2095,11 @@ void Case::solve_mixed(Equation& E, const xcal_solver_setup& SS, double* field, 
         }
         if (SS.solver == XCAL_SOLVER_CG) {
             kr_defect(stream, A, E.nz.p, b, field, V.r, V.x);
-            krylov_iterate<float>(E, SS, E.nz32.p, E.P32.p, (const float*)V.r, V.r, V, S, hS, gk);
+            krylov_iterate<float>(E, SS, E.nz32.p, E.P32.p, (const float*)V.r, V.r, V, S, hS, gk, chunk_graph[gk]);
         } else {
             kr_defect(stream, A, E.nz.p, b, field, ws.fd.p, V.x);
-            krylov_iterate<float>(E, SS, E.nz32.p, E.P32.p, (const float*)ws.fd.p, ws.fd.p, V, S, hS, gk);
+            krylov_iterate<float>(E, SS, E.nz32.p, E.P32.p, (const float*)ws.fd.p, ws.fd.p, V, S, hS, gk,
+                                  chunk_graph[gk]);
         }
         if (hS->outer_conv) break;  // this defect already met the target
         total += hS->iter;

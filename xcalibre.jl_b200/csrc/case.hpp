@@ -294,6 +294,7 @@ struct Case {
         double* field;
         const double* b;
         int slot, kslot, gk;
+        ChunkGraph* chunks = nullptr;  // [plain, profiled]; else the case's own of gk
     };
     SolveRef solve_ref(int eqn, int comp);
     double solve_system_ref(const SolveRef& R, int* iters, bool fp64);
@@ -361,7 +362,7 @@ struct Case {
     int* factor_err() { return batch_err ? batch_err : ws.err.p; }
     template <class T>
     void krylov_iterate(Equation& E, const xcal_solver_setup& SS, const T* nz, const T* P, const T* c, const T* r0,
-                        const KrylovVecs<T>& V, KScalars* S, KScalars* hS, int gk);
+                        const KrylovVecs<T>& V, KScalars* S, KScalars* hS, int gk, ChunkGraph* chunks);
     void solve_mixed(Equation& E, const xcal_solver_setup& SS, double* field, const double* b, KScalars* S,
                      KScalars* hS, int gk, int* iters);
     // mixed precision, CG + Jacobi: whether the inner solves of E run on the

@@ -219,6 +219,18 @@ struct xcal_equation {
     std::vector<std::unique_ptr<DBuf<double>>> arrays;  // term fluxes and source fields, storage order
     DBuf<double> prev, phi, stage;
     bool euler = false, extrapolated = false;
+    // captured chunks of its solves: they hold this equation's arrays and the
+    // solver and preconditioner they were captured with
+    Case::ChunkGraph chunks[2];
+    int chunks_of[2] = {-1, -1};  // that solver and preconditioner
+    void drop_chunks() {
+        for (auto& g : chunks)
+            if (g.exec) {
+                cudaGraphExecDestroy(g.exec);
+                g.exec = nullptr;
+            }
+    }
+    ~xcal_equation() { drop_chunks(); }
 };
 
 namespace {
@@ -410,7 +422,10 @@ int32_t xcal_equation_solve(xcal_equation* q, const xcal_solver_setup* setup, do
                              setup->smoother_loops, setup->smoother_omega);
         // the p system's Krylov workspace and scalars (report slot 6); FP64
         // whatever the case's precision
-        Case::SolveRef R{&q->E, *setup, q->phi.p, q->E.b[0].p, 0, 1, 6};
+        if (q->chunks_of[0] != setup->solver || q->chunks_of[1] != setup->precond) q->drop_chunks();
+        q->chunks_of[0] = setup->solver;
+        q->chunks_of[1] = setup->precond;
+        Case::SolveRef R{&q->E, *setup, q->phi.p, q->E.b[0].p, 0, 1, 6, q->chunks};
         int its = 0;
         const double r = c->solve_system_ref(R, &its, true);
         launch_gather(c->stream, m.nC, q->phi.p, m.d_inv.p, c->io.p);

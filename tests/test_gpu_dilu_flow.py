@@ -163,3 +163,34 @@ def test_dilu_form_changed_between_steps(x, ctx, modes):
         dm.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("before", [False, True])
+def test_dilu_mode_back_to_default(x, ctx, before):
+    """Mode 0 after another mode, set before or after the first step, is a new
+    case's choice: the same forms and as many launches per step."""
+    mesh = x.build_mesh3(MESHES["4620"](x))
+    out = []
+    for modes in ((), (1, 0), (2, 0), (3, 0)):
+        cfg, keep = _config(x, mesh, "mixed")
+        dm = x.DeviceMesh(ctx, mesh)
+        c = x.Case(dm, cfg)
+        _start(x, c, mesh)
+        if before:
+            for m in modes:
+                c.set_dilu_mode(m)
+        c.simple_iterate(1)
+        if not before:
+            for m in modes:
+                c.set_dilu_mode(m)
+            _start(x, c, mesh)
+        t = c.tuning()
+        l0 = x.launch_count()
+        c.simple_iterate(1)
+        out.append((t, x.launch_count() - l0))
+        c.close()
+        dm.close()
+    assert out[0][0]["U"]["dilu_grid"] and out[0][0]["p"]["dilu_grid"]
+    for o in out[1:]:
+        assert o[0] == out[0][0]
+        assert o[1] == out[0][1]

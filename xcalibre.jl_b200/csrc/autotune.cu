@@ -122,11 +122,7 @@ void Case::autotune() {
                 g_spmv_choice[k] = sh;
             }
         }
-        if (dilu_mode != 0) {
-            E.use_block = dilu_mode == 1;
-            E.use_grid = dilu_mode == 3;
-            E.use_flow = E.flow_D = false;
-        } else if (SS.precond == XCAL_PRECOND_DILU) {
+        if (dilu_mode == 0 && SS.precond == XCAL_PRECOND_DILU) {
             TuneKey k = key_of(1, tsz, E);
             std::unique_lock<std::mutex> lk(g_tune_mu);
             auto it = g_dilu_choice.find(k);

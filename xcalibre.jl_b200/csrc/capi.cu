@@ -475,14 +475,7 @@ int32_t xcal_case_set_inner_cg(xcal_case* cs, int32_t mode) {
 int32_t xcal_case_set_dilu_mode(xcal_case* cs, int32_t mode) {
     if (!cs || mode < 0 || mode > 3) return XCAL_ERR_INVALID;
     Case* c = cs->c.get();
-    if (mode == c->dilu_mode) return XCAL_OK;
-    c->drop_graphs();  // they hold the previous form
-    c->dilu_mode = mode;
-    if (mode != 0) {
-        c->U.use_block = c->P.use_block = mode == 1;
-        c->U.use_grid = c->P.use_grid = mode == 3;
-        c->U.use_flow = c->P.use_flow = c->U.flow_D = c->P.flow_D = false;
-    }
+    c->set_dilu_mode(mode);
     return XCAL_OK;
 }
 

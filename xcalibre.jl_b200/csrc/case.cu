@@ -2613,6 +2613,19 @@ void Case::set_inner_cg(int mode) {
     }
 }
 
+void Case::set_dilu_mode(int mode) {
+    if (mode == dilu_mode) return;
+    drop_graphs();  // they hold the previous form
+    dilu_mode = mode;
+    for (Equation* E : {&U, &P}) {
+        E->use_block = mode == 1;
+        E->use_grid = mode == 3;
+        // back at 0 as a new case is, its launch shapes yet to be chosen
+        E->use_flow = E->flow_D = mode == 0 && !E->lower_off.empty();
+    }
+    if (mode == 0) tuned = false;
+}
+
 void Case::set_graph_mode(bool on) {
     if (on == graph_mode) return;
     sync();

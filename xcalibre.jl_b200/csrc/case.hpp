@@ -402,6 +402,7 @@ struct Case {
     bool no_auto_graph = false;  // a capture failed: replay_step() leaves this case host-driven
     void piso_body(double r3[3], double& rp);
     void set_graph_mode(bool on);
+    void set_dilu_mode(int mode);
     void courant_to_slot();
     void capture_while(const std::function<void(cudaGraphConditionalHandle)>& body);
     void solve_captured(int eqn, int comp);

@@ -194,3 +194,43 @@ def test_dilu_mode_back_to_default(x, ctx, before):
     for o in out[1:]:
         assert o[0] == out[0][0]
         assert o[1] == out[0][1]
+
+
+_SIZE_CLASS = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np
+import __graft_entry__ as ge
+x = ge.load_package()
+ctx = x.Context(0)
+n = []
+for dims in ((128, 64, 64), (100, 90, 80)):
+    mesh = x.build_mesh3(x.channel_polymesh(*dims))
+    model, config = x.cases.channel_case(mesh, iterations=2)
+    config.solvers["p"].preconditioner = x.DILU()
+    cfg, keep = x.build_config(model, config)
+    c = x.Case(x.DeviceMesh(ctx, mesh), cfg)
+    l0 = x.launch_count()
+    c.tuning()
+    n.append(x.launch_count() - l0)
+    l0 = x.launch_count()
+    c.tuning()
+    assert x.launch_count() == l0
+    c.close()
+print("trials", *n)
+"""
+
+
+def test_dilu_form_timed_above_the_untimed_sizes():
+    """524,288 rows take the dataflow untimed, 720,000 (of the same power of
+    two) have their forms timed although a case of the first size came before
+    (a process of its own: choices are kept per process)."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _SIZE_CLASS, root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    n = [int(v) for v in r.stdout.split()[-2:]]
+    # p's trials: each form at least three times
+    assert n[1] >= 9, n

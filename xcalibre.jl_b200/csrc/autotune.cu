@@ -75,6 +75,7 @@ static SpmvShape tune_spmv(Case& C, Equation& E, const T* nz, const T* x, T* y) 
 // 20.3 / 18.6), where the fused BiCGSTAB then shares one sweep among three
 // components.  Above, both are timed (884,736 rows FP32: 117 / 155; 2.1M rows:
 // 233 / 192, FP64 283 / 252).
+constexpr int FLOW_UNTIMED_ROWS = 524288;
 template <class T>
 static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, T* out) {
     const int reps = (int)std::max(3L, std::min(20L, 20000000L / std::max(E.nnz_csr, 1L)));
@@ -82,7 +83,6 @@ static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, 
     kr_flow_unset(C.stream, C.flow_scratch<T>(out), (size_t)E.n * sizeof(T));
     int best = 4;
     float best_ms = 1e30f;
-    if (E.n <= 524288) return best;
     for (int form = 2; form <= 4; ++form) {
         E.use_block = false;
         E.use_grid = form == 3;
@@ -127,7 +127,9 @@ void Case::autotune() {
             std::unique_lock<std::mutex> lk(g_tune_mu);
             auto it = g_dilu_choice.find(k);
             int form;
-            if (it != g_dilu_choice.end()) {
+            if (E.n <= FLOW_UNTIMED_ROWS) {  // not in the cache: its class (524,288 rows) also holds sizes to be timed
+                form = 4;
+            } else if (it != g_dilu_choice.end()) {
                 form = it->second;
             } else {
                 lk.unlock();

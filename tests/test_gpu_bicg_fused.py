@@ -80,3 +80,27 @@ def test_fused_mixed(x, ctx, name, pre, rtol):
     for out in outs[1:]:
         for a, b in zip(outs[0], out):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_captured_step_is_the_same_under_profiling(x, ctx, prec):
+    """A step captured in graph mode while profiling is on is the one captured
+    with it off: as many launches, then and once profiling is off again."""
+    mesh = x.build_mesh3(MESHES["2049"](x))
+    counts = []
+    for profiled in (False, True):
+        cfg, keep = _config(x, mesh, x.DILU, 0.1, prec)
+        dm = x.DeviceMesh(ctx, mesh)
+        c = x.Case(dm, cfg)
+        c.set_graph_mode(True)
+        c.set_profiling(profiled)
+        n = []
+        for k in range(2):
+            l0 = x.launch_count()
+            out = _run(x, c, mesh)
+            n.append(x.launch_count() - l0)
+            c.set_profiling(False)
+        counts.append(n)
+        c.close()
+        dm.close()
+    assert counts[0][1] == counts[1][1], counts

@@ -693,14 +693,16 @@ static void bf_finish(cudaStream_t s, const BfView<T, NC>& V) {
 // The fused solve covers BiCGSTAB without a smoother at every size (momentum
 // solve per SIMPLE iteration, components in turn with the fastest DILU form
 // against this, ms: 884,736 cells mixed 2.35 / 1.08, FP64 2.45 / 1.17; 2.1M cells
-// mixed 3.50 / 2.24, FP64 3.95 / 2.74).  A chosen DILU form, and profiling, which
-// times the separate kernels, keep those; a batch runs its own batched ones.
-bool Case::use_fused(const Equation& E, const xcal_solver_setup& SS) {
-    if (SS.solver != XCAL_SOLVER_BICGSTAB || SS.smoother_loops > 0 || profiling || batch_err || dilu_mode != 0)
-        return false;
+// mixed 3.50 / 2.24, FP64 3.95 / 2.74).  A chosen DILU form keeps the separate
+// kernels, and so does profiling, which times them, but for a captured step
+// (captured): nothing is timed in it, and it outlives the profiling.  A batch
+// runs its own batched ones.
+bool Case::use_fused(const Equation& E, const xcal_solver_setup& SS, bool captured) {
+    if (SS.solver != XCAL_SOLVER_BICGSTAB || SS.smoother_loops > 0 || batch_err || dilu_mode != 0) return false;
+    if (profiling && !captured) return false;
     if (SS.precond != XCAL_PRECOND_DILU) return true;
     // the sweeps are cooperative launches, under capture inside WHILE bodies
-    return E.flow_D && !E.lower_off.empty() && (capturing ? kr_coop_capture_ok(true) : coop_ok_here());
+    return E.flow_D && !E.lower_off.empty() && (captured ? kr_coop_capture_ok(true) : coop_ok_here());
 }
 
 // Components may be solved side by side when no boundary condition of one
@@ -724,8 +726,8 @@ bool Case::components_apart() {
 // first fused momentum solve (a case in a batch has none), never under capture;
 // where they (above 64 MB) would take more than a quarter of the free memory the
 // components are solved in turn
-void Case::reserve_fused() {
-    if (bf.ready || bf.refused || capturing || !use_fused(U, cfg.U_solver) || !components_apart()) return;
+void Case::reserve_fused(bool captured) {
+    if (bf.ready || bf.refused || capturing || !use_fused(U, cfg.U_solver, captured) || !components_apart()) return;
     const bool mixed = cfg.precision == XCAL_PREC_MIXED;
     const size_t n = U.n, T = (n + RED_TILE - 1) / RED_TILE;
     // one allocation: seven cost a new case's first step 0.1-0.2 ms (1,073 and

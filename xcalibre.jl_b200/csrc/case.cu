@@ -1951,7 +1951,7 @@ Case::SolveRef Case::solve_ref(int eqn, int comp) {
 double Case::solve_system(int eqn, int comp, int* iters) {
     {
         const SolveRef R = solve_ref(eqn, comp);
-        if (use_fused(*R.E, R.SS)) {
+        if (use_fused(*R.E, R.SS, capturing)) {
             double res = 0.0;
             if (cfg.precision == XCAL_PREC_MIXED)
                 fused_solve<float, 1>(*R.E, R.SS, &R, &res);
@@ -2116,8 +2116,8 @@ void Case::solve_mixed(Equation& E, const xcal_solver_setup& SS, double* field, 
 
 void Case::solve_equation_U(double res[3]) {  // Solve_1_api.jl:233-266
     discretise(XCAL_EQN_U);
-    reserve_fused();
-    if (bf.ready && use_fused(U, cfg.U_solver) && components_apart()) {
+    reserve_fused(capturing);
+    if (bf.ready && use_fused(U, cfg.U_solver, capturing) && components_apart()) {
         SolveRef R[3];
         for (int d = 0; d < 3; ++d) {
             bc_relax_U(d, bf.diag + (size_t)d * U.n);
@@ -2424,7 +2424,7 @@ void Case::piso_body(double r3[3], double& rp) {
 void Case::capture_step() {
     if (step_graph) return;
     autotune();
-    reserve_fused();
+    reserve_fused(true);
     sync();
     const long long t0 = t_launch_count;
     body_kernels_captured = 0;

@@ -347,9 +347,9 @@ struct Case {
         KScalars* S = nullptr;
     } bf;
     int apart = -1;  // components_apart(), once known
-    bool use_fused(const Equation& E, const xcal_solver_setup& SS);
+    bool use_fused(const Equation& E, const xcal_solver_setup& SS, bool captured);
     bool components_apart();
-    void reserve_fused();
+    void reserve_fused(bool captured);
     template <class T, int NC>
     BfView<T, NC> bf_view(Equation& E, const xcal_solver_setup& SS, const SolveRef* R);
     template <class T, int NC>

@@ -447,13 +447,10 @@ int32_t xcal_case_set_persistent(xcal_case* cs, int32_t mode) {
         mode != 512 && mode != 1024)
         return XCAL_ERR_INVALID;
     Case* c = cs->c.get();
-    if (mode != c->persistent_cg && c->step_graph) {  // a captured step holds the previous form
-        c->sync();
-        cudaGraphExecDestroy(c->step_graph);
-        c->step_graph = nullptr;
-    }
-    c->persistent_cg = mode;
-    return XCAL_OK;
+    XCAL_GUARD(c->ctx, {
+        if (mode != c->persistent_cg) c->drop_graphs();  // a captured step holds the previous form
+        c->persistent_cg = mode;
+    })
 }
 
 int32_t xcal_case_solve_report(const xcal_case* cs, int32_t* iters7, int32_t* status7, int64_t* itmax_hits) {
@@ -475,8 +472,7 @@ int32_t xcal_case_set_inner_cg(xcal_case* cs, int32_t mode) {
 int32_t xcal_case_set_dilu_mode(xcal_case* cs, int32_t mode) {
     if (!cs || mode < 0 || mode > 3) return XCAL_ERR_INVALID;
     Case* c = cs->c.get();
-    c->set_dilu_mode(mode);
-    return XCAL_OK;
+    XCAL_GUARD(c->ctx, c->set_dilu_mode(mode));
 }
 
 int32_t xcal_case_tuning(xcal_case* cs, int32_t* out6) {

@@ -1000,7 +1000,7 @@ Case::Case(xcal_ctx* c, const DevMesh* m, const xcal_config* cf) : ctx(c), mesh(
 // form they were captured with, and the dataflow form relies on scratch that
 // only its own refresh resets: a form may change only with the graphs gone.
 void Case::drop_graphs() {
-    if (stream) cudaStreamSynchronize(stream);
+    if (stream) cudaStreamSynchronize(stream);  // an error stays for the next call to report
     for (auto& row : chunk_graph)
         for (auto& g : row)
             if (g.exec) {

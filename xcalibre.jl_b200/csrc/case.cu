@@ -1783,23 +1783,30 @@ void Case::capture_while(const std::function<void(cudaGraphConditionalHandle)>& 
     XCAL_CUDA(cudaGraphAddNode(&node, g, deps, nd, &prm));
     cudaGraph_t bodyg = prm.conditional.phGraph_out[0];
     if (!side[side_depth]) XCAL_CUDA(cudaStreamCreateWithFlags(&side[side_depth], cudaStreamNonBlocking));
-    cudaStream_t outer = stream;
-    stream = side[side_depth++];
     const long long kb = t_launch_count;
-    XCAL_CUDA(cudaStreamBeginCaptureToGraph(stream, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    try {
-        body(h);
-    } catch (...) {
+    {
+        // whatever fails below, the case is back on its own stream after it:
+        // a step that cannot be captured is driven from the host
+        struct Side {
+            Case& c;
+            cudaStream_t outer;
+            explicit Side(Case& cs) : c(cs), outer(cs.stream) { c.stream = c.side[c.side_depth++]; }
+            ~Side() {
+                c.stream = outer;
+                --c.side_depth;
+            }
+        } on_side(*this);
+        XCAL_CUDA(cudaStreamBeginCaptureToGraph(stream, bodyg, nullptr, nullptr, 0,
+                                                cudaStreamCaptureModeThreadLocal));
         cudaGraph_t tmp;
-        cudaStreamEndCapture(stream, &tmp);
-        stream = outer;
-        --side_depth;
-        throw;
+        try {
+            body(h);
+        } catch (...) {
+            cudaStreamEndCapture(stream, &tmp);
+            throw;
+        }
+        XCAL_CUDA(cudaStreamEndCapture(stream, &tmp));
     }
-    cudaGraph_t tmp;
-    XCAL_CUDA(cudaStreamEndCapture(stream, &tmp));
-    stream = outer;
-    --side_depth;
     last_body_kernels = t_launch_count - kb;
     if (side_depth == 0) body_kernels_captured += last_body_kernels;
     XCAL_CUDA(cudaStreamUpdateCaptureDependencies(stream, &node, 1, cudaStreamSetCaptureDependencies));
@@ -2445,13 +2452,16 @@ void Case::capture_step() {
         capturing = false;
         cudaStreamEndCapture(stream, &g);
         if (g) cudaGraphDestroy(g);
+        cudaGetLastError();
+        g_launch_count.fetch_sub(t_launch_count - t0, std::memory_order_relaxed);
+        t_launch_count = t0;
         throw;
     }
     capturing = false;
-    XCAL_CUDA(cudaStreamEndCapture(stream, &g));
     const long long captured = t_launch_count - t0;
     g_launch_count.fetch_sub(captured, std::memory_order_relaxed);
     t_launch_count = t0;
+    XCAL_CUDA(cudaStreamEndCapture(stream, &g));
     step_top_kernels = captured - body_kernels_captured;
     cudaError_t e = cudaGraphInstantiate(&step_graph, g, 0);
     cudaGraphDestroy(g);

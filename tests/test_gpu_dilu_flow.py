@@ -199,14 +199,18 @@ def test_dilu_mode_back_to_default(x, ctx, before):
 _SIZE_CLASS = """
 import sys
 sys.path.insert(0, sys.argv[1])
+prec, sizes = sys.argv[2], [tuple(map(int, a.split("x"))) for a in sys.argv[3:]]
 import numpy as np
 import __graft_entry__ as ge
 x = ge.load_package()
 ctx = x.Context(0)
 n = []
-for dims in ((128, 64, 64), (100, 90, 80)):
+for dims in sizes:
     mesh = x.build_mesh3(x.channel_polymesh(*dims))
-    model, config = x.cases.channel_case(mesh, iterations=2)
+    model, config = x.cases.channel_case(mesh, iterations=2, precision=prec)
+    u = config.solvers["U"]
+    config.solvers["U"] = x.SolverSetup(solver=x.Cg(), preconditioner=x.Jacobi(), convergence=u.convergence,
+                                        relax=u.relax, rtol=u.rtol)
     config.solvers["p"].preconditioner = x.DILU()
     cfg, keep = x.build_config(model, config)
     c = x.Case(x.DeviceMesh(ctx, mesh), cfg)
@@ -221,16 +225,46 @@ print("trials", *n)
 """
 
 
-def test_dilu_form_timed_above_the_untimed_sizes():
-    """524,288 rows take the dataflow untimed, 720,000 (of the same power of
-    two) have their forms timed although a case of the first size came before
-    (a process of its own: choices are kept per process)."""
+def _trials(prec, *sizes):
+    """Kernels each case's tuning launched, the cases made in turn in a process
+    of its own (choices are kept per process); only p's DILU is tuned."""
     import os
     import subprocess
     import sys
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, "-c", _SIZE_CLASS, root], capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", _SIZE_CLASS, root, prec, *sizes], capture_output=True, text=True,
+                       timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
-    n = [int(v) for v in r.stdout.split()[-2:]]
-    # p's trials: each form at least three times
-    assert n[1] >= 9, n
+    return [int(v) for v in r.stdout.split("trials")[1].split()]
+
+
+def test_dilu_form_timed_above_the_untimed_sizes():
+    """524,288 rows take the dataflow untimed, 720,000 (of the same power of
+    two) have their forms timed although a case of the first size came before."""
+    n = _trials("fp64", "128x64x64", "100x90x80")
+    assert n[0] == 0 and n[1] >= 9, n  # three forms, each at least three times
+
+
+@pytest.mark.parametrize("prec,dims,one_block", [("mixed", (7, 73, 1), False), ("mixed", (8, 8, 8), True),
+                                                 ("mixed", (819, 5, 1), True), ("mixed", (16, 16, 16), False),
+                                                 ("fp64", (8, 8, 8), False)])
+def test_dilu_form_of_small_systems(x, ctx, prec, dims, one_block):
+    """A DILU-CG in mixed precision runs one-block sweeps at 512 to 4,095 rows
+    and the dataflow at 511 and 4,096, with the results of the level kernels; a
+    BiCGSTAB (fused) and FP64 take the dataflow."""
+    mesh = x.build_mesh3(x.channel_polymesh(*dims, seed=2))
+    out = []
+    for mode in (0, 2):
+        cfg, keep = _config(x, mesh, prec)
+        dm = x.DeviceMesh(ctx, mesh)
+        c = x.Case(dm, cfg)
+        c.set_inner_cg(1)
+        c.set_dilu_mode(mode)
+        if mode == 0:
+            t = c.tuning()
+            assert t["p"]["dilu_one_block"] == one_block and not t["U"]["dilu_one_block"]
+        out.append(_run(x, c, mesh))
+        c.close()
+        dm.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

@@ -7,8 +7,9 @@
 //  * how a DILU application of a system of more than 524,288 rows runs: rows
 //    waiting for the values they read (dataflow), one launch per level, or
 //    every level in one cooperative launch with a grid barrier between levels
-//    (the fused BiCGSTAB, which shares the waits among components, is always
-//    a dataflow).
+//    (smaller ones take the dataflow or, some FP32 ones, one-block sweeps
+//    untimed; the fused BiCGSTAB, which shares the waits among components, is
+//    always a dataflow).
 // Each candidate is timed with CUDA events on the case's own matrix at first
 // use; choices are cached per size class (value size, log2 rows, entries per
 // row), so later cases of the same class reuse them without timing.
@@ -68,13 +69,9 @@ static SpmvShape tune_spmv(Case& C, Equation& E, const T* nz, const T* x, T* y) 
 }
 
 // the fastest DILU form on this system: 2 one launch per level, 3 one
-// cooperative launch over every level, 4 dataflow.  Up to 524,288 rows dataflow
-// is taken as it is: measured on B200 (us per application, dataflow against
-// the best other form) 27,025 rows FP64 37 / 88, 262,144 rows FP32 61 / 131;
-// one-block sweeps come within reach only below some 4k rows (1,518 rows FP32
-// 20.3 / 18.6), where the fused BiCGSTAB then shares one sweep among three
-// components.  Above, both are timed (884,736 rows FP32: 117 / 155; 2.1M rows:
-// 233 / 192, FP64 283 / 252).
+// cooperative launch over every level, 4 dataflow (884,736 rows FP32, us per
+// application, dataflow / the best other form: 117 / 155; 2.1M rows: 233 / 192,
+// FP64 283 / 252).  Up to FLOW_UNTIMED_ROWS nothing is timed (untimed_form).
 constexpr int FLOW_UNTIMED_ROWS = 524288;
 template <class T>
 static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, T* out) {
@@ -97,6 +94,21 @@ static int tune_dilu(Case& C, Equation& E, const T* nz, const T* D, const T* b, 
     E.use_grid = sg;
     E.use_flow = sf;
     return best;
+}
+
+// Up to FLOW_UNTIMED_ROWS dataflow is taken as it is: measured on B200 (us per
+// application, dataflow / the best other form) 27,025 rows FP64 37 / 88, 262,144
+// rows FP32 61 / 131.  But an FP32 system of 512 to 4,095 rows whose solve
+// applies DILU by itself (alone: a CG, or a smoothed BiCGSTAB; the fused one
+// shares a dataflow among its components) takes one-block sweeps, 1: y in shared
+// memory and one launch, not a cooperative one behind a memset.  Whole DILU-CG
+// iterations, us, dataflow / one block, FP32: 250 rows 48.4 / 53.8, 512 rows
+// 50.1 / 45.4, 1,073 rows 43.3 / 35.8, 1,920 rows 58.1 / 49.9, 3,072 rows 51.3 /
+// 49.1, 4,160 rows 53.3 / 54.1, 5,984 rows 49.8 / 54.0; FP64 250 rows 35.4 / 40.4,
+// 1,073 rows 36.8 / 38.2, 3,072 rows 47.1 / 54.4.  (Timed alone, back to back, the launch hides: the
+// dataflow then looks faster at 1,920 rows too.)
+static int untimed_form(int n, bool fp32, bool alone) {
+    return fp32 && alone && n >= 512 && n < 4096 ? 1 : 4;
 }
 
 void Case::autotune() {
@@ -123,12 +135,13 @@ void Case::autotune() {
             }
         }
         if (dilu_mode == 0 && SS.precond == XCAL_PRECOND_DILU) {
+            const bool alone = SS.solver == XCAL_SOLVER_CG || SS.smoother_loops > 0;
             TuneKey k = key_of(1, tsz, E);
             std::unique_lock<std::mutex> lk(g_tune_mu);
             auto it = g_dilu_choice.find(k);
             int form;
             if (E.n <= FLOW_UNTIMED_ROWS) {  // not in the cache: its class (524,288 rows) also holds sizes to be timed
-                form = 4;
+                form = untimed_form(E.n, mixed, alone);
             } else if (it != g_dilu_choice.end()) {
                 form = it->second;
             } else {

@@ -91,3 +91,24 @@ def test_resident_batch_mixed_sizes(x, ctx):
             batch.close()
             for c, keep in members:
                 c.close()
+
+
+@pytest.mark.parametrize("n", [(7, 5, 3), (69, 49, 20)])
+def test_resident_tables_only_where_read(x, ctx, n):
+    """A system none of whose solves can be a resident CG holds no tables for
+    it: a Jacobi-BiCGSTAB U against a Jacobi-CG U."""
+    mesh = x.build_mesh3(x.channel_polymesh(*n, seed=2))
+    size = {}
+    for u in ("Bicgstab", "Cg"):
+        model, config = x.cases.channel_case(mesh, iterations=2)
+        s = config.solvers["U"]
+        config.solvers["U"] = x.SolverSetup(solver=getattr(x, u)(), preconditioner=x.Jacobi(),
+                                            convergence=s.convergence, relax=s.relax, rtol=s.rtol)
+        cfg, keep = x.build_config(model, config)
+        dm = x.DeviceMesh(ctx, mesh)
+        c = x.Case(dm, cfg)
+        size[u] = c.footprint()[0]
+        c.close()
+        dm.close()
+    # two bytes per row at least
+    assert size["Cg"] - size["Bicgstab"] >= 2 * mesh.n_cells, size

@@ -797,8 +797,9 @@ size_t estimate_case_bytes(long nC, long nF, long nB, int mixed, int dilu_U, int
     // partials and small buffers
     b += nC * (26.0 + 9.0) * 8.0 + nF * 8.0 * 8.0 + (mixed ? 52.0 * nC + 16384.0 : 0.0);
     b += 3.0 * 8.0 * (nC / 2048 + 1) + 4096.0;
-    // resident CG: four buffers of a partial per tile and block; about two halo
-    // entries per three rows, each with its partner and row, in two equations
+    // resident CG: four buffers of a partial per tile and block; in up to two
+    // equations a count per row and (cluster form) about two halo entries per
+    // three rows, each with its partner and row
     const double T = (nC + 2047) / 2048;
     if (T <= RES_TILES_MAX) b += 32.0 * T * T + 4.0 * nC + (T > 1 ? 0.67 * nC * 2 * 6.0 : 0.0);
     // permutations (mesh) and the field staging buffer (case)

@@ -37,7 +37,7 @@ struct BSys {
     KScalars* S;
     double* part0;
     double* part1;
-    double* ring;  // resident CG: 4 ntiles^2 doubles
+    double* ring;  // resident CG: 4 ntiles^2 doubles (or null)
     int n;
     int ntiles;
     // level-ordered triangles and the scratch of the DILU sweeps

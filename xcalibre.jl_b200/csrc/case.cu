@@ -56,10 +56,10 @@ CSRView Equation::view() const {
     v.cf_slot = d_cf_slot.p;
     v.tile_slots = tile_slots;
     v.tile_halo = tile_halo;
-    v.hoff = d_hoff.p;
-    v.hdst = d_hdst.p;
-    v.hrow = d_hrow.p;
-    v.rowh = d_rowh.p;
+    v.hoff = d_halo.p;
+    v.hdst = d_halo.p + halo_dst;
+    v.rowh = reinterpret_cast<const unsigned short*>(d_halo.p + halo_row);
+    v.hrow = v.rowh + n;
     v.fslot = d_fslot.p;
     return v;
 }
@@ -426,11 +426,78 @@ static void build_fold(Equation& E, cudaStream_t s, bool uniform_ok) {
     E.fold_built = true;
 }
 
+// most tiles the resident CG takes on this device: one per SM
+static int resident_tiles() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        sms = 0;
+    }
+    return std::min(sms, RES_TILES_MAX);
+}
+
+// What the resident CG keeps per tile, and its halo entries (CSRView), for
+// systems of at most one tile per SM: one upload, and where each entry's value
+// goes only for the cluster form (a device allocation costs some 0.35 ms, the
+// lists of 62,403 cells on the host about as much).
+static void build_resident(Equation& E, const std::vector<int>& trans, cudaStream_t s) {
+    constexpr int TILE = 2048;
+    const int n = E.n, T = (n + TILE - 1) / TILE;
+    if (T > resident_tiles()) return;
+    const bool cluster = T <= PERSIST_CLUSTER_MAX;
+    std::vector<int> hoff(1, 0), hslot;
+    std::vector<unsigned short> rowh(n), hrow;
+    int nh = 0;
+    for (int r0 = 0; r0 < n; r0 += TILE) {
+        const int r1 = std::min(n, r0 + TILE);
+        for (int r = r0; r < r1; ++r) {
+            rowh[r] = (unsigned short)std::min(nh - hoff.back(), 65535);
+            const int b = E.base(r);
+            for (int k = 0; k < E.len[r]; ++k) {
+                const int e = b + SELL_C * k, c = E.colval[e];
+                if (c >= r0 && c < r1) continue;
+                if (cluster) {
+                    hslot.push_back(e);
+                    hrow.push_back((unsigned short)(r - r0));
+                }
+                ++nh;
+            }
+        }
+        E.tile_halo = std::max(E.tile_halo, nh - hoff.back());
+        E.tile_slots = std::max(E.tile_slots, E.slice[(r1 + SELL_C - 1) / SELL_C] - E.slice[r0 / SELL_C]);
+        hoff.push_back(nh);
+    }
+    std::vector<int> hdst(hslot.size());
+    if (cluster) {
+        std::vector<int> entry(E.nnz, -1);
+        for (int g = 0; g < nh; ++g) entry[hslot[g]] = g;
+        for (int g = 0; g < nh; ++g) {
+            if (trans[hslot[g]] < 0) {  // an entry without its transposed one: not this form
+                E.tile_slots = E.tile_halo = 0;
+                return;
+            }
+            hdst[g] = entry[trans[hslot[g]]];
+        }
+    }
+    // hoff, hdst, then the 16-bit rowh and hrow
+    E.halo_dst = (int)hoff.size();
+    E.halo_row = E.halo_dst + (int)hdst.size();
+    std::vector<int> all(E.halo_row + (rowh.size() + hrow.size() + 1) / 2);
+    std::copy(hoff.begin(), hoff.end(), all.begin());
+    std::copy(hdst.begin(), hdst.end(), all.begin() + E.halo_dst);
+    unsigned short* sh = reinterpret_cast<unsigned short*>(all.data() + E.halo_row);
+    std::copy(rowh.begin(), rowh.end(), sh);
+    std::copy(hrow.begin(), hrow.end(), sh + n);
+    E.d_halo.upload(all, s);
+    XCAL_CUDA(cudaStreamSynchronize(s));  // the host copy goes out of scope
+}
+
 // ---------------------------------------------------------------------------
 // equation pattern (sparse_matrix_connectivity + extend_matrix + sparsecsr)
 // ---------------------------------------------------------------------------
 void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& bcs, int nvec,
-                           bool need_dilu, cudaStream_t s) {
+                           bool need_dilu, bool resident, cudaStream_t s) {
     int n = E.n = m.nC;
     E.use_flow = E.flow_D = need_dilu;
     std::vector<std::vector<int>> extra(n);
@@ -508,40 +575,7 @@ void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& b
                 if (!set[e]) trans[e] = E.find(E.colval[e], i);
             }
     }
-    // what the resident CG keeps per tile, and its halo entries (CSRView)
-    constexpr int TILE = 2048;
-    E.tile_slots = E.tile_halo = 0;
-    if (n <= RES_TILES_MAX * TILE) {
-        std::vector<int> hoff(1, 0), hslot, entry(E.nnz, -1);
-        std::vector<unsigned short> hrow, rowh(n);
-        bool ok = true;
-        for (int r0 = 0; r0 < n; r0 += TILE) {
-            const int r1 = std::min(n, r0 + TILE);
-            for (int r = r0; r < r1; ++r) {
-                rowh[r] = (unsigned short)std::min((int)hslot.size() - hoff.back(), 65535);
-                for (int k = 0; k < E.len[r]; ++k) {
-                    const int e = E.base(r) + SELL_C * k, c = E.colval[e];
-                    if (c >= r0 && c < r1) continue;
-                    ok = ok && trans[e] >= 0;
-                    entry[e] = (int)hslot.size();
-                    hslot.push_back(e);
-                    hrow.push_back((unsigned short)(r - r0));
-                }
-            }
-            E.tile_halo = std::max(E.tile_halo, (int)hslot.size() - hoff.back());
-            E.tile_slots = std::max(E.tile_slots, E.slice[(r1 + SELL_C - 1) / SELL_C] - E.slice[r0 / SELL_C]);
-            hoff.push_back((int)hslot.size());
-        }
-        std::vector<int> hdst(hslot.size());
-        for (size_t g = 0; ok && g < hslot.size(); ++g) hdst[g] = entry[trans[hslot[g]]];
-        E.n_halo = (long)hslot.size();
-        if (!ok) E.tile_slots = 0;  // an entry without its transposed one: not this form
-        E.d_hoff.upload(hoff, s);
-        E.d_hdst.upload(hdst, s);
-        E.d_hrow.upload(hrow, s);
-        E.d_rowh.upload(rowh, s);
-        XCAL_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
-    }
+    if (resident) build_resident(E, trans, s);
     E.d_slice.upload(E.slice, s);
     E.d_len.upload(E.len, s);
     E.d_colval.upload(E.colval, s);
@@ -798,14 +832,21 @@ Case::Case(xcal_ctx* c, const DevMesh* m, const xcal_config* cf) : ctx(c), mesh(
     XCAL_CUDA(cudaMallocHost(&h_res, 16 * sizeof(double)));
     int nC = m->nC, nF = m->nF;
     std::vector<xcal_bc> bU(cfg.bc_U, cfg.bc_U + cfg.n_bc_U), bP(cfg.bc_p, cfg.bc_p + cfg.n_bc_p);
-    build_equation(U, *m, bU, 3, cfg.U_solver.precond == XCAL_PRECOND_DILU, stream);
+    // a system's tables for the resident CG are built where a solve on it may
+    // be one: a CG with Jacobi or no preconditioner
+    auto cg = [](const xcal_solver_setup& ss) {
+        return ss.solver == XCAL_SOLVER_CG && ss.precond != XCAL_PRECOND_DILU;
+    };
+    build_equation(U, *m, bU, 3, cfg.U_solver.precond == XCAL_PRECOND_DILU, cg(cfg.U_solver), stream);
     // the p system's storage also carries k, omega, kl and the wall distance:
     // its DILU levels are needed when any solve on it is DILU-preconditioned
     auto dilu = [](const xcal_solver_setup& ss) { return ss.precond == XCAL_PRECOND_DILU; };
     const bool p_dilu = dilu(cfg.p_solver) || (has_k() && dilu(cfg.k_solver)) ||
                         (rans_kw() && dilu(cfg.omega_solver)) || (lke() && dilu(cfg.kl_solver)) ||
                         (has_y() && dilu(cfg.y_solver));
-    build_equation(P, *m, bP, 1, p_dilu, stream);
+    const bool p_cg = cg(cfg.p_solver) || (has_k() && cg(cfg.k_solver)) || (rans_kw() && cg(cfg.omega_solver)) ||
+                      (lke() && cg(cfg.kl_solver)) || (has_y() && cg(cfg.y_solver));
+    build_equation(P, *m, bP, 1, p_dilu, p_cg, stream);
     build_bc_table(bcU, *m, cfg.bc_U, cfg.n_bc_U, 3, &U, stream);
     build_bc_table(bcP, *m, cfg.bc_p, cfg.n_bc_p, 1, &P, stream);
     build_bc_table(bcNut, *m, cfg.bc_nut, cfg.n_bc_nut, 1, nullptr, stream);
@@ -931,7 +972,7 @@ Case::Case(xcal_ctx* c, const DevMesh* m, const xcal_config* cf) : ctx(c), mesh(
     }
     ws.part0.alloc(T);
     ws.part1.alloc(T);
-    if (T <= RES_TILES_MAX) ws.ring.alloc(4L * T * T);
+    if (T <= resident_tiles()) ws.ring.alloc(4L * T * T);
     ws.bar.alloc(2);
     ws.bar.zero(stream);
     ws.err.alloc(1);

@@ -89,9 +89,8 @@ struct Equation {
     DBuf<int> d_slice, d_colval, d_diag, d_trans, d_cf_slot, d_fslot;
     DBuf<unsigned char> d_len;
     int tile_slots = 0, tile_halo = 0;  // CSRView: what the resident CG keeps per tile
-    long n_halo = 0;                    // its halo entries over all tiles
-    DBuf<int> d_hoff, d_hdst;
-    DBuf<unsigned short> d_hrow, d_rowh;
+    DBuf<int> d_halo;                   // its hoff, hdst, rowh and hrow (where any solve may use it)
+    int halo_dst = 0, halo_row = 0;     // where hdst and rowh start in it
     int base(int r) const { return slice[r / SELL_C] + r % SELL_C; }
     DBuf<double> nz, nz0, diag0, P;
     DBuf<float> nz32, P32;  // mixed precision: FP32 copies for the inner solves
@@ -124,11 +123,11 @@ struct Equation {
     int find(int i, int j) const;  // slot or -1
 };
 
-// the CSR pattern, slot maps and (need_dilu) DILU level structures of an
-// equation on mesh m (periodic BCs add their partner entries); the BC table
+// the CSR pattern, slot maps, (need_dilu) DILU level structures and (resident)
+// resident-CG tables of an equation on mesh m (periodic BCs add their partner entries); the BC table
 // of a field (E: the equation whose periodic slots it resolves, or null)
 void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& bcs, int nvec, bool need_dilu,
-                    cudaStream_t s);
+                    bool resident, cudaStream_t s);
 struct BCTable;
 void build_bc_table(BCTable& T, const DevMesh& m, const xcal_bc* bcs, int nbc, int ncomp, const Equation* E,
                     cudaStream_t s);
@@ -147,7 +146,7 @@ struct BCTable {
 
 struct KrylovWS {
     DBuf<double> x, dx, r, z, p, q, v, s, t, part0, part1;
-    DBuf<double> ring;  // resident CG: four buffers of a partial per tile and block
+    DBuf<double> ring;  // resident CG: four buffers of a partial per tile and block (up to one tile per SM)
     DBuf<float> fx, fr, fz, fp, fq, fv, fs, ft, fd;  // mixed precision inner vectors
     DBuf<double> fpart;  // folded inner CG: block partials (2 x FOLD_MAX_BLOCKS)
     DBuf<float2> frp;    // folded inner CG: two buffers of n (r, p_old) pairs

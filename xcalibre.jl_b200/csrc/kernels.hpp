@@ -176,7 +176,7 @@ template <class T>
 bool kr_cg_persist(cudaStream_t s, const CSRView& A, const T* nz, const T* P, int jacobi, T* x, T* r, T* z, T* P0,
                    T* P1, KScalars* S, double* part, double* part2, double* ring, unsigned int* bar, int* err,
                    int max_iters, int width = 0, int pf_kb = 0, bool reset_err = true);
-// ring: 4 ntiles^2 doubles (systems of at most RES_TILES_MAX tiles), set up by kr_cg_start
+// ring: 4 ntiles^2 doubles, set up by kr_cg_start (null: more tiles than the resident form takes)
 // width: 0 = the resident form (cg_resident_body) where the system has at
 // most one tile per SM and its tiles' slots fit shared memory, else the
 // cluster form where it has at most PERSIST_CLUSTER_MAX tiles, else the

@@ -979,7 +979,7 @@ bool kr_cg_persist(cudaStream_t s, const CSRView& A, const T* nz, const T* P, in
                 return true;
             }
         }
-        if (nt <= std::min(resident_sms(kr, smem), RES_TILES_MAX)) {
+        if (ring && nt <= std::min(resident_sms(kr, smem), RES_TILES_MAX)) {
             if (reset_err) XCAL_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
             CSRView Av = A;
             void* args[] = {&Av, (void*)&nz, (void*)&P, &jacobi, &x,   &r,     &z,    &P0,

@@ -250,7 +250,7 @@ __device__ __forceinline__ void cg_start_body(const TileCtx& tc, int n, const T*
                            double* part, double* ring) {
     __shared__ TileSmem<NT, 1> sh;
     // the resident CG's exchange buffers start unset (cg_resident_body)
-    if (tc.ntiles <= RES_TILES_MAX)
+    if (ring)
         for (int k = threadIdx.x; k < 4 * tc.ntiles; k += blockDim.x)
             ring[((size_t)(k / tc.ntiles) * tc.ntiles + tc.tile) * tc.ntiles + k % tc.ntiles] =
                 __longlong_as_double(-1LL);

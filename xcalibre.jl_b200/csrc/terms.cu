@@ -294,7 +294,7 @@ int32_t xcal_equation_create(xcal_case* cs, int32_t n_terms, const xcal_term* te
             if (bcs[b].type == XCAL_BC_PERIODIC || bcs[b].type == XCAL_BC_PERIODIC_PARENT)
                 fail(XCAL_ERR_UNSUPPORTED, "equation: periodic boundaries are not supported for term lists");
         std::vector<xcal_bc> bv(bcs, bcs + n_bcs);
-        build_equation(q->E, m, bv, 1, true, c->stream);
+        build_equation(q->E, m, bv, 1, true, true, c->stream);
         build_bc_table(q->bc, m, bcs, n_bcs, 1, &q->E, c->stream);
         q->E.b[0].alloc(m.nC);
         q->E.b[0].zero(c->stream);

@@ -468,8 +468,11 @@ __global__ void __launch_bounds__(FLOW_THREADS) k_dilu_flow(int n, LevelView<T> 
 // its lower neighbours (dilu_D_pos's operands and order).  No barrier: the
 // blocks draw chunks of positions from a ticket, so a chunk's dependencies
 // belong to chunks already drawn by running blocks, and the kernel needs no
-// co-residency (it also runs inside a batch's per-case graphs).
-__global__ void __launch_bounds__(FLOW_THREADS) k_dilu_D_flow(int n, LevelDView L, const double* __restrict__ nz,
+// co-residency (it also runs inside a batch's per-case graphs).  Two blocks per
+// SM: the compiler's own choice, 80 registers for three, spills (64^3 mixed: a
+// pass 19.09 ms with it, 18.98 with two; factor 49 us at 262,144 rows, 75 us at
+// 884,736).
+__global__ void __launch_bounds__(FLOW_THREADS, 2) k_dilu_D_flow(int n, LevelDView L, const double* __restrict__ nz,
                                                               double* D, unsigned int* ticket, int* err,
                                                               int spin_limit) {
     __shared__ int sh_chunk;

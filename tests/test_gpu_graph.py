@@ -156,3 +156,43 @@ def test_persistent_multi_tile_identical(x, ctx, prec):
         assert o[3] > 0
         assert np.array_equal(out[0][0], o[0])
         assert np.array_equal(out[0][1], o[1]) and np.array_equal(out[0][2], o[2])
+
+
+_FIRST_RUN = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import __graft_entry__ as ge
+x = ge.load_package()
+ctx = x.Context(0)
+mesh = x.build_mesh3(x.channel_polymesh(16, 8, 8, seed=1))
+n = []
+for k in range(2):
+    model, config = x.cases.channel_case(mesh, iterations=2, precision=sys.argv[2])
+    cfg, keep = x.build_config(model, config)
+    dm = x.DeviceMesh(ctx, mesh)
+    c = x.Case(dm, cfg)
+    c.set_field(x._abi.FIELD_U, model.momentum.U)
+    c.set_field(x._abi.FIELD_P, model.momentum.p)
+    l0 = x.launch_count()
+    c.simple_iterate(2)
+    n.append(x.launch_count() - l0)
+    if k == 0:
+        c.tuning()
+    c.close()
+    dm.close()
+print("launches", *n)
+"""
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_no_trials_for_fused_solves(prec):
+    """The first case of a process launches no trials of kernels its solves do
+    not run: as many launches as a second one, whose choices are cached."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _FIRST_RUN, root, prec], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    n = [int(v) for v in r.stdout.split("launches")[1].split()]
+    assert n[0] == n[1], n

@@ -111,14 +111,22 @@ static int untimed_form(int n, bool fp32, bool alone) {
     return fp32 && alone && n >= 512 && n < 4096 ? 1 : 4;
 }
 
-void Case::autotune() {
-    if (tuned || capturing) return;
-    tuned = true;
+// all: also for an equation whose solves are fused now.  Those read neither
+// choice, and the trials were most of a short first run's launches (two steps
+// of the smoke case: 510 of 589); they are made once profiling, another DILU
+// form or a smoother brings the separate kernels back.
+void Case::autotune(bool all) {
+    if (capturing) return;
     const bool mixed = cfg.precision == XCAL_PREC_MIXED;
     const int tsz = mixed ? 4 : 8;
+    bool ran = false;
     for (int e = 0; e < 2; ++e) {
         Equation& E = e == 0 ? U : P;
         const xcal_solver_setup& SS = e == 0 ? cfg.U_solver : cfg.p_solver;
+        // p's system also carries k, omega, kl and the wall distance
+        const bool own = e == 0 || !(has_k() || has_y());
+        if (E.tuned || (own && !all && use_fused(E, SS, false))) continue;
+        E.tuned = ran = true;
         if (SS.solver == XCAL_SOLVER_BICGSTAB) {
             TuneKey k = key_of(0, tsz, E);
             std::unique_lock<std::mutex> lk(g_tune_mu);
@@ -157,7 +165,7 @@ void Case::autotune() {
             E.use_flow = form == 4;
         }
     }
-    sync();
+    if (ran) sync();
 }
 
 }  // namespace xcal

@@ -479,7 +479,7 @@ int32_t xcal_case_tuning(xcal_case* cs, int32_t* out6) {
     if (!cs || !out6) return XCAL_ERR_INVALID;
     Case* c = cs->c.get();
     XCAL_GUARD(c->ctx, {
-        c->autotune();
+        c->autotune(true);
         const Equation* E[2] = {&c->U, &c->P};
         for (int e = 0; e < 2; ++e) {
             out6[3 * e] = E[e]->spmv_shape.rows_per_thread;

@@ -2673,8 +2673,8 @@ void Case::set_dilu_mode(int mode) {
         E->use_grid = mode == 3;
         // back at 0 as a new case is, its launch shapes yet to be chosen
         E->use_flow = E->flow_D = mode == 0 && !E->lower_off.empty();
+        E->tuned = E->tuned && mode != 0;
     }
-    if (mode == 0) tuned = false;
 }
 
 void Case::set_graph_mode(bool on) {

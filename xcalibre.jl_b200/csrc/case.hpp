@@ -117,6 +117,7 @@ struct Equation {
     bool flow_D = false;      // the DILU factor as a dataflow (k_dilu_D_flow)
     bool use_grid = false;    // else as one cooperative launch over every level (k_dilu_grid)
     SpmvShape spmv_shape;     // BiCGSTAB SpMV row mapping / block size
+    bool tuned = false;       // the autotuner has chosen them
     bool dilu_block() const { return use_block; }
     bool has_periodic = false;
     CSRView view() const;
@@ -370,8 +371,7 @@ struct Case {
     bool use_fold(const Equation& E, const xcal_solver_setup& SS, bool captured) const;
     void fold_iterate(Equation& E, double* field, const KrylovVecs<float>& V, KScalars* S, KScalars* hS, int gk);
     int last_outer[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // mixed: defect-correction steps of the last solve per system
-    bool tuned = false;
-    void autotune();  // launch-shape autotuner (autotune.cu), once per case
+    void autotune(bool all = false);  // launch-shape autotuner (autotune.cu), once per equation
 
     // ---- graph mode: one SIMPLE iteration / PISO step captured as a CUDA
     // graph; the Krylov (and defect-correction) loops are conditional WHILE

@@ -604,14 +604,15 @@ int32_t xcal_case_stream(const xcal_case* cs, void** stream);
  * ms = summed device time, launches = timed launches that did work.  Inside
  * the steady-state CUDA-graph chunks only sampled iterations are timed. */
 int32_t xcal_case_set_profiling(xcal_case* cs, int32_t enable);
-/* graph mode (off by default): each xcal_simple_iterate iteration /
- * xcal_piso_step step replays one CUDA graph captured on first use; when off,
- * the library drives a step from the host or, where that is faster (FP64 cases
- * of at most 524,288 cells, from their third step on), replays it too.  The
+/* graph mode (enable: 0 off, the default; -1 never; anything else on): each
+ * xcal_simple_iterate iteration / xcal_piso_step step replays one CUDA graph
+ * captured on first use; when off, the library drives a step from the host or,
+ * where that is faster (FP64 cases of at most 524,288 cells, from their third
+ * step on), replays it too; never: every step is driven from the host.  The
  * Krylov loops run as conditional WHILE nodes whose stopping tests are taken
- * on the device (at most itmax/4 + 2 loop bodies), so a step needs one host
- * synchronisation.  Results are identical to the default mode.  Per-kernel
- * profiling does not apply inside the graph. */
+ * on the device (at most itmax/4 + 2 loop bodies of a CG, itmax + 2 of a
+ * BiCGSTAB), so a step needs one host synchronisation.  Results are identical
+ * in every mode.  Per-kernel profiling does not apply inside the graph. */
 int32_t xcal_case_set_graph_mode(xcal_case* cs, int32_t enable);
 /* persistent CG (on by default): a CG solve with Jacobi or no preconditioner
  * runs as one launch whenever the system's tiles fit the GPU at once;

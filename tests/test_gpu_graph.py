@@ -1,7 +1,8 @@
 """Graph mode: a SIMPLE iteration / PISO step replayed as one CUDA graph with
 device-driven Krylov loops (conditional WHILE nodes) gives the same results,
-bit for bit, as the default host-polled mode -- FP64 and mixed precision,
-steady and transient (periodic LES)."""
+bit for bit, as host-polled steps and as the default, which replays small FP64
+cases from their third step on -- FP64 and mixed precision, steady and
+transient (periodic LES)."""
 import numpy as np
 import pytest
 
@@ -14,8 +15,7 @@ def _run(x, ctx, mesh, model, config, graph, steps, pref=None, piso=False):
     c = x.Case(dm, cfg)
     c.set_field(x._abi.FIELD_U, model.momentum.U)
     c.set_field(x._abi.FIELD_P, model.momentum.p)
-    if graph:
-        c.set_graph_mode(True)
+    c.set_graph_mode(True if graph else None)  # None: host-polled, whatever the size
     if piso:
         res, co = c.piso_step(steps)
     else:
@@ -196,3 +196,80 @@ def test_no_trials_for_fused_solves(prec):
     assert r.returncode == 0, r.stderr[-2000:]
     n = [int(v) for v in r.stdout.split("launches")[1].split()]
     assert n[0] == n[1], n
+
+
+def _replay_modes(x, ctx, mesh, build, step, names):
+    """Seven FP64 steps, the fields set anew before the fifth, never replayed,
+    replayed from the third on (the default) and always: results, launches of
+    the last step and reports per mode."""
+    out = []
+    for mode in (None, False, True):
+        model, config, pref, fields = build()
+        cfg, keep = x.build_config(model, config, pref=pref)
+        dm = x.DeviceMesh(ctx, mesh)
+        c = x.Case(dm, cfg)
+        c.set_graph_mode(mode)
+        res = []
+        for k in range(7):
+            if k in (0, 4):
+                for f, v in fields(k).items():
+                    c.set_field(getattr(x._abi, f), v)
+            l0 = x.launch_count()
+            res.append(step(c))
+            launches = x.launch_count() - l0
+        out.append((np.array(res), [c.get_field(getattr(x._abi, f)) for f in names], c.solve_report(), launches))
+        c.close()
+        dm.close()
+    for o in out[1:]:
+        assert np.array_equal(o[0], out[0][0])
+        for a, b in zip(o[1], out[0][1]):
+            assert np.array_equal(a, b)
+        for key in ("iterations", "status"):
+            assert np.array_equal(o[2][key], out[0][2][key]), key
+        assert o[2]["itmax_hits"] == out[0][2]["itmax_hits"]
+    # the default's last step is the captured one, the first mode's is not
+    assert out[1][3] == out[2][3] != out[0][3], [o[3] for o in out]
+
+
+@pytest.mark.parametrize("pre", ["Jacobi", "DILU"])
+def test_replayed_steps_equal_host_driven(x, ctx, pre):
+    mesh = x.build_mesh3(x.channel_polymesh(16, 8, 8, seed=11))
+
+    def build():
+        model, config = x.cases.channel_case(mesh, iterations=7)
+        config.solvers["p"].preconditioner = getattr(x, pre)()
+        config.solvers["p"].itmax = 25  # some solves stop there
+        rng = np.random.default_rng(3)
+        U = [0.1 * rng.standard_normal((3, mesh.n_cells)) for _ in range(2)]
+        return model, config, None, lambda k: {"FIELD_U": U[k // 4], "FIELD_P": np.zeros(mesh.n_cells)}
+
+    _replay_modes(x, ctx, mesh, build, lambda c: c.simple_iterate(1)[0][0], ("FIELD_U", "FIELD_P", "FIELD_MDOTF"))
+
+
+def test_replayed_piso_steps_equal_host_driven(x, ctx):
+    mesh = x.build_mesh3(x.periodic_box_polymesh(10, seed=4))
+    U = [x.cases.fourier_field(mesh, seed=s) for s in (4, 5)]
+
+    def build():
+        model, config = x.cases.periodic_les_case(mesh, steps=7, U0=U[0])
+        return model, config, 0.0, lambda k: {"FIELD_U": U[k // 4], "FIELD_P": np.zeros(mesh.n_cells)}
+
+    _replay_modes(x, ctx, mesh, build, lambda c: np.append(c.piso_step(1)[0][0], c.max_courant()),
+                  ("FIELD_U", "FIELD_P", "FIELD_NUT"))
+
+
+def test_replayed_komega_steps_equal_host_driven(x, ctx):
+    from test_gpu_komega import komega_channel_case
+    mesh = x.build_mesh3(x.channel_polymesh(14, 8, 8, seed=2))
+    n = mesh.n_cells
+
+    def build():
+        model, config = komega_channel_case(x, mesh, 7, "DILU")
+        U = np.zeros((3, n))
+        U[0] = 1.0
+        return model, config, None, lambda k: {"FIELD_U": U * (1.0 + 0.1 * k), "FIELD_P": np.zeros(n),
+                                               "FIELD_K": np.full(n, 0.01), "FIELD_OMEGA": np.full(n, 10.0),
+                                               "FIELD_NUT": np.full(n, 1e-3)}
+
+    _replay_modes(x, ctx, mesh, build, lambda c: c.simple_iterate(1)[0][0],
+                  ("FIELD_U", "FIELD_P", "FIELD_K", "FIELD_OMEGA", "FIELD_NUT"))

@@ -952,10 +952,12 @@ class Case:
         mode = int(on) if isinstance(on, bool) else int(on)
         self._chk(lib().xcal_case_set_persistent(self.h, mode))
 
-    def set_graph_mode(self, on: bool = True):
+    def set_graph_mode(self, on: bool | None = True):
         """Replay each SIMPLE iteration / PISO step as one captured CUDA graph
-        (device-driven Krylov loops; same results as the default mode)."""
-        self._chk(lib().xcal_case_set_graph_mode(self.h, 1 if on else 0))
+        (device-driven Krylov loops); False: where the library finds that
+        faster; None: never, every step is driven from the host.  Same
+        results."""
+        self._chk(lib().xcal_case_set_graph_mode(self.h, -1 if on is None else 1 if on else 0))
 
     def profile(self, which: int):
         """(summed device ms, timed launches) of a kernel class:

@@ -227,7 +227,7 @@ struct Batch {
         check_compatible(c);
         c->autotune();
         c->sync();
-        if (c->graph_mode) c->set_graph_mode(false);
+        if (c->graph_mode) c->set_graph_mode(0);
         cudaEvent_t ev = nullptr;
         XCAL_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         joined.push_back(ev);

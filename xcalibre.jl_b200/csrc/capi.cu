@@ -492,7 +492,7 @@ int32_t xcal_case_tuning(xcal_case* cs, int32_t* out6) {
 int32_t xcal_case_set_graph_mode(xcal_case* cs, int32_t enable) {
     if (!cs) return XCAL_ERR_INVALID;
     Case* c = cs->c.get();
-    XCAL_GUARD(c->ctx, { c->set_graph_mode(enable != 0); })
+    XCAL_GUARD(c->ctx, { c->set_graph_mode(enable == -1 ? -1 : enable != 0); })
 }
 
 int32_t xcal_case_get_profile(const xcal_case* cs, int32_t which, double* ms, int64_t* launches) {

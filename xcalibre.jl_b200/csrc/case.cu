@@ -2580,7 +2580,7 @@ void Case::add_phases() {
 // cells 18.9 / 20.3), nor above REPLAY_MAX_CELLS (no difference at 2.1M cells).
 bool Case::replay_step() {
     if (graph_mode) return true;
-    if (no_auto_graph || profiling || batch_err || iteration < 3 || cfg.precision != XCAL_PREC_FP64 ||
+    if (never_replay || no_auto_graph || profiling || batch_err || iteration < 3 || cfg.precision != XCAL_PREC_FP64 ||
         mesh->nC > REPLAY_MAX_CELLS || !kr_coop_capture_ok(false) || !kr_cluster_capture_ok(false))
         return false;
     try {
@@ -2677,7 +2677,9 @@ void Case::set_dilu_mode(int mode) {
     }
 }
 
-void Case::set_graph_mode(bool on) {
+void Case::set_graph_mode(int mode) {
+    const bool on = mode > 0;
+    never_replay = mode < 0;
     if (on == graph_mode) return;
     sync();
     if (step_graph) {

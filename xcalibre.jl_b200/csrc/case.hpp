@@ -398,9 +398,10 @@ struct Case {
     void mark(int k);
     void add_phases();
     bool replay_step();
+    bool never_replay = false;   // steps are host-driven unless graph_mode
     bool no_auto_graph = false;  // a capture failed: replay_step() leaves this case host-driven
     void piso_body(double r3[3], double& rp);
-    void set_graph_mode(bool on);
+    void set_graph_mode(int mode);  // 1 always replay, 0 as replay_step() decides, -1 never
     void set_dilu_mode(int mode);
     void courant_to_slot();
     void capture_while(const std::function<void(cudaGraphConditionalHandle)>& body);

@@ -572,11 +572,17 @@ int32_t xcal_residual_noalloc(int32_t n, const int32_t* rowptr, const int32_t* c
  * kernel launched after it still ran (the context stayed usable). */
 int32_t xcal_check_bounded_wait(xcal_ctx* ctx, int64_t spin_limit, int32_t* gave_up, int32_t* flag_set,
                                 int32_t* ran_after);
-/* the same for the kernels whose rows or blocks wait for values of others:
+/* the same for the waits of a kernel's rows or blocks for one another's values:
  * `which` runs on a small system one of whose values is never written, giving
  * up after spin_limit polls (1 .. 2,097,152).  gave_up = 1 when the kernel
  * ended without that value; flag_set and ran_after as above. */
-enum { XCAL_WAIT_DILU_FACTOR = 0 };
+enum {
+    XCAL_WAIT_DILU_FACTOR = 0, /* the factor's kernel */
+    XCAL_WAIT_DILU_LOWER = 1,  /* ticketed forward sweep */
+    XCAL_WAIT_DILU_UPPER = 2,  /* ticketed backward sweep */
+    XCAL_WAIT_FUSED = 3,       /* a row of the fused BiCGSTAB, its last component missing */
+    XCAL_WAIT_RESIDENT_CG = 4  /* the resident CG's exchange, one block of two */
+};
 int32_t xcal_check_wait(xcal_ctx* ctx, int32_t which, int64_t spin_limit, int32_t* gave_up, int32_t* flag_set,
                         int32_t* ran_after);
 /* that barrier on a case's stream, with the error flag of its DILU solves: the

@@ -9,7 +9,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-KINDS = {"dilu_factor": 0}
+KINDS = {"dilu_factor": 0, "dilu_lower": 1, "dilu_upper": 2, "fused": 3, "resident_cg": 4}
 
 
 @pytest.mark.parametrize("kind", list(KINDS))
@@ -20,6 +20,7 @@ def test_wait_gives_up(x, ctx, kind):
     assert code == 0, L.xcal_last_error(ctx.h)
     assert (gave.value, flag.value, after.value) == (1, 1, 1)
     assert L.xcal_check_wait(ctx.h, KINDS[kind], 0, None, None, None) == x._abi.XCAL_ERR_INVALID
+    assert L.xcal_check_wait(ctx.h, len(KINDS), 1, None, None, None) == x._abi.XCAL_ERR_INVALID
 
 
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])

@@ -143,7 +143,8 @@ __device__ __forceinline__ int bf_mask(const BfView<T, NC>& V, bool running) {
 // column are set in every running component, then finish()
 template <class T, int NC, class F>
 __device__ __forceinline__ bool bf_wait(T* const (&ys)[NC], int run, const int* __restrict__ col, int base, int c,
-                                        const int (&cj)[FLOW_U], T (&yv)[NC][FLOW_U], int* err, F&& finish) {
+                                        const int (&cj)[FLOW_U], T (&yv)[NC][FLOW_U], int* err, F&& finish,
+                                        int spin_limit = FLOW_SPIN_LIMIT) {
     bool fin = c < 0;
 #pragma unroll
     for (int d = 0; d < NC; ++d)
@@ -169,10 +170,7 @@ __device__ __forceinline__ bool bf_wait(T* const (&ys)[NC], int run, const int* 
             }
         }
         if (__all_sync(0xffffffffu, fin)) return true;
-        if (spins > FLOW_SPIN_LIMIT || ((spins & 1023) == 1023 && *(volatile int*)err)) {
-            *(volatile int*)err = 1;
-            return false;
-        }
+        if (flow_give_up(spins, spin_limit, err)) return false;
         if (!fin) {
 #pragma unroll
             for (int d = 0; d < NC; ++d)
@@ -617,6 +615,34 @@ __global__ void k_bf_record(const KScalars* S, int* out, int* hits) {
     if (S[d].status == KS_TIRED) atomicAdd(hits, 1);
     out[2 * d] = S[d].mixed ? S[d].total : S[d].iter;
     out[2 * d + 1] = S[d].status;
+}
+
+// bf_wait of a warp whose first row needs, in the last component, a value that
+// nothing writes; left[lane]: whether the lane left without its row
+__global__ void k_bf_wait_check(double* y0, double* y1, double* y2, const int* col, int* err, int spin_limit,
+                                int* left) {
+    double* ys[BF_MAX] = {y0, y1, y2};
+    const int cj[FLOW_U] = {};
+    double yv[BF_MAX][FLOW_U];
+    const bool ok = bf_wait<double, BF_MAX>(ys, (1 << BF_MAX) - 1, col, 0, threadIdx.x == 0 ? 1 : 0, cj, yv, err,
+                                            [] {}, spin_limit);
+    left[threadIdx.x] = ok ? 0 : 1;
+}
+bool check_fused_wait(int spin_limit, int* err) {
+    DBuf<double> y;
+    DBuf<int> col, left;
+    y.alloc(BF_MAX);
+    y.zero(0);
+    kr_flow_unset(0, y.p + BF_MAX - 1, sizeof(double));
+    col.alloc(1);
+    col.zero(0);
+    left.alloc(32);
+    left.zero(0);
+    k_bf_wait_check<<<1, 32>>>(y.p, y.p + 1, y.p + 2, col.p, err, spin_limit, left.p);
+    XCAL_CHECK_LAUNCH();
+    int h[32];
+    XCAL_CUDA(cudaMemcpy(h, left.p, sizeof(h), cudaMemcpyDeviceToHost));
+    return std::count(h, h + 32, 1) == 32;
 }
 
 // ---------------------------------------------------------------------------

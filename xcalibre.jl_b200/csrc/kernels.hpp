@@ -326,6 +326,8 @@ void kr_flow_unset(cudaStream_t s, void* p, size_t bytes);
 // gives up (0: the usual limit)
 void kr_dilu_D_flow(cudaStream_t s, int n, const LevelDView& L, const double* nz, double* D, unsigned int* ticket,
                     int* err, int spin_limit = 0);
+// a fused BiCGSTAB's wait made to run out (bicg_fused.cu): whether the whole warp left
+bool check_fused_wait(int spin_limit, int* err);
 void kr_residual(cudaStream_t s, const CSRView& A, const double* nz, const double* x, const double* b, KScalars* S,
                  double* part0, double* part1, double* out);
 // device-driven solve control of graph mode (conditional WHILE nodes)

@@ -815,7 +815,7 @@ __device__ __forceinline__ int flow_ticket(unsigned int* ticket, int* sh, bool o
 // marks out's rows unset for the backward rows
 template <class T>
 __device__ __forceinline__ bool flow_lower_rows(int n, const LevelView<T>& lo, const T* __restrict__ b, T* y, T* out,
-                                                int k0, int* err) {
+                                                int k0, int* err, int spin_limit = FLOW_SPIN_LIMIT) {
     const int k = k0 + (threadIdx.x & 31);
     int i = 0, c = -1, base = 0;
     int cj[FLOW_U];
@@ -846,7 +846,7 @@ __device__ __forceinline__ bool flow_lower_rows(int n, const LevelView<T>& lo, c
             sum = sum + (ld_stream(lo.val + e) * ld_flow(y + ld_stream(lo.col + e))) * ld_stream(lo.dinv + e);
         }
         st_flow(y + i, rhs - sum);
-    });
+    }, spin_limit);
 }
 
 // backward_substitution! (preconditioners_1_DILU.jl:100-114) of the warp's
@@ -854,7 +854,7 @@ __device__ __forceinline__ bool flow_lower_rows(int n, const LevelView<T>& lo, c
 // values in y, which are marked unset again)
 template <class T>
 __device__ __forceinline__ bool flow_upper_rows(int n, const LevelView<T>& up, const T* __restrict__ D, T* y, T* out,
-                                                int k0, int* err) {
+                                                int k0, int* err, int spin_limit = FLOW_SPIN_LIMIT) {
     const int k = k0 + (threadIdx.x & 31);
     int i = 0, c = -1, base = 0;
     int cj[FLOW_U];
@@ -885,7 +885,7 @@ __device__ __forceinline__ bool flow_upper_rows(int n, const LevelView<T>& up, c
             sum = sum + ld_stream(up.val + e) * ld_flow((const T*)out + ld_stream(up.col + e));
         }
         st_flow(out + i, (yi - sum) / Di);
-    });
+    }, spin_limit);
 }
 
 // update_dilu_diagonal! row i (preconditioners_1_DILU.jl:43-82)
@@ -1459,7 +1459,7 @@ __device__ __forceinline__ double res_tile_sum(const double* pr, double* sm8) {
 // buf; the block polls its own row and leaves it unset again (release: with
 // everything the block wrote before).  false: gave up.
 __device__ __forceinline__ bool res_exchange(double tot, const TileCtx& tc, double* buf, bool release, int* err,
-                                             double& sum) {
+                                             double& sum, int spin_limit) {
     const int T = tc.ntiles, lane = threadIdx.x & 31;
     if (T == 1) {
         sum = 0.0 + tot;
@@ -1482,7 +1482,7 @@ __device__ __forceinline__ bool res_exchange(double tot, const TileCtx& tc, doub
 #pragma unroll
         for (int j = 0; j < 8; ++j) all = all && !flow_unset(w[j]);
         if (__all_sync(0xffffffffu, all)) break;
-        if (spins > FLOW_SPIN_LIMIT || ((spins & 1023) == 1023 && *(volatile int*)err)) {
+        if (flow_give_up(spins, spin_limit, err)) {
             ok = false;
             break;
         }
@@ -1493,11 +1493,7 @@ __device__ __forceinline__ bool res_exchange(double tot, const TileCtx& tc, doub
             row[32 * j + lane] = flow_unset_value<double>();
             w[j] = 0.0 + w[j];
         }
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) {
-        if (lane == 0) *(volatile int*)err = 1;
-        return false;
-    }
+    if (!ok) return false;
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1)
 #pragma unroll
@@ -1536,7 +1532,8 @@ template <class T, bool CL>
 __device__ __forceinline__ void cg_resident_body(const TileCtx& tc, const CSRView& A, const T* __restrict__ nz,
                                                  const T* __restrict__ Pj, int jacobi, T* x, const T* r, T* z, const T* pg,
                                                  KScalars* S, double* ring, int* err, int max_iters, int slots,
-                                                 int halo, unsigned char* smem) {
+                                                 int halo, unsigned char* smem,
+                                                 int spin_limit = FLOW_SPIN_LIMIT) {
     __shared__ double sm8[8];
     __shared__ ResState st;
     double* pr = reinterpret_cast<double*>(smem);
@@ -1646,7 +1643,8 @@ __device__ __forceinline__ void cg_resident_body(const TileCtx& tc, const CSRVie
         double pAp = 0.0;
         if constexpr (CL) pAp = res_exchange_cl(tot, tc, cl_part[0]);
         if (threadIdx.x < 32) {
-            const bool ok = CL || res_exchange(tot, tc, ring + (size_t)(ran & 1) * tc.ntiles * tc.ntiles, false, err, pAp);
+            const bool ok = CL || res_exchange(tot, tc, ring + (size_t)(ran & 1) * tc.ntiles * tc.ntiles, false, err, pAp,
+                                             spin_limit);
             if (threadIdx.x == 0) {
                 const double lim = epsT * st.pNorm2;
                 if (!ok) {
@@ -1686,7 +1684,8 @@ __device__ __forceinline__ void cg_resident_body(const TileCtx& tc, const CSRVie
         if constexpr (CL) g = res_exchange_cl(tot, tc, cl_part[1]);
         if (threadIdx.x < 32) {
             const bool ok =
-                CL || res_exchange(tot, tc, ring + (size_t)(2 + (ran & 1)) * tc.ntiles * tc.ntiles, true, err, g);
+                CL || res_exchange(tot, tc, ring + (size_t)(2 + (ran & 1)) * tc.ntiles * tc.ntiles, true, err, g,
+                                   spin_limit);
             if (threadIdx.x == 0) {  // cg_finalize on the block's copy of the state
                 const double rn = sqrt(g);
                 const bool solved = (rn <= eps) || (rn + 1.0 <= 1.0);

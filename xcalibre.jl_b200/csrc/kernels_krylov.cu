@@ -909,7 +909,11 @@ int persist_cluster_size(const void* kernel, int tiles, size_t smem) {
     if (tiles <= 0 || tiles > PERSIST_CLUSTER_MAX) return 0;
     int C = 1;
     while (C < tiles) C *= 2;
-    // schedulability per (kernel, C), found once
+    // schedulability per (kernel, C, with shared memory or without), found once:
+    // asked for the most a block may have, so that the answers are a handful
+    // however many systems come along (a block of 1024 threads has an SM to
+    // itself whatever it asks for)
+    if (smem > 0) smem = RES_SMEM_MAX;
     static std::mutex mu;
     static std::map<std::tuple<const void*, int, size_t>, bool> ok;
     std::lock_guard<std::mutex> lk(mu);

@@ -619,7 +619,7 @@ void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& b
             for (int i = 0; i < n; ++i) rows[cur[lvl[i]]++] = i;
         }
         E.d_lower_rows.upload(rows, s);
-        E.h_lower_rows = rows;
+        const std::vector<int> lower_rows = rows;
         E.d_lower_off.upload(E.lower_off, s);
         std::fill(lvl.begin(), lvl.end(), 0);
         maxl = 0;
@@ -639,11 +639,10 @@ void build_equation(Equation& E, const DevMesh& m, const std::vector<xcal_bc>& b
             for (int i = 0; i < n; ++i) rows[cur[lvl[i]]++] = i;
         }
         E.d_upper_rows.upload(rows, s);
-        E.h_upper_rows = rows;
         E.d_upper_off.upload(E.upper_off, s);
         // level-ordered copies of the strictly lower / upper entries
         for (int tri = 0; tri < 2; ++tri) {
-            const std::vector<int>& order = tri == 0 ? E.h_lower_rows : E.h_upper_rows;
+            const std::vector<int>& order = tri == 0 ? lower_rows : rows;
             LevelSell& L = tri == 0 ? E.lsell : E.usell;
             const int nsl2 = (n + SELL_C - 1) / SELL_C;
             std::vector<int> sl(nsl2 + 1, 0);
@@ -2573,11 +2572,13 @@ void Case::add_phases() {
 
 // Whether this iteration replays the step graph: in graph mode, and otherwise
 // from the third iteration on where launches and host round trips are a good
-// part of it.  Measured on B200 (ms per pass, host-driven / graph): 1,073 cells
-// 5.6 / 4.7 (10 iterations), 7,500 cells with k, omega and kl 10.4 / 8.9 (5),
-// 116,440 cells DILU-CG 25.5 / 22.8 (3); the capture costs about 1 ms once.  Not
-// in mixed precision, whose captured momentum solves are not fused (262,144
-// cells 18.9 / 20.3), nor above REPLAY_MAX_CELLS (no difference at 2.1M cells).
+// part of it.  Measured on B200 (ms per SIMPLE iteration, host-driven / graph):
+// FP64 1,073 cells 0.58 / 0.51, 27,025 cells 1.05 / 0.96, 262,144 cells 4.39 / 4.30,
+// 884,736 cells 23.5 / 23.4; 7,500 cells with k, omega and kl 2.1 / 1.8, 116,440
+// cells DILU-CG 8.5 / 7.6; the capture costs about 1 ms once.  Not above
+// REPLAY_MAX_CELLS, where there is no difference, and not in mixed precision,
+// where there is less to gain (1,073 cells 0.70 / 0.66, 27,025 cells 0.98 / 0.94,
+// 262,144 cells 4.07 / 4.01): such cases replay in graph mode only.
 bool Case::replay_step() {
     if (graph_mode) return true;
     if (never_replay || no_auto_graph || profiling || batch_err || iteration < 3 || cfg.precision != XCAL_PREC_FP64 ||

@@ -108,7 +108,6 @@ struct Equation {
     // DILU level schedules (rows grouped by dependency level)
     DBuf<int> d_lower_rows, d_upper_rows;
     std::vector<int> lower_off, upper_off;
-    std::vector<int> h_lower_rows, h_upper_rows;  // host copies (batched level lists)
     DBuf<int> d_lower_off, d_upper_off;           // level offsets (one-block sweeps)
     LevelSell lsell, usell;                       // level-ordered triangles (level-kernel sweeps)
     // launch choices (autotune.cu); neither changes any result

@@ -1388,10 +1388,11 @@ __device__ __forceinline__ void cg_persist_mt_body(const CSRView& A, const T* __
 // ---- persistent CG with the matrix resident in shared memory ----
 // For systems of at most one canonical tile per SM.  The block of tile t
 // keeps the tile's slots (values, and columns as 16-bit local indices) in
-// shared memory for the whole solve, and x, r, z, p, q of its rows in
-// registers (1024 threads, two rows each), so an iteration touches L2 only
-// for the values other tiles own: the tile's halo, one entry per slot whose
-// column lies outside it.  Per iteration
+// shared memory for the whole solve, z of its rows and halo beside them, and x,
+// r, p, q of its rows in registers (1024 threads, two rows each), so an
+// iteration touches L2 only for the values other tiles own: the tile's halo,
+// one entry per slot whose column lies outside it (and in a cluster not even
+// for those).  Per iteration
 //   each thread forms p_k = z + beta p_{k-1} for its rows and its halo
 //   entries once (not once per slot), into shared memory;
 //   q = A p_k from shared memory; <p_k, q>;
@@ -1408,17 +1409,17 @@ __device__ __forceinline__ void cg_persist_mt_body(const CSRView& A, const T* __
 // iterations later, by a block that has acquired this one's <r, z> in between,
 // whose release covers the reset and z.  <p, q> needs no release: its block has
 // written nothing since but its own rows' resets, and whoever overwrites the z
-// it read depends on the
-// partial those reads went into.  Arithmetic and
+// it read depends on the partial those reads went into.  Arithmetic and
 // reduction trees are cg_persist_body's, so the results are the same bit for
 // bit.  Waits are bounded as in grid_barrier.
 //
 // What bounds it: shared-memory bandwidth of the slots (2048 rows x 7 slots x
 // 18 bytes and their bank conflicts, 1.2 us FP32, 2.4 us FP64) and the two
 // exchanges (1.2-1.5 us each in a cluster, 2.5-3.5 us through L2).  Measured
-// on B200, us per iteration, this against the forms without the matrix in
-// shared memory (FP64): 1,073 rows 4.0 / 7.0, 7,500 rows 6.1 / 11.2, 27,025
-// rows 7.7 / 12.2, 129,150 rows 8.7 / 13.2.
+// on B200, us per iteration over whole solves, loading the matrix included,
+// this against the forms without it in shared memory: FP64 1,073 rows 3.5 / 8.3,
+// 7,500 rows 6.6 / 11.7, 27,025 rows 7.0 / 12.1, 129,150 rows 9.2 / 15.1; FP32 3.1 /
+// 7.4, 4.7 / 9.3, 5.0 / 9.3, 7.5 / 11.5.
 constexpr int RES_THREADS = 1024;
 constexpr int RES_ROWS = RED_TILE / RES_THREADS;  // rows per thread
 constexpr int RES_HALO_PT = 4;                    // halo entries per thread
@@ -1524,8 +1525,8 @@ __device__ __forceinline__ double res_exchange_cl(double tot, const TileCtx& tc,
 // CL: the system's tiles are the blocks of one thread-block cluster; z and the
 // partials travel through distributed shared memory, with no trip to L2 in an
 // iteration.  The owner of a row writes its z into the halo entries that read
-// it (27,025 rows: 6.6 us per iteration; 7.7 us when the entries were read
-// from their owners at the start of the next iteration).  The same through L2,
+// it (27,025 rows, long solves: 6.6 us per iteration; 7.7 us when the entries
+// were read from their owners at the start of the next iteration).  The same through L2,
 // with a tag beside each z, measured slower than a coalesced z array behind
 // the <r, z> exchange's release (62,403 rows: 19.4 against 18.5 ms per pass).
 template <class T, bool CL>

@@ -873,19 +873,22 @@ bool persist_launch(PersistCaps& c, int w, const void* kernel, int ntiles, cudaS
 
 int resident_sms(const void* kernel, size_t smem) {
     if (smem > (size_t)RES_SMEM_MAX) return 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    // per device and kernel: the limit set here is the current device's
     static std::mutex mu;
-    static std::map<const void*, int> sms;  // per kernel, one device type
+    static std::map<std::pair<int, const void*>, int> sms;
     std::lock_guard<std::mutex> lk(mu);
-    auto it = sms.find(kernel);
+    const auto key = std::make_pair(dev, kernel);
+    auto it = sms.find(key);
     if (it == sms.end()) {
-        int dev = 0, m = 0, per = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        int m = 0, per = 0;
+        if (cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM_MAX) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, RES_THREADS, RES_SMEM_MAX) != cudaSuccess)
             per = 0;
         cudaGetLastError();
-        it = sms.emplace(kernel, per > 0 ? m : 0).first;
+        it = sms.emplace(key, per > 0 ? m : 0).first;
     }
     return it->second;
 }
@@ -909,15 +912,17 @@ int persist_cluster_size(const void* kernel, int tiles, size_t smem) {
     if (tiles <= 0 || tiles > PERSIST_CLUSTER_MAX) return 0;
     int C = 1;
     while (C < tiles) C *= 2;
-    // schedulability per (kernel, C, with shared memory or without), found once:
+    // schedulability per (device, kernel, C, with shared memory or without), found once:
     // asked for the most a block may have, so that the answers are a handful
     // however many systems come along (a block of 1024 threads has an SM to
     // itself whatever it asks for)
     if (smem > 0) smem = RES_SMEM_MAX;
     static std::mutex mu;
-    static std::map<std::tuple<const void*, int, size_t>, bool> ok;
+    static std::map<std::tuple<int, const void*, int, size_t>, bool> ok;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     std::lock_guard<std::mutex> lk(mu);
-    auto key = std::make_tuple(kernel, C, smem);
+    auto key = std::make_tuple(dev, kernel, C, smem);
     auto it = ok.find(key);
     if (it == ok.end()) {
         bool good = true;

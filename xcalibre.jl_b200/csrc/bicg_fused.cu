@@ -654,23 +654,14 @@ static void bf_flow_pre(cudaStream_t s, const BfView<T, NC>& V) {
     const int want = (V.A.n + FLOW_THREADS - 1) / FLOW_THREADS;
     if constexpr (PRE != XCAL_PRECOND_DILU) {
         k_bf_flow<T, NC, PRE, MODE><<<want, FLOW_THREADS, 0, s>>>(V);
+        XCAL_CHECK_LAUNCH();
     } else {
         const int blocks = std::min(flow_grid(k), want);
-        if (blocks <= 0) fail(XCAL_ERR_CUDA, "fused BiCGSTAB: the DILU kernel does not fit the device");
         BfView<T, NC> Vv = V;
         void* args[] = {&Vv};
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(FLOW_THREADS);
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        XCAL_CUDA(cudaLaunchKernelExC(&cfg, k, args));
+        if (!flow_launch(k, blocks, s, args))
+            fail(XCAL_ERR_CUDA, "fused BiCGSTAB: the DILU kernel does not fit the device");
     }
-    XCAL_CHECK_LAUNCH();
 }
 template <class T, int NC, int MODE>
 static void bf_flow(cudaStream_t s, const BfView<T, NC>& V, int pre) {

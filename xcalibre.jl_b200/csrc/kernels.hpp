@@ -224,8 +224,9 @@ void persist_cluster_launch(const void* kernel, int C, int nclusters, cudaStream
 // Resident form: whether `kernel` (RES_THREADS threads a block) runs with
 // `smem` bytes of dynamic shared memory, and the device's SM count (0: not)
 int resident_sms(const void* kernel, size_t smem);
-// cooperative launch of the resident form over ntiles blocks
-void resident_launch(const void* kernel, int ntiles, size_t smem, cudaStream_t s, void** args);
+// cooperative launch of the resident form over ntiles blocks (false: nothing
+// launched, as fewer SMs are to be had)
+bool resident_launch(const void* kernel, int ntiles, size_t smem, cudaStream_t s, void** args);
 void kr_finish(cudaStream_t s, int n, const double* x, const double* dx, double* field);
 template <class T>
 void kr_bicg_start(cudaStream_t s, int n, const T* c, const T* r, T* p, KScalars* S, double* part0, double* part1);
@@ -319,6 +320,9 @@ bool kr_dilu_flow(cudaStream_t s, int n, const LevelView<T>& lo, const LevelView
 // co-resident blocks of FLOW_THREADS threads of a dataflow kernel (0: none)
 constexpr int FLOW_THREADS = 256;
 int flow_grid(const void* kernel);
+// cooperative launch of one on `blocks` blocks or, where those are refused, on
+// as many as are taken (false: none)
+bool flow_launch(const void* kernel, int blocks, cudaStream_t s, void** args);
 // marks values as not yet computed (all bits one)
 void kr_flow_unset(cudaStream_t s, void* p, size_t bytes);
 // the DILU factor in the same way (D is set to unset values first; ticket:

@@ -359,8 +359,7 @@ bool kb_cg_resident(cudaStream_t s, const BSys<T>* sys, const int2* tmap, int nt
     if (ntiles_total <= 0 || ntiles_total > resident_sms(k, smem)) return false;
     XCAL_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
     void* args[] = {(void*)&sys, (void*)&tmap, &jacobi, &err, &max_iters, &slots, &halo};
-    resident_launch(k, ntiles_total, smem, s, args);
-    return true;
+    return resident_launch(k, ntiles_total, smem, s, args);
 }
 template <class T>
 int kb_cg_cluster_size(int tiles, int slots, int halo) {

@@ -893,7 +893,7 @@ int resident_sms(const void* kernel, size_t smem) {
     return it->second;
 }
 
-void resident_launch(const void* kernel, int ntiles, size_t smem, cudaStream_t s, void** args) {
+bool resident_launch(const void* kernel, int ntiles, size_t smem, cudaStream_t s, void** args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ntiles);
     cfg.blockDim = dim3(RES_THREADS);
@@ -904,8 +904,14 @@ void resident_launch(const void* kernel, int ntiles, size_t smem, cudaStream_t s
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    XCAL_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has are ours
+        cudaGetLastError();
+        return false;
+    }
+    XCAL_CUDA(e);
     XCAL_CHECK_LAUNCH();
+    return true;
 }
 
 int persist_cluster_size(const void* kernel, int tiles, size_t smem) {
@@ -996,8 +1002,7 @@ bool kr_cg_persist(cudaStream_t s, const CSRView& A, const T* nz, const T* P, in
             CSRView Av = A;
             void* args[] = {&Av, (void*)&nz, (void*)&P, &jacobi, &x,   &r,     &z,    &P0,
                             &S,  &ring,      &err,      &max_iters, &slots, &halo};
-            resident_launch(kr, nt, smem, s, args);
-            return true;
+            if (resident_launch(kr, nt, smem, s, args)) return true;
         }
     }
     // the automatic choice past the one-tile-per-block forms: one block per
@@ -1297,6 +1302,28 @@ int flow_grid(const void* kernel) {
     }
     return it->second;
 }
+bool flow_launch(const void* kernel, int blocks, cudaStream_t s, void** args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(FLOW_THREADS);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    for (; blocks > 0; blocks /= 2) {
+        cfg.gridDim = dim3(blocks);
+        const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has are ours
+            cudaGetLastError();
+            continue;
+        }
+        XCAL_CUDA(e);
+        XCAL_CHECK_LAUNCH();
+        return true;
+    }
+    return false;
+}
 template <class T>
 bool kr_dilu_flow(cudaStream_t s, int n, const LevelView<T>& lo, const LevelView<T>& up, const T* D, const T* b,
                   T* y, T* out, unsigned int* bar, int* err, const KScalars* S) {
@@ -1305,18 +1332,7 @@ bool kr_dilu_flow(cudaStream_t s, int n, const LevelView<T>& lo, const LevelView
     XCAL_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned int), s));
     LevelView<T> l = lo, u = up;
     void* args[] = {&n, &l, &u, (void*)&D, (void*)&b, &y, &out, &bar, &err, (void*)&S};
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(FLOW_THREADS);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    XCAL_CUDA(cudaLaunchKernelExC(&cfg, (const void*)k_dilu_flow<T>, args));
-    XCAL_CHECK_LAUNCH();
-    return true;
+    return flow_launch((const void*)k_dilu_flow<T>, blocks, s, args);
 }
 template bool kr_dilu_flow<double>(cudaStream_t, int, const LevelView<double>&, const LevelView<double>&,
                                    const double*, const double*, double*, double*, unsigned int*, int*,

@@ -190,3 +190,21 @@ def test_case_carries_on_after_its_batch(x, ctx):
         dm.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_footprint_of_a_case_alone(x, ctx, prec):
+    """What a case allocates at its first step alone (the fused momentum
+    solve's vectors) is within the share of its footprint the serving loop
+    reserves for it."""
+    from importlib import import_module
+    share = import_module(x.__name__ + ".serve").SOLO_SHARE
+    for kind, n in (("channel", 12), ("cavity", 40), ("channel", 30)):
+        c, keep = _mk(x, ctx, kind, n, 1, prec, 1e-3)
+        est = x.api.footprint_estimate(c.mesh, prec, dilu_U=True, dilu_p=False)
+        before = sum(c.footprint())
+        c.set_graph_mode(True)
+        c.simple_iterate(1)
+        after = sum(c.footprint())
+        assert before < after <= est + est // share, (before, after, est)
+        c.close()

@@ -169,3 +169,32 @@ def test_reservations_bound_set_up_ahead(serve, monkeypatch):
     assert [r.status for r in res] == ["converged"] * 8
     assert ledger.peak <= 2000, ledger.peak
     assert ledger.held == 0
+
+
+@pytest.mark.parametrize("size,alone", [(4000, True), (4500, False)])
+def test_last_case_alone_stays_within_the_budget(serve, monkeypatch, size, alone):
+    """The last case of a drained stream runs alone only where what it then
+    allocates besides its footprint fits the budget, finished cases freed."""
+    reqs = _stream(serve, 2)
+    sizes = {reqs[0].rid: 1000, reqs[1].rid: size}
+    ledger = Ledger()
+    DM, CS, BT = fakes(serve, ledger, lambda m: sizes[m.rid], poisoned={reqs[0].rid}, iters_to_converge=6)
+    went_alone = []
+
+    class Alone(CS):
+        def set_graph_mode(self, on=True):
+            ledger.take(self, self.nbytes // 5)
+            self.nbytes += self.nbytes // 5
+            went_alone.append(self.rid)
+
+    monkeypatch.setattr(serve.A, "DeviceMesh", DM)
+    monkeypatch.setattr(serve.A, "Case", Alone)
+    monkeypatch.setattr(serve.A, "Batch", BT)
+    monkeypatch.setattr(serve.Server, "footprint", lambda self, req: sizes[req.rid])
+    srv = serve.Server(ctx=None, budget_bytes=5000, max_cases=4, precision="mixed", max_iters=50, build_threads=0,
+                       free_every=16)
+    res = srv.run(reqs, realtime=False)
+    assert {r.rid: r.status for r in res} == {reqs[0].rid: "diverged", reqs[1].rid: "converged"}
+    assert ledger.peak <= 5000, ledger.peak
+    assert ledger.held == 0
+    assert (reqs[1].rid in went_alone) == alone
